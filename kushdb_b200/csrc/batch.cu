@@ -18,8 +18,13 @@
 //      matched build row's accumulator (the dimension key is the table's
 //      primary key, so the build row is the group; duplicate build keys are
 //      detected and reported);
-//   3. output -- compact each query's touched build rows into its result.
-// Each CTA owns a fixed chunk of one query's rows (block x 16), and chunks
+//   3. order  -- put each query's touched build rows (its groups) in the
+//      order of their first fact rows.  A fact row matches at most one build
+//      row, so the first rows of a query's groups differ: a bitmap over its
+//      fact rows with one bit per group, and the number of bits before a
+//      group's own, give the group's place without a sort;
+//   4. output -- write every group at its place.
+// Each CTA owns a fixed chunk of one query's rows (block x 4), and chunks
 // are numbered query after query, so the CTAs resident at any moment work on
 // a few queries and their join tables and accumulators stay in L2.
 // Capacities are sized when the batch is configured, so no phase needs a
@@ -44,8 +49,15 @@
 namespace kdb {
 namespace {
 
-constexpr int kRowsPerThread = 16;  // rows of one chunk per thread
-constexpr int kProbeUnroll = 4;     // independent probes in flight per thread
+// Rows of one chunk per thread.  Every phase is a chain of dependent random
+// accesses per row (bound by their latency, not by bytes), so the SMs want
+// many warps: few rows per thread and few registers.  Measured on 24 queries
+// of 10k to 2M fact rows, build 64 / 39 us with 16 / 4 dimension rows per
+// thread; probe with 4 rows in flight per thread (63 registers, half the
+// warps) 157 us, one row at a time 107 us (2 or 8 rows per thread: the same
+// within 2%; 16: 20% slower on queries of 100k rows, too few CTAs).
+constexpr int kRowsPerThread = 4;
+constexpr int kDimUnroll = 4;  // rows of one thread in flight when marking and writing groups
 
 struct QueryDesc {
   // dimension side
@@ -68,10 +80,14 @@ struct QueryDesc {
   int64_t acc_base;
   // result region out[out_base ...] (capacity nd)
   int64_t out_base;
-  // CTA ranges of the three phases (one chunk of rows per CTA)
+  // first-row bitmap first[bit_base ...], kOrderWords words per order chunk
+  int64_t bit_base;
+  // CTA ranges of the phases (one chunk of rows, or of bitmap words, per CTA);
+  // the mark and output phases share the dimension side's chunks
   int32_t build_block0, build_blocks;
   int32_t probe_block0, probe_blocks;
   int32_t out_block0, out_blocks;
+  int32_t order_block0, order_blocks;
 };
 
 // Per build row: the running sum and the complement of the first fact row
@@ -81,6 +97,16 @@ struct Acc {
   unsigned long long first_inv;
 };
 static_assert(sizeof(Acc) == 16, "Acc layout");
+
+// One word of a query's first-row bitmap: the bits of 32 fact rows, and the
+// groups whose first row lies before them.
+struct FirstWord {
+  uint32_t bits;
+  uint32_t before;
+};
+static_assert(sizeof(FirstWord) == 8, "FirstWord layout");
+constexpr int kOrderThreads = 256;
+constexpr int kOrderWords = 4 * kOrderThreads;  // bitmap words per CTA of the order phase
 
 // 64-bit mix of the key: the top bits choose the sub-table, the low 32 bits
 // the home slot inside it, so the two are independent.
@@ -106,7 +132,10 @@ __device__ __forceinline__ int FindQuery(const QueryDesc* qs, int nq, int block)
   int lo = 0, hi = nq - 1;
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
-    int b0 = kPhase == 0 ? qs[mid].build_block0 : kPhase == 1 ? qs[mid].probe_block0 : qs[mid].out_block0;
+    int b0 = kPhase == 0   ? qs[mid].build_block0
+             : kPhase == 1 ? qs[mid].probe_block0
+             : kPhase == 2 ? qs[mid].out_block0
+                           : qs[mid].order_block0;
     if (b0 <= block) lo = mid;
     else hi = mid - 1;
   }
@@ -174,85 +203,151 @@ __global__ void BatchBuild(const QueryDesc* __restrict__ qs, int nq, unsigned lo
   }
 }
 
-// sum and first fact row per build row; kProbeUnroll rows per thread are
-// loaded and hashed together so their table reads overlap.
-// eager: the measures of the unrolled rows load with their keys, so their
-// HBM latency overlaps the probes (otherwise only matching rows load them)
+// Sum and first fact row per build row.
+// eager: a row's measures load with its key, so their HBM latency overlaps
+// the probe (otherwise only matching rows load them: 6% slower)
 __global__ void BatchProbe(const QueryDesc* __restrict__ qs, int nq, const unsigned long long* __restrict__ slots,
                            int fanout_bits, Acc* __restrict__ acc, int eager) {
   int64_t r0, r1;
   const QueryDesc& q = Chunk<1>(qs, nq, r0, r1);
-  const int64_t step = blockDim.x;
-  for (int64_t base = r0 + threadIdx.x; base < r1; base += kProbeUnroll * step) {
-    int32_t k[kProbeUnroll];
-    double mp[kProbeUnroll], md[kProbeUnroll];
-    uint32_t pos[kProbeUnroll];
-    const unsigned long long* sub[kProbeUnroll];
-    unsigned long long e[kProbeUnroll];
-#pragma unroll
-    for (int j = 0; j < kProbeUnroll; j++) {
-      const int64_t r = base + j * step;
-      k[j] = r < r1 ? __ldcs(q.f_fk + r) : 0;
-      mp[j] = eager && r < r1 ? __ldcs(q.f_price + r) : 0.0;
-      md[j] = eager && r < r1 ? __ldcs(q.f_disc + r) : 0.0;
+  for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+    const int32_t k = __ldcs(q.f_fk + r);
+    double pr = 0.0, di = 0.0;
+    if (eager) {
+      pr = __ldcs(q.f_price + r);
+      di = __ldcs(q.f_disc + r);
     }
-#pragma unroll
-    for (int j = 0; j < kProbeUnroll; j++) {
-      const uint64_t h = KeyHash(k[j]);
-      sub[j] = slots + q.slot_base + static_cast<int64_t>(SubTable(h, fanout_bits)) * q.sub_cap;
-      pos[j] = HomeSlot(h, q.sub_cap);
-      e[j] = base + j * step < r1 ? sub[j][pos[j]] : 0ULL;
-    }
-#pragma unroll
-    for (int j = 0; j < kProbeUnroll; j++) {
-      const int64_t r = base + j * step;
-      if (r >= r1) continue;
-      unsigned long long s = e[j];
-      uint32_t i = pos[j];
-      for (uint32_t n = 0; s != 0 && n < q.sub_cap; n++) {
-        if (static_cast<uint32_t>(s >> 32) == static_cast<uint32_t>(k[j])) {
-          Acc* a = acc + q.acc_base + (static_cast<int64_t>(static_cast<uint32_t>(s)) - 1);
-          // plain per-row IEEE arithmetic, like the reference's generated code
-          const double pr = eager ? mp[j] : __ldcs(q.f_price + r), di = eager ? md[j] : __ldcs(q.f_disc + r);
-          const double v = __dmul_rn(pr, __dsub_rn(1.0, di));
-          atomicAdd(&a->sum, v);
-          // the first fact row only moves down: skip the atomic once an
-          // earlier row is already recorded (a stale read costs one atomic)
-          const unsigned long long fi = ~static_cast<unsigned long long>(r);
-          if (__ldcg(&a->first_inv) < fi) atomicMax(&a->first_inv, fi);
-          break;  // keys are unique on the build side
+    const uint64_t h = KeyHash(k);
+    const unsigned long long* sub = slots + q.slot_base + static_cast<int64_t>(SubTable(h, fanout_bits)) * q.sub_cap;
+    uint32_t i = HomeSlot(h, q.sub_cap);
+    unsigned long long s = sub[i];
+    for (uint32_t n = 0; s != 0 && n < q.sub_cap; n++) {
+      if (static_cast<uint32_t>(s >> 32) == static_cast<uint32_t>(k)) {
+        Acc* a = acc + q.acc_base + (static_cast<int64_t>(static_cast<uint32_t>(s)) - 1);
+        if (!eager) {
+          pr = __ldcs(q.f_price + r);
+          di = __ldcs(q.f_disc + r);
         }
-        if (++i == q.sub_cap) i = 0;
-        s = sub[j][i];
+        // plain per-row IEEE arithmetic, like the reference's generated code
+        atomicAdd(&a->sum, __dmul_rn(pr, __dsub_rn(1.0, di)));
+        // the first fact row only moves down: skip the atomic once an
+        // earlier row is already recorded (a stale read costs one atomic)
+        const unsigned long long fi = ~static_cast<unsigned long long>(r);
+        if (__ldcg(&a->first_inv) < fi) atomicMax(&a->first_inv, fi);
+        break;  // keys are unique on the build side
       }
+      if (++i == q.sub_cap) i = 0;
+      s = sub[i];
     }
   }
 }
 
-// per query: build rows with a match -> (key, sum, first fact row); one
-// counter atomic per warp
+// Per group: the bit of its first fact row, and a count per order chunk
+// (counted in shared memory while the query's chunks fit there: a million
+// groups on a few hundred counters queue in L2 otherwise, 84 against 14 us
+// for 24 queries of 10k to 2M fact rows).
+constexpr int kMarkChunks = 1024;
+__global__ void BatchMark(const QueryDesc* __restrict__ qs, int nq, const Acc* __restrict__ acc,
+                          FirstWord* __restrict__ first, uint32_t* __restrict__ chunk_groups) {
+  int64_t r0, r1;
+  __shared__ uint32_t groups[kMarkChunks];
+  const QueryDesc& q = Chunk<2>(qs, nq, r0, r1);
+  const int chunks = q.order_blocks;
+  const bool in_shared = chunks <= kMarkChunks;
+  if (in_shared) {
+    for (int i = threadIdx.x; i < chunks; i += blockDim.x) groups[i] = 0;
+    __syncthreads();
+  }
+  const int64_t step = blockDim.x;
+  for (int64_t base = r0 + threadIdx.x; base < r1; base += kDimUnroll * step) {
+    unsigned long long inv[kDimUnroll];
+#pragma unroll
+    for (int j = 0; j < kDimUnroll; j++)
+      inv[j] = base + j * step < r1 ? acc[q.acc_base + base + j * step].first_inv : 0ULL;
+#pragma unroll
+    for (int j = 0; j < kDimUnroll; j++) {
+      if (inv[j] == 0) continue;
+      const unsigned long long f = ~inv[j];
+      atomicOr(&first[q.bit_base + static_cast<int64_t>(f >> 5)].bits, 1u << (f & 31));
+      const int c = static_cast<int>(f / (32 * kOrderWords));
+      if (in_shared) atomicAdd(&groups[c], 1u);
+      else atomicAdd(&chunk_groups[q.order_block0 + c], 1u);
+    }
+  }
+  if (in_shared) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < chunks; i += blockDim.x)
+      if (groups[i]) atomicAdd(&chunk_groups[q.order_block0 + i], groups[i]);
+  }
+}
+
+// Groups before every bitmap word: the groups of the query's earlier chunks
+// plus a block scan of this chunk's bit counts.  The query's last chunk
+// also knows its number of groups.
+__global__ void __launch_bounds__(kOrderThreads) BatchOrder(const QueryDesc* __restrict__ qs, int nq,
+                                                            const uint32_t* __restrict__ chunk_groups,
+                                                            FirstWord* __restrict__ first,
+                                                            unsigned long long* __restrict__ out_count) {
+  __shared__ int sq;
+  __shared__ uint32_t earlier[kOrderThreads / 32], wsum[kOrderThreads / 32];
+  if (threadIdx.x == 0) sq = FindQuery<3>(qs, nq, blockIdx.x);
+  __syncthreads();
+  const QueryDesc& q = qs[sq];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t e = 0;
+  for (int c = q.order_block0 + threadIdx.x; c < static_cast<int>(blockIdx.x); c += kOrderThreads) e += chunk_groups[c];
+  FirstWord* w = first + q.bit_base + static_cast<int64_t>(blockIdx.x - q.order_block0) * kOrderWords + 4 * threadIdx.x;
+  uint4* v = reinterpret_cast<uint4*>(w);  // two words each
+  uint4 a = v[0], b = v[1];
+  const uint32_t c0 = __popc(a.x), c1 = __popc(a.z), c2 = __popc(b.x), c3 = __popc(b.z);
+  const uint32_t mine = c0 + c1 + c2 + c3;
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+    e += __shfl_xor_sync(0xffffffffu, e, o);
+  }
+  if (lane == 31) wsum[warp] = incl;
+  if (lane == 0) earlier[warp] = e;
+  __syncthreads();
+  uint32_t run = incl - mine;
+  for (int k = 0; k < kOrderThreads / 32; k++) run += earlier[k] + (k < warp ? wsum[k] : 0u);
+  a.y = run;
+  a.w = run + c0;
+  b.y = run + c0 + c1;
+  b.w = run + c0 + c1 + c2;
+  v[0] = a;
+  v[1] = b;
+  if (threadIdx.x == kOrderThreads - 1 && static_cast<int>(blockIdx.x) == q.order_block0 + q.order_blocks - 1)
+    out_count[sq] = run + mine;
+}
+
+// Every group to its place among its query's groups.
 __global__ void BatchOutput(const QueryDesc* __restrict__ qs, int nq, const Acc* __restrict__ acc,
-                            int32_t* __restrict__ out_key, double* __restrict__ out_sum,
-                            unsigned long long* __restrict__ out_first, unsigned long long* __restrict__ out_count) {
+                            const FirstWord* __restrict__ first, int32_t* __restrict__ out_key,
+                            double* __restrict__ out_sum) {
   int64_t r0, r1;
   const QueryDesc& q = Chunk<2>(qs, nq, r0, r1);
-  const int qi = static_cast<int>(&q - qs);
-  const unsigned lane = threadIdx.x & 31;
-  for (int64_t rb = r0; rb < r1; rb += blockDim.x) {  // uniform trip count per warp
-    const int64_t r = rb + threadIdx.x;
-    Acc a{0.0, 0ULL};
-    if (r < r1) a = acc[q.acc_base + r];
-    const bool hit = a.first_inv != 0;
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if (m == 0) continue;
-    unsigned long long o0 = 0;
-    if (lane == 0) o0 = atomicAdd(out_count + qi, static_cast<unsigned long long>(__popc(m)));
-    o0 = __shfl_sync(0xffffffffu, o0, 0);
-    if (hit) {
-      const int64_t o = q.out_base + static_cast<int64_t>(o0) + __popc(m & ((1u << lane) - 1));
-      out_key[o] = q.d_key[r];
-      out_sum[o] = a.sum;
-      out_first[o] = ~a.first_inv;
+  const int64_t step = blockDim.x;
+  for (int64_t base = r0 + threadIdx.x; base < r1; base += kDimUnroll * step) {
+    Acc a[kDimUnroll];
+    FirstWord w[kDimUnroll];
+#pragma unroll
+    for (int j = 0; j < kDimUnroll; j++) {
+      a[j] = Acc{0.0, 0ULL};
+      if (base + j * step < r1) a[j] = acc[q.acc_base + base + j * step];
+    }
+#pragma unroll
+    for (int j = 0; j < kDimUnroll; j++)
+      w[j] = a[j].first_inv ? first[q.bit_base + static_cast<int64_t>(~a[j].first_inv >> 5)] : FirstWord{0, 0};
+#pragma unroll
+    for (int j = 0; j < kDimUnroll; j++) {
+      if (a[j].first_inv == 0) continue;
+      const unsigned bit = static_cast<unsigned>(~a[j].first_inv) & 31u;
+      const int64_t o = q.out_base + w[j].before + __popc(w[j].bits & ((1u << bit) - 1));
+      out_key[o] = q.d_key[base + j * step];
+      out_sum[o] = a[j].sum;
     }
   }
 }
@@ -280,7 +375,7 @@ class Batch {
     const int parts = 1 << fbits;
     const int nq = static_cast<int>(host_qs_.size());
     const int64_t chunk = static_cast<int64_t>(cfg.block) * kRowsPerThread;
-    int64_t bb = 0, pb = 0, ob = 0;
+    int64_t bb = 0, pb = 0, ob = 0, rb = 0;
     for (auto& q : host_qs_) {
       if (q.nd >= static_cast<int64_t>(UINT32_MAX))
         throw Error(KDB_ERR_CAPACITY, "batch dimension table too large");
@@ -294,11 +389,17 @@ class Batch {
       q.out_block0 = static_cast<int32_t>(ob);
       q.out_blocks = static_cast<int32_t>(blocks(q.nd));
       ob += q.out_blocks;
+      q.order_block0 = static_cast<int32_t>(rb);
+      q.order_blocks = static_cast<int32_t>(
+          std::max<int64_t>(1, (q.nf + 32 * kOrderWords - 1) / (32 * static_cast<int64_t>(kOrderWords))));
+      q.bit_base = rb * kOrderWords;
+      rb += q.order_blocks;
       if (bb > INT_MAX || pb > INT_MAX) throw Error(KDB_ERR_CAPACITY, "batch too large");
     }
     build_grid_ = static_cast<int>(bb);
     probe_grid_ = static_cast<int>(pb);
     out_grid_ = static_cast<int>(ob);
+    order_grid_ = static_cast<int>(rb);
     KDB_CUDA(cudaMalloc(&d_qs_, sizeof(QueryDesc) * nq));
     KDB_CUDA(cudaMemcpy(d_qs_, host_qs_.data(), sizeof(QueryDesc) * nq, cudaMemcpyHostToDevice));
     // largest sub-table population per query (all dimension rows, so it
@@ -341,16 +442,20 @@ class Batch {
     KDB_CUDA(cudaMalloc(&acc_, sizeof(Acc) * acc_total));
     KDB_CUDA(cudaMalloc(&out_key_, sizeof(int32_t) * acc_total));
     KDB_CUDA(cudaMalloc(&out_sum_, sizeof(double) * acc_total));
-    KDB_CUDA(cudaMalloc(&out_first_, sizeof(unsigned long long) * acc_total));
-    KDB_CUDA(cudaMalloc(&out_count_, sizeof(unsigned long long) * nq));
-    KDB_CUDA(cudaMalloc(&err_, sizeof(int)));
+    KDB_CUDA(cudaMalloc(&first_, sizeof(FirstWord) * kOrderWords * order_grid_));
+    KDB_CUDA(cudaMalloc(&chunk_groups_, sizeof(uint32_t) * order_grid_));
+    // the error word and every query's group count come back together
+    KDB_CUDA(cudaMalloc(&status_, StatusBytes()));
+    if (!host_block_) host_block_ = ctx_.AcquireHostBlock(StatusBytes());
+    host_status_ = reinterpret_cast<unsigned long long*>(host_block_.get());
+    std::memset(host_status_, 0, StatusBytes());
     Capture();
   }
 
   // Replays the batch (all phases of all queries).
   void Run() {
     KDB_CUDA(cudaGraphLaunch(exec_, ctx_.stream));
-    ctx_.kernel_launches += 3;
+    ctx_.kernel_launches += 5;
   }
 
   float RunTimed(int reps) {
@@ -369,37 +474,22 @@ class Batch {
     return ms / reps;
   }
 
-  int CheckError() {
-    int e = 0;
-    KDB_CUDA(cudaMemcpyAsync(&e, err_, sizeof(int), cudaMemcpyDeviceToHost, ctx_.stream));
-    KDB_CUDA(cudaStreamSynchronize(ctx_.stream));
-    return e;
-  }
+  // The error word of the last run (which has been waited for).
+  int CheckError() const { return static_cast<int>(host_status_[0]); }
 
   // Result of query q: groups in first-match order of the fact stream.
-  void Result(int q, std::vector<int32_t>& keys, std::vector<double>& sums) {
-    unsigned long long n = 0;
-    KDB_CUDA(cudaMemcpyAsync(&n, out_count_ + q, sizeof(n), cudaMemcpyDeviceToHost, ctx_.stream));
+  // Copies at most `cap` groups into the arrays given; returns their number.
+  int64_t Result(int q, int32_t* keys, double* sums, int64_t cap) {
     KDB_CUDA(cudaStreamSynchronize(ctx_.stream));
-    const QueryDesc& d = host_qs_[q];
-    std::vector<int32_t> k(n);
-    std::vector<double> s(n);
-    std::vector<unsigned long long> f(n);
-    if (n) {
-      KDB_CUDA(cudaMemcpyAsync(k.data(), out_key_ + d.out_base, 4 * n, cudaMemcpyDeviceToHost, ctx_.stream));
-      KDB_CUDA(cudaMemcpyAsync(s.data(), out_sum_ + d.out_base, 8 * n, cudaMemcpyDeviceToHost, ctx_.stream));
-      KDB_CUDA(cudaMemcpyAsync(f.data(), out_first_ + d.out_base, 8 * n, cudaMemcpyDeviceToHost, ctx_.stream));
-      KDB_CUDA(cudaStreamSynchronize(ctx_.stream));
-    }
-    std::vector<size_t> order(n);
-    for (size_t i = 0; i < n; i++) order[i] = i;
-    std::sort(order.begin(), order.end(), [&](size_t a, size_t b) { return f[a] < f[b]; });
-    keys.resize(n);
-    sums.resize(n);
-    for (size_t i = 0; i < n; i++) {
-      keys[i] = k[order[i]];
-      sums[i] = s[order[i]];
-    }
+    const int64_t n = static_cast<int64_t>(host_status_[1 + q]);
+    const int64_t base = host_qs_[q].out_base, m = std::min(n, cap);
+    if (m <= 0) return n;
+    if (keys)
+      KDB_CUDA(cudaMemcpyAsync(keys, out_key_ + base, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, ctx_.stream));
+    if (sums)
+      KDB_CUDA(cudaMemcpyAsync(sums, out_sum_ + base, sizeof(double) * m, cudaMemcpyDeviceToHost, ctx_.stream));
+    KDB_CUDA(cudaStreamSynchronize(ctx_.stream));
+    return n;
   }
 
   const BatchConfig& config() const { return cfg_; }
@@ -422,48 +512,60 @@ class Batch {
     KDB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(slots_, 0, sizeof(unsigned long long) * std::max<int64_t>(slot_total_, 1), s);
     cudaMemsetAsync(acc_, 0, sizeof(Acc) * acc_total_, s);
-    cudaMemsetAsync(out_count_, 0, sizeof(unsigned long long) * nq, s);
-    cudaMemsetAsync(err_, 0, sizeof(int), s);
-    BatchBuild<<<build_grid_, cfg_.block, 0, s>>>(d_qs_, nq, slots_, fanout_bits_, err_);
+    cudaMemsetAsync(first_, 0, sizeof(FirstWord) * kOrderWords * order_grid_, s);
+    cudaMemsetAsync(chunk_groups_, 0, sizeof(uint32_t) * order_grid_, s);
+    cudaMemsetAsync(status_, 0, StatusBytes(), s);
+    int* err = reinterpret_cast<int*>(status_);
+    BatchBuild<<<build_grid_, cfg_.block, 0, s>>>(d_qs_, nq, slots_, fanout_bits_, err);
     BatchProbe<<<probe_grid_, cfg_.block, 0, s>>>(d_qs_, nq, slots_, fanout_bits_, acc_,
                                                    ctx_.OptStr("KDB_BATCH_LAZY_MEASURES") ? 0 : 1);
-    BatchOutput<<<out_grid_, cfg_.block, 0, s>>>(d_qs_, nq, acc_, out_key_, out_sum_, out_first_, out_count_);
+    BatchMark<<<out_grid_, cfg_.block, 0, s>>>(d_qs_, nq, acc_, first_, chunk_groups_);
+    BatchOrder<<<order_grid_, kOrderThreads, 0, s>>>(d_qs_, nq, chunk_groups_, first_, status_ + 1);
+    BatchOutput<<<out_grid_, cfg_.block, 0, s>>>(d_qs_, nq, acc_, first_, out_key_, out_sum_);
+    cudaMemcpyAsync(host_status_, status_, StatusBytes(), cudaMemcpyDeviceToHost, s);
     cudaGraph_t g;
     KDB_CUDA(cudaStreamEndCapture(s, &g));
     KDB_CUDA(cudaGraphInstantiate(&exec_, g, 0));
     cudaGraphDestroy(g);
   }
 
+  size_t StatusBytes() const { return sizeof(unsigned long long) * (host_qs_.size() + 1); }
+
   void Release() {
     if (exec_) cudaGraphExecDestroy(exec_);
     exec_ = nullptr;
     for (void* p : {static_cast<void*>(d_qs_), static_cast<void*>(slots_), static_cast<void*>(acc_),
-                    static_cast<void*>(out_key_), static_cast<void*>(out_sum_), static_cast<void*>(out_first_),
-                    static_cast<void*>(out_count_), static_cast<void*>(err_)})
+                    static_cast<void*>(out_key_), static_cast<void*>(out_sum_), static_cast<void*>(first_),
+                    static_cast<void*>(chunk_groups_), static_cast<void*>(status_)})
       if (p) cudaFree(p);
     d_qs_ = nullptr;
     slots_ = nullptr;
     acc_ = nullptr;
-    out_first_ = out_count_ = nullptr;
+    first_ = nullptr;
+    chunk_groups_ = nullptr;
+    status_ = nullptr;
     out_key_ = nullptr;
     out_sum_ = nullptr;
-    err_ = nullptr;
   }
 
   Context& ctx_;
   std::vector<QueryDesc> host_qs_;
   BatchConfig cfg_;
   int fanout_bits_ = 0;
-  int build_grid_ = 0, probe_grid_ = 0, out_grid_ = 0;
+  int build_grid_ = 0, probe_grid_ = 0, out_grid_ = 0, order_grid_ = 0;
   int64_t slot_total_ = 0, acc_total_ = 0;
   QueryDesc* d_qs_ = nullptr;
   unsigned long long* slots_ = nullptr;
   Acc* acc_ = nullptr;
   int32_t* out_key_ = nullptr;
   double* out_sum_ = nullptr;
-  unsigned long long* out_first_ = nullptr;
-  unsigned long long* out_count_ = nullptr;
-  int* err_ = nullptr;
+  FirstWord* first_ = nullptr;
+  uint32_t* chunk_groups_ = nullptr;
+  // the error word, then one group count per query; the graph ends by
+  // copying them to host_status_ (in a pinned block of the context's pool)
+  unsigned long long* status_ = nullptr;
+  unsigned long long* host_status_ = nullptr;
+  std::shared_ptr<char> host_block_;
   cudaGraphExec_t exec_ = nullptr;
 };
 
@@ -603,14 +705,7 @@ int64_t kdb_batch_result(kdb_batch* b, int32_t q, int32_t* keys, double* sums, i
   if (!b || q < 0 || q >= b->b->num_queries()) return KDB_ERR_INVALID;
   int64_t n = -1;
   int rc = BGuard(b->owner, [&] {
-    std::vector<int32_t> k;
-    std::vector<double> s;
-    b->b->Result(q, k, s);
-    n = static_cast<int64_t>(k.size());
-    for (int64_t i = 0; i < std::min<int64_t>(n, cap); i++) {
-      if (keys) keys[i] = k[i];
-      if (sums) sums[i] = s[i];
-    }
+    n = b->b->Result(q, keys, sums, cap);
   });
   return rc == KDB_OK ? n : rc;
 }

@@ -84,3 +84,20 @@ def test_batch_rejects_non_unique_dimension_keys():
         b.run()
     b.close()
     e.close()
+
+
+# the group order's edges: one bitmap word (32 fact rows), one order chunk
+# (32768 fact rows), several chunks with a partial last one
+@pytest.mark.parametrize("facts", [1, 31, 32, 33, 32_767, 32_768, 32_769, 65_537, 300_001])
+def test_batch_group_order_at_bitmap_edges(facts):
+    from kushdb_b200.engine import Batch, Engine
+    with Engine(0) as e:
+        qs = [wl.batch_tables(n_queries=1, min_fact=n + 0.5, max_fact=n + 0.5, seed=n, prefix=f"be{i}_")[0]
+              for i, n in enumerate((facts, 1000, facts))]
+        for d, f, _, _ in qs:
+            e.register_table(d)
+            e.register_table(f)
+        b = Batch(e, [wl.batch_query_desc(*q) for q in qs])
+        _check_against_plain(e, b, qs)
+        _check_against_plain(e, b, qs)  # a second run of the same graph
+        b.close()
