@@ -149,6 +149,25 @@ struct PackSegs {
   int n = 0;
 };
 
+// Join indexes grouped together (Executor::BuildGroupedIndexes): per index
+// the table of distinct hashes with the groups' lengths, every row's {slot,
+// place in its group} (slot ~0: left out), and where the rows go.
+constexpr int kMaxIndexBatch = 16;
+constexpr int kIndexRows = 1024;  // rows per CTA of the counting and filling kernels
+struct IndexBuild {
+  uint64_t* slots;
+  uint32_t* lens;
+  uint2* place;
+  uint32_t* srow;
+  unsigned long long* used;  // rows of the groups laid out so far
+  int64_t cap;               // slots
+  int64_t n;                 // rows
+};
+struct IndexBatch {
+  IndexBuild index[kMaxIndexBatch];
+  int n = 0;
+};
+
 // The device work of one query execution, kept to be replayed as a CUDA
 // graph when the same plan runs again over unchanged tables.
 struct Recorder {
@@ -373,6 +392,8 @@ class Context {
   // device), no pass computes it.
   bool RangeSortItems(void* items, int64_t n, Arena& arena, unsigned long long* ties = nullptr,
                       uint32_t tie_mask = 0, const unsigned long long* key_range = nullptr);
+  // lays out the groups counted in every index of `b` and fills their rows
+  void GroupIndexRows(const IndexBatch& b);
   // exclusive prefix sum of a[0..n) in place, the total into a[n]
   void ScanU64(uint64_t* a, int64_t n, const char* tag = "skinner scan");
   // the same over *n_ptr elements (a device word), skipped when *n_ptr > cap

@@ -553,6 +553,114 @@ __global__ void KdbTextGather(const char* __restrict__ raw, int64_t n, const int
 }  // namespace
 
 namespace {
+
+// Where CTA `block` works in a batch of indexes, each taking `units` / `per`
+// CTAs: the index, and the CTA's number within it.
+template <typename UNITS>
+__device__ __forceinline__ int IndexOfBlock(const IndexBatch& b, int64_t block, int64_t per, UNITS units,
+                                            int64_t* within) {
+  int j = 0;
+  for (; j + 1 < b.n; j++) {
+    const int64_t c = (units(b.index[j]) + per - 1) / per;
+    if (block < c) break;
+    block -= c;
+  }
+  *within = block;
+  return j;
+}
+
+constexpr int kPlaceSlots = 4096;  // slots per CTA
+
+// Every group its place among its index's rows: the groups of a CTA's slots
+// are laid out next to each other, one atomic per CTA (the order of the
+// groups does not matter).  Reads 4 bytes per slot; only occupied slots are
+// read and written whole.
+__global__ void __launch_bounds__(256) PlaceIndexGroups(const __grid_constant__ IndexBatch b) {
+  __shared__ unsigned ws[8];
+  __shared__ unsigned long long base;
+  int64_t within;
+  const IndexBuild& x =
+      b.index[IndexOfBlock(b, blockIdx.x, kPlaceSlots, [](const IndexBuild& i) { return i.cap; }, &within)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t s0 = within * kPlaceSlots;
+  uint4 len[4];
+  unsigned mine = 0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int64_t s = s0 + 4 * (q * 256 + threadIdx.x);  // capacities are multiples of 1024
+    len[q] = s < x.cap ? *reinterpret_cast<const uint4*>(x.lens + s) : make_uint4(0, 0, 0, 0);
+    mine += len[q].x + len[q].y + len[q].z + len[q].w;
+  }
+  unsigned incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) ws[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned total = 0;
+    for (int w = 0; w < 8; w++) total += ws[w];
+    base = total ? atomicAdd(x.used, static_cast<unsigned long long>(total)) : 0ULL;
+  }
+  __syncthreads();
+  unsigned run = static_cast<unsigned>(base) + incl - mine;
+  for (int w = 0; w < warp; w++) run += ws[w];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int64_t s = s0 + 4 * (q * 256 + threadIdx.x);
+    const unsigned l[4] = {len[q].x, len[q].y, len[q].z, len[q].w};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (l[k]) {
+        x.slots[s + k] = (x.slots[s + k] & 0xffffffff00000000ULL) | (run + 1u);
+        run += l[k];
+      }
+  }
+}
+
+__global__ void __launch_bounds__(256) FillIndexRows(const __grid_constant__ IndexBatch b) {
+  int64_t within;
+  const IndexBuild& x =
+      b.index[IndexOfBlock(b, blockIdx.x, kIndexRows, [](const IndexBuild& i) { return i.n; }, &within)];
+  static_assert(kIndexRows == 4 * 256, "four rows per thread");
+  uint2 p[4];
+  unsigned first[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const int64_t r = within * kIndexRows + u * 256 + threadIdx.x;
+    p[u] = r < x.n ? x.place[r] : make_uint2(~0u, 0u);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u++) first[u] = p[u].x != ~0u ? static_cast<unsigned>(x.slots[p[u].x]) : 0u;
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+    if (p[u].x != ~0u)
+      x.srow[first[u] - 1u + p[u].y] = static_cast<uint32_t>(within * kIndexRows + u * 256 + threadIdx.x);
+}
+
+}  // namespace
+
+void Context::GroupIndexRows(const IndexBatch& b) {
+  if (dry) return;
+  int64_t place = 0, fill = 0;
+  for (int j = 0; j < b.n; j++) {
+    place += (b.index[j].cap + kPlaceSlots - 1) / kPlaceSlots;
+    fill += (b.index[j].n + kIndexRows - 1) / kIndexRows;
+  }
+  if (fill == 0) return;
+  const IndexBatch batch = b;
+  TimedStart("index groups");
+  Issue([=](cudaStream_t s) { PlaceIndexGroups<<<static_cast<unsigned>(place), 256, 0, s>>>(batch); });
+  TimedStop();
+  TimedStart("index rows");
+  Issue([=](cudaStream_t s) { FillIndexRows<<<static_cast<unsigned>(fill), 256, 0, s>>>(batch); });
+  TimedStop();
+  KDB_CUDA(cudaGetLastError());
+}
+
+namespace {
 __global__ void SpinDelay(long long cycles) {
   const long long t0 = clock64();
   while (clock64() - t0 < cycles) {

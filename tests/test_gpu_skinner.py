@@ -121,3 +121,55 @@ def test_episode_batches_keep_the_result(engine, batch, policy):
         assert batches == episodes
     elif episodes > 4 * batch:
         assert batches < episodes
+
+
+# the grouped indexes' edges: one row, a CTA's rows (1024) and one more or
+# less, several CTAs; unique keys, few keys, one key for every row, NULL keys
+@pytest.mark.parametrize("rows", [1, 2, 1023, 1024, 1025, 40_003])
+@pytest.mark.parametrize("keys", ["unique", "few", "one", "null"])
+def test_grouped_index_edges_match_oracle(engine, rows, keys):
+    import numpy as np
+    from kushdb_b200.data import HostColumn, HostTable, catalog_of
+    from kushdb_b200.plan import (AggregateOperator, ColRef, Count, Eq, Max, OperatorSchema, OutputOperator,
+                                  ScanOperator, SkinnerJoinOperator, Sum, Type, VirtColRef)
+    from oracle import Oracle
+    rng = np.random.default_rng(rows)
+    n_b = 700
+    k = {"unique": rng.permutation(rows), "few": rng.integers(0, 5, rows), "one": np.full(rows, 3),
+         "null": rng.integers(0, 50, rows)}[keys].astype(np.int32)
+    nulls = (rng.random(rows) < 0.5).astype(np.int8) if keys == "null" else None
+    a = HostTable(f"ix_a_{rows}_{keys}")
+    a.add(HostColumn("k", Type.Int(), values=k, nulls=nulls))
+    a.add(HostColumn("v", Type.Int(), values=rng.integers(0, 1000, rows).astype(np.int32)))
+    b = HostTable(f"ix_b_{rows}_{keys}")
+    b.add(HostColumn("k", Type.Int(), values=rng.integers(0, 60, n_b).astype(np.int32)))
+    b.add(HostColumn("g", Type.BigInt(), values=rng.integers(0, 20, n_b)))
+    c = HostTable(f"ix_c_{rows}_{keys}")
+    c.add(HostColumn("g", Type.BigInt(), values=np.arange(25)))
+    tables = [a, b, c]
+    db = catalog_of(tables)
+    scans = []
+    for t in tables:
+        s = OperatorSchema()
+        s.AddGeneratedColumns(db[t.name], list(t.columns))
+        scans.append(ScanOperator(s, db[t.name]))
+    js = OperatorSchema()
+    js.AddPassthroughColumns(scans[0], ["v"], 0)
+    js.AddPassthroughColumns(scans[2], ["g"], 2)
+    join = SkinnerJoinOperator(js, scans, [Eq(ColRef(scans[0], "k", 0), ColRef(scans[1], "k", 1)),
+                                           Eq(ColRef(scans[1], "g", 1), ColRef(scans[2], "g", 2))])
+    aggs = [Count(), Sum(ColRef(join, "v")), Max(ColRef(join, "g"))]
+    out = OperatorSchema()
+    for i, name in enumerate(("n", "total", "most")):
+        out.AddDerivedColumn(name, VirtColRef(aggs[i], i))
+    plan = OutputOperator(AggregateOperator(out, join, aggs))
+    o = Oracle()
+    for t in tables:
+        engine.register_table(t)
+        o.register_table(t)
+    engine.set_skinner(5000, seed=1)
+    try:
+        g = engine.execute(plan)
+    finally:
+        engine.set_skinner()
+    assert compare(g, o.execute(plan)) == ""
