@@ -722,6 +722,12 @@ class Executor {
     return static_cast<int64_t>(h);
   }
 
+  // A device counter and the device error word in one round trip.
+  int64_t ReadU64Checked(const uint64_t* d, const char* what) {
+    if (ctx_.dry) return 2;
+    return static_cast<int64_t>(ctx_.ReadWordChecked(d, what));
+  }
+
   MatBuffer AllocMat(const std::vector<SchemaCol>& schema, int64_t cap) {
     MatBuffer m;
     m.cap = std::max<int64_t>(cap, 1);
@@ -801,6 +807,7 @@ class Executor {
   MatBuffer RunGroupBy(const Operator& op, bool any_order = false, const Operator* order_by = nullptr);
   MatBuffer RunOrderBy(const Operator& op);
   MatBuffer RunSkinner(const Operator& op, const SkinnerAgg* agg = nullptr);
+  MatBuffer SkinnerRows(const Operator& child);
   MatBuffer SmallOrderBy(const Operator& op, MatBuffer& m);
   MatBuffer LargeOrderBy(const Operator& op, MatBuffer& m);
   // Returns true when it also counted ties into *ties (range sort taken).
@@ -1932,8 +1939,7 @@ MatBuffer Executor::MaterializeStream(const Operator& op, const uint32_t* order,
     int64_t src_rows = 0;
     EmitStream(ks, eg, op, sink, src_rows);
     LaunchPipeline(ks, src_rows, "materialize");
-    int64_t produced = ReadU64(counter);
-    ctx_.CheckDeviceError("materialize");
+    int64_t produced = ReadU64Checked(counter, "materialize");
     if (produced <= out.cap) {
       out.rows = produced;
       return out;
@@ -1974,8 +1980,7 @@ MatBuffer Executor::MaterializeCounted(const Operator& op, const std::function<v
   kc.L("if (threadIdx.x == 0) " + offp + "[blockIdx.x] = kdb_block_rows;");
   LaunchPipeline(kc, src_rows, "materialize count", block);
   ctx_.ScanU64(offsets, grid, "materialize offsets");
-  const int64_t produced = ReadU64(offsets + grid);
-  ctx_.CheckDeviceError("materialize");
+  const int64_t produced = ReadU64Checked(offsets + grid, "materialize");
   if (on_count) on_count(produced);
 
   KernelSource ks;
@@ -4283,12 +4288,11 @@ class SkinnerEngine : public JoinEnv {
     } else {
       out_ = alloc_out_(1 << 12);
     }
-    // result count, work, the two task queues' counts, then per episode of
+    // result count, a spare word, the two task queues' counts, then per episode of
     // a batch its results and its work (all read back together)
     stats_ = arena_.AllocT<uint64_t>(4 + 2 * kMaxBatch);
     ctx_.Memset(stats_, 0, (4 + 2 * kMaxBatch) * sizeof(uint64_t));
     count_ = stats_;
-    work_ = stats_ + 1;
     tcount_ = stats_ + 2;
     eres_ = stats_ + 4;
     ework_ = stats_ + 4 + kMaxBatch;
@@ -4536,10 +4540,8 @@ class SkinnerEngine : public JoinEnv {
       Grow(total);  // the batch reruns into the larger buffer
       uint64_t keep = static_cast<uint64_t>(produced_);
       ctx_.H2D(count_, &keep, sizeof(uint64_t));
-      ctx_.Memset(work_, 0, sizeof(uint64_t));
       ctx_.Memset(eres_, 0, sizeof(uint64_t) * 2 * K);
     }
-    ctx_.Memset(work_, 0, sizeof(uint64_t));
     ctx_.Memset(eres_, 0, sizeof(uint64_t) * 2 * K);
     // per episode: reward, and the next slice size of its leftmost table
     // so its work matches the budget
@@ -4595,9 +4597,33 @@ class SkinnerEngine : public JoinEnv {
     for (int t = 0; t < T; t++) ks.L("card[" + std::to_string(t) + "] = (int64_t)" + ks.Word(static_cast<uint64_t>(cards_[t])) + ";");
     ks.L("const int nep = (int)a.w[" + std::to_string(w_nep_) + "];");
     ks.L("const int64_t S = (int64_t)a.w[" + std::to_string(w_total_) + "];");
+    // tuples examined and results per episode of the batch: a thread counts
+    // its current episode's in registers, adds them to its CTA's shared
+    // counters when it moves to another episode, and the CTA adds those to
+    // the device counters once at its end (one atomic per thread on those few
+    // words queued for about 300 us per launch)
+    ks.L("__shared__ unsigned long long kdb_swk[" + KB + "], kdb_snres[" + KB + "];");
+    ks.L("for (int e = threadIdx.x; e < " + KB + "; e += blockDim.x) { kdb_swk[e] = 0; kdb_snres[e] = 0; }");
+    if (agg_) {
+      // the CTA's aggregate state (layout of SkinnerAgg::state)
+      ks.L("__shared__ unsigned long long kdb_sfa[" + std::to_string(agg_->nw) + "];");
+      ks.Open("if (threadIdx.x == 0)");
+      for (int w = 0; w < agg_->nw; w++) {
+        const size_t j = static_cast<size_t>(w) / 2;
+        const bool min_word = w % 2 == 0 && j < agg_->plans->size() &&
+                              (*agg_->plans)[j].kind == StateKind::MinMaxKey && (*agg_->plans)[j].is_min;
+        ks.L("kdb_sfa[" + std::to_string(w) + "] = " + (min_word ? "~0ULL" : "0ULL") + ";");
+      }
+      ks.Close();
+    }
+    ks.L("__syncthreads();");
     ks.L("int cur_e = -1; int64_t s0 = 0, e_start = 0;");
+    ks.L("unsigned long long wk = 0, nres = 0;");
+    ks.L("auto flush_ep = [&]() { if (wk) atomicAdd(&kdb_swk[cur_e], wk); if (nres) atomicAdd(&kdb_snres[cur_e], nres); "
+         "wk = 0; nres = 0; };");
     ks.Open("auto use_ep = [&](int e)");
     ks.L("if (e == cur_e) return;");
+    ks.L("flush_ep();");
     ks.L("cur_e = e;");
     ks.L("const uint64_t* q = " + EP + " + (int64_t)e * " + EPW + ";");
     ks.L("for (int p = 0; p < " + TS + "; p++) { ord[p] = (int32_t)q[p]; lk[p] = (int32_t)(int64_t)q[" + TS +
@@ -4613,14 +4639,11 @@ class SkinnerEngine : public JoinEnv {
     ks.L("return e;");
     ks.indent--;
     ks.L("};");
-    // tuples examined and results, per episode of the batch
-    ks.L("unsigned long long wk[" + KB + "]; unsigned long long nres[" + KB + "];");
-    ks.L("for (int e = 0; e < " + KB + "; e++) { wk[e] = 0; nres[e] = 0; }");
     w_phase_ = ks.Arg(0);
     w_qin_ = ks.Arg(0);
     ks.L("int64_t rows[" + TS + "]; int64_t iti[" + TS + "]; int64_t ite[" + TS + "];");
     if (agg_) {
-      ks.L("unsigned long long fa_nres = 0; int64_t fa_rows = 0;");
+      ks.L("int64_t fa_rows = 0;");
       for (size_t j = 0; j < agg_->plans->size(); j++) {
         const AggPlan& p = (*agg_->plans)[j];
         const std::string J = std::to_string(j);
@@ -4744,7 +4767,7 @@ class SkinnerEngine : public JoinEnv {
         }
         ks.L("fa_c" + J + "++;");
       }
-      ks.L("fa_rows++; fa_nres++; nres[cur_e]++;");
+      ks.L("fa_rows++; nres++;");
       w_count_ = ks.Arg(0);
     } else {
       Scope sc;
@@ -4754,7 +4777,7 @@ class SkinnerEngine : public JoinEnv {
       for (const auto& c : op_.output) vals.push_back(eg.Emit(*c.expr, sc));
       int wc = ks.Arg(0);
       w_count_ = wc;
-      ks.L("nres[cur_e]++;");
+      ks.L("nres++;");
       ks.L("uint64_t slot = kdb_alloc_slot((unsigned long long*)a.w[" + std::to_string(wc) + "]);");
       ks.Open("if (slot < a.w[" + std::to_string(w_cap_) + "])");
       for (size_t c = 0; c < vals.size(); c++) {
@@ -4814,7 +4837,7 @@ class SkinnerEngine : public JoinEnv {
     ks.L("const int phase = (int)a.w[" + std::to_string(w_phase_) + "];");
     ks.Open("if (phase == 0)");
     ks.Open("for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < S; x += (int64_t)gridDim.x * blockDim.x)");
-    ks.L("use_ep(ep_of(x)); rows[ord[0]] = s0 + (x - e_start); wk[cur_e]++;");
+    ks.L("use_ep(ep_of(x)); rows[ord[0]] = s0 + (x - e_start); wk++;");
     if (T == 1) {
       ks.L("if (conds_ok(sched[0])) emit();");
     } else {
@@ -4841,7 +4864,7 @@ class SkinnerEngine : public JoinEnv {
       ks.L("use_ep(ep_of(lo)); rows[ord[0]] = s0 + (lo - e_start);");
       ks.L("const int64_t c1 = cand(1, (int64_t)(" + BG + "[lo] + (w - " + OF + "[lo])));");
       ks.L("if (c1 < 0 || c1 < off[ord[1]]) continue;");
-      ks.L("rows[ord[1]] = c1; wk[cur_e]++;");
+      ks.L("rows[ord[1]] = c1; wk++;");
       ks.L("if (!conds_ok(sched[1])) continue;");
       // depth-first over positions from..T-1, the earlier ones bound; with
       // `preset` position `from`'s run is already in [iti, ite) (a task);
@@ -4865,7 +4888,7 @@ class SkinnerEngine : public JoinEnv {
         ks.Close();
         ks.L("int t = ord[p];");
         ks.L("if (c < off[t]) continue;");
-        ks.L("rows[t] = c; wk[cur_e]++;");
+        ks.L("rows[t] = c; wk++;");
         ks.L("if (!conds_ok(sched[p])) continue;");
         ks.Open("if (p == " + std::to_string(T - 1) + ")");
         ks.L("emit();");
@@ -4907,7 +4930,7 @@ class SkinnerEngine : public JoinEnv {
         ks.L("use_ep(ep_of(lo)); rows[ord[0]] = s0 + (lo - e_start);");
         ks.L("const int64_t c1 = cand(1, (int64_t)(" + BG + "[lo] + (w - " + OF + "[lo])));");
         ks.Open("if (c1 >= 0 && c1 >= off[ord[1]])");
-        ks.L("rows[ord[1]] = c1; wk[cur_e]++;");
+        ks.L("rows[ord[1]] = c1; wk++;");
         ks.Open("if (conds_ok(sched[1]))");
         ks.Open("if (fits)");
         ks.L("init(2);");
@@ -4945,7 +4968,7 @@ class SkinnerEngine : public JoinEnv {
         ks.L("rows[ord[1]] = cand(1, (int64_t)(" + BG + "[lo] + (w - " + OF + "[lo])));");
         ks.L("const int64_t c2 = cand(2, (int64_t)(" + B2 + "[w] + (w2 - " + O2 + "[w])));");
         ks.L("if (c2 < 0 || c2 < off[ord[2]]) continue;");
-        ks.L("rows[ord[2]] = c2; wk[cur_e]++;");
+        ks.L("rows[ord[2]] = c2; wk++;");
         ks.L("if (!conds_ok(sched[2])) continue;");
         if (T == 3) ks.L("emit();");
         else depth_first("3", false, "0");
@@ -4954,48 +4977,67 @@ class SkinnerEngine : public JoinEnv {
         ks.Close();
       }
       if (split_) {
-        // Phase 4: the queued tasks of queue qin, one per thread, each
-        // continuing depth-first from its position; their hot runs go to
-        // the other queue
+        // Phase 4: the queued tasks of queue qin, the candidates of one
+        // shared by kTaskLanes threads, each continuing depth-first from its
+        // position; their hot runs go to the other queue
         ks.Open("else if (phase == 4)");
         ks.L("const int qi = (int)a.w[" + std::to_string(w_qin_) + "];");
         ks.L("const uint64_t nq = " + TC + "[qi];");
         ks.L("const uint64_t nt = nq < " + TCAP + " ? nq : " + TCAP + ";");
         ks.L("const uint64_t* tq = qi ? " + TQ1 + " : " + TQ0 + ";");
-        ks.Open("for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nt; w += (uint64_t)gridDim.x * blockDim.x)");
-        ks.L("const uint64_t* t = tq + w * " + TW + ";");
+        const std::string LANES = std::to_string(kTaskLanes);
+        ks.Open("for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nt * " + LANES +
+                "; w += (uint64_t)gridDim.x * blockDim.x)");
+        ks.L("const uint64_t* t = tq + w / " + LANES + " * " + TW + ";");
         ks.L("use_ep((int)t[3 + " + TS + "]);");
         ks.L("const int tp = (int)t[0];");
-        ks.L("iti[tp] = (int64_t)t[1]; ite[tp] = (int64_t)t[2];");
+        ks.L("const int64_t share = ((int64_t)(t[2] - t[1]) + " + LANES + " - 1) / " + LANES + ";");
+        ks.L("iti[tp] = (int64_t)t[1] + (int64_t)(w % " + LANES + ") * share; ite[tp] = iti[tp] + share;");
+        ks.L("if (ite[tp] > (int64_t)t[2]) ite[tp] = (int64_t)t[2];");
         ks.L("for (int k = 0; k < " + TS + "; k++) rows[k] = (int64_t)t[3 + k];");
         depth_first("tp", true, "1 - qi");
         ks.Close();
         ks.Close();
       }
     }
-    {
-      const std::string WT = ks.Ptr(work_, "unsigned long long");
-      const std::string ER = ks.Ptr(eres_, "unsigned long long"), EW = ks.Ptr(ework_, "unsigned long long");
-      ks.Open("for (int e = 0; e < nep; e++)");
-      ks.L("if (wk[e]) { atomicAdd(&" + EW + "[e], wk[e]); atomicAdd(" + WT + ", wk[e]); }");
-      ks.L("if (nres[e]) atomicAdd(&" + ER + "[e], nres[e]);");
-      ks.Close();
-    }
+    ks.L("flush_ep();");
     if (agg_) {
-      std::string ST = ks.Ptr(agg_->state, "unsigned long long");
       ks.Open("if (fa_rows)");
       for (size_t j = 0; j < agg_->plans->size(); j++) {
         const AggPlan& p = (*agg_->plans)[j];
         const std::string J = std::to_string(j), V = std::to_string(2 * j), C = std::to_string(2 * j + 1);
         if (p.kind == StateKind::MinMaxKey)
-          ks.L(std::string(p.is_min ? "atomicMin" : "atomicMax") + "(&" + ST + "[" + V + "], (unsigned long long)fa_v" +
-               J + ");");
+          ks.L(std::string(p.is_min ? "atomicMin" : "atomicMax") + "(&kdb_sfa[" + V + "], (unsigned long long)fa_v" + J + ");");
         else if (p.kind == StateKind::SumI64)
-          ks.L("atomicAdd(&" + ST + "[" + V + "], (unsigned long long)fa_v" + J + ");");
-        ks.L("atomicAdd(&" + ST + "[" + C + "], (unsigned long long)fa_c" + J + ");");
+          ks.L("atomicAdd(&kdb_sfa[" + V + "], (unsigned long long)fa_v" + J + ");");
+        ks.L("atomicAdd(&kdb_sfa[" + C + "], (unsigned long long)fa_c" + J + ");");
       }
-      ks.L("atomicAdd(&" + ST + "[" + std::to_string(agg_->nw - 2) + "], (unsigned long long)fa_rows);");
-      ks.L("atomicAdd((unsigned long long*)a.w[" + std::to_string(w_count_) + "], fa_nres);");
+      ks.L("atomicAdd(&kdb_sfa[" + std::to_string(agg_->nw - 2) + "], (unsigned long long)fa_rows);");
+      ks.Close();
+    }
+    ks.L("__syncthreads();");
+    {
+      const std::string ER = ks.Ptr(eres_, "unsigned long long"), EW = ks.Ptr(ework_, "unsigned long long");
+      ks.Open("for (int e = threadIdx.x; e < nep; e += blockDim.x)");
+      ks.L("if (kdb_swk[e]) atomicAdd(&" + EW + "[e], kdb_swk[e]);");
+      ks.L("if (kdb_snres[e]) atomicAdd(&" + ER + "[e], kdb_snres[e]);");
+      ks.Close();
+    }
+    if (agg_) {
+      std::string ST = ks.Ptr(agg_->state, "unsigned long long");
+      const std::string R = std::to_string(agg_->nw - 2);
+      ks.Open("if (threadIdx.x == 0 && kdb_sfa[" + R + "])");
+      for (size_t j = 0; j < agg_->plans->size(); j++) {
+        const AggPlan& p = (*agg_->plans)[j];
+        const std::string V = std::to_string(2 * j), C = std::to_string(2 * j + 1);
+        if (p.kind == StateKind::MinMaxKey)
+          ks.L(std::string(p.is_min ? "atomicMin" : "atomicMax") + "(&" + ST + "[" + V + "], kdb_sfa[" + V + "]);");
+        else if (p.kind == StateKind::SumI64)
+          ks.L("atomicAdd(&" + ST + "[" + V + "], kdb_sfa[" + V + "]);");
+        ks.L("atomicAdd(&" + ST + "[" + C + "], kdb_sfa[" + C + "]);");
+      }
+      ks.L("atomicAdd(&" + ST + "[" + R + "], kdb_sfa[" + R + "]);");
+      ks.L("atomicAdd((unsigned long long*)a.w[" + std::to_string(w_count_) + "], kdb_sfa[" + R + "]);");
       ks.Close();
     }
     std::string src = ks.Kernel("kdb_skinner_episode", 128);
@@ -5075,16 +5117,21 @@ class SkinnerEngine : public JoinEnv {
   MatBuffer out_;
   uint64_t* stats_ = nullptr;
   uint64_t* count_ = nullptr;
-  uint64_t* work_ = nullptr;
   // Hot runs: a depth-first walk that meets a candidate run longer than
   // split_run_ at position 3 or deeper pushes it, in chunks of split_run_,
   // as tasks {position, begin, end, bound rows} to a queue instead of
   // walking it alone; the host then runs the queued tasks grid-wide (their
   // own hot runs go to the other queue) until both are empty.  A full queue
-  // leaves the run to the thread that met it.
+  // leaves the run to the thread that met it.  A candidate costs its thread
+  // about a microsecond of dependent loads and a round of tasks about 25 us,
+  // so runs split early and kTaskLanes threads share a task: on a Zipf 1.5
+  // chain of 8 tables (200k rows) 1.2 ms with chunks of 32, 1.6 with 128, 2.2
+  // to 3.6 with 512; one thread per task of up to 1024 took 2.2 ms for one
+  // round of tasks.
   bool split_ = false;
-  int64_t split_run_ = 1024;
-  int64_t task_cap_ = 1 << 16;
+  static constexpr int kTaskLanes = 16;
+  int64_t split_run_ = 32;
+  int64_t task_cap_ = 1 << 18;
   uint64_t* tasks_[2] = {nullptr, nullptr};
   uint64_t* tcount_ = nullptr;
   int w_qin_ = 0;
@@ -5117,6 +5164,40 @@ class SkinnerEngine : public JoinEnv {
   uint64_t* offs_ = nullptr;  // per slice tuple: candidate count, then its exclusive prefix
   std::vector<int> out_ptr_words_;
 };
+
+// The rows of a Skinner child.  An unfiltered scan that passes base columns
+// through is its table: the join then reads the resident columns (rows in
+// table order) instead of a copy, which cost three launches and two round
+// trips per table.  TEXT columns are stored differently in a buffer, and a
+// column whose NULLs the schema does not announce (or the reverse) is left to
+// the scan's own rules.
+MatBuffer Executor::SkinnerRows(const Operator& child) {
+  const bool scan = child.kind == OpKind::SCAN || (child.kind == OpKind::SCAN_SELECT && child.filters.empty());
+  auto it = scan ? ctx_.tables.find(child.relation) : ctx_.tables.end();
+  if (it == ctx_.tables.end() || child.output.empty()) return Materialize(child);
+  for (const auto& sc : child.scan_columns)
+    if (ctx_.Column(child.relation, sc.name).type.id != sc.type.id) return Materialize(child);
+  MatBuffer m;
+  m.rows = m.cap = std::max<int64_t>(it->second.rows, 0);
+  m.pos_is_index = true;
+  for (const auto& c : child.output) {
+    const Expr& e = *c.expr;
+    const bool direct = child.kind == OpKind::SCAN ? e.kind == ExprKind::ColRef && e.child_idx == 0
+                                                   : e.kind == ExprKind::VirtColRef;
+    if (!direct || e.column_idx < 0 || e.column_idx >= static_cast<int>(child.scan_columns.size()))
+      return Materialize(child);
+    const DevColumn& col = ctx_.Column(child.relation, child.scan_columns[e.column_idx].name);
+    if (col.type.id == TypeId::TEXT || !(col.type == e.type) || e.nullable != (col.nulls != nullptr))
+      return Materialize(child);
+    MatCol mc;
+    mc.type = col.type;
+    mc.nullable = e.nullable;
+    mc.data = col.data;
+    mc.nulls = col.nulls;
+    m.cols.push_back(mc);
+  }
+  return m;
+}
 
 MatBuffer Executor::RunSkinner(const Operator& op, const SkinnerAgg* agg) {
   ctx_.NotReplayable();  // episode decisions follow the host's UCT search
@@ -5157,7 +5238,7 @@ MatBuffer Executor::RunSkinner(const Operator& op, const SkinnerAgg* agg) {
         cached = std::make_shared<BuildEntry>(ctx_);
         arena_.RedirectTo(&cached->arena);
         try {
-          cached->mat = Materialize(child);
+          cached->mat = SkinnerRows(child);
           cached->index.resize(cached->mat.cols.size());
           std::vector<std::pair<const MatBuffer*, int>> want;
           for (int c : index_cols[t]) want.emplace_back(&cached->mat, c);
@@ -5176,7 +5257,7 @@ MatBuffer Executor::RunSkinner(const Operator& op, const SkinnerAgg* agg) {
       index_for[t] = cached->index;
       continue;
     }
-    if (!mats_.count(&child)) mats_[&child] = Materialize(child);
+    if (!mats_.count(&child)) mats_[&child] = SkinnerRows(child);
     index_for[t].resize(mats_.at(&child).cols.size());
   }
   std::vector<const MatBuffer*> mats;

@@ -132,8 +132,11 @@ void Context::D2H(void* h, const void* d, size_t bytes) {
     std::memset(h, 0, bytes);
     return;
   }
-  if (bytes) KDB_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, stream));
+  constexpr size_t kStaged = size_t(64) << 10;
+  void* to = bytes && bytes <= kStaged ? HostStage(bytes) : h;
+  if (bytes) KDB_CUDA(cudaMemcpyAsync(to, d, bytes, cudaMemcpyDeviceToHost, stream));
   KDB_CUDA(cudaStreamSynchronize(stream));
+  if (to != h) std::memcpy(h, to, bytes);
 }
 
 void* Context::HostStage(size_t bytes) {
@@ -287,6 +290,7 @@ Context::~Context() {
     if (e) cudaEventDestroy(e);
   if (dev_stage_) cudaFreeAsync(dev_stage_, stream);
   cudaStreamSynchronize(stream);
+  cudaFree(scan_sums_);
   if (owns_catalog_) {
     for (auto& [n, t] : tables)
       for (auto& [cn, c] : t.cols) FreeColumn(c);
@@ -747,17 +751,34 @@ void Context::EndQueryProfile() {
   timings.clear();
 }
 
+// Small downloads go through the pinned staging buffer: a copy into pageable
+// memory makes the driver wait for it, stage it and copy it again.
 void Context::CheckDeviceError(const char* what) {
   if (dry) return;
-  int err[4] = {0, 0, 0, 0};
-  KDB_CUDA(cudaMemcpyAsync(err, d_err, sizeof(err), cudaMemcpyDeviceToHost, stream));
+  int* err = static_cast<int*>(HostStage(sizeof(int) * 4));
+  KDB_CUDA(cudaMemcpyAsync(err, d_err, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream));
   KDB_CUDA(cudaStreamSynchronize(stream));
-  if (err[0]) {
-    KDB_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * 4, stream));
-    if (err[0] == 1) throw Error(-4, std::string(what) + ": device table capacity exceeded");
-    if (err[0] == 2) throw Error(-6, std::string(what) + ": bounded device wait gave up");
-    throw Error(-5, std::string(what) + ": unsupported value on device");
-  }
+  ThrowDeviceError(err[0], what);
+}
+
+uint64_t Context::ReadWordChecked(const uint64_t* d, const char* what) {
+  uint64_t* h = static_cast<uint64_t*>(HostStage(2 * sizeof(uint64_t)));
+  KDB_CUDA(cudaMemcpyAsync(h, d, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
+  KDB_CUDA(cudaMemcpyAsync(h + 1, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  KDB_CUDA(cudaStreamSynchronize(stream));
+  const uint64_t word = h[0];
+  int err;
+  std::memcpy(&err, h + 1, sizeof(err));
+  ThrowDeviceError(err, what);
+  return word;
+}
+
+void Context::ThrowDeviceError(int err, const char* what) {
+  if (!err) return;
+  KDB_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * 4, stream));
+  if (err == 1) throw Error(-4, std::string(what) + ": device table capacity exceeded");
+  if (err == 2) throw Error(-6, std::string(what) + ": bounded device wait gave up");
+  throw Error(-5, std::string(what) + ": unsupported value on device");
 }
 
 }  // namespace kdb

@@ -404,6 +404,8 @@ class Context {
   // device decode of a TEXT .kdb image at d_raw (kernels.cu)
   void DecodeKdbText(const char* d_raw, int64_t n, int64_t* toff, char* tchars);
   void CheckDeviceError(const char* what);
+  // the word at `d` and the device error word, in one round trip
+  uint64_t ReadWordChecked(const uint64_t* d, const char* what);
 
   EnumDicts HostEnums() const;
 
@@ -411,6 +413,9 @@ class Context {
   std::shared_ptr<ProgramCache> cache_ = std::make_shared<ProgramCache>();
   cudaEvent_t query_ev_[2] = {nullptr, nullptr};
   bool owns_catalog_ = true;
+  uint64_t* scan_sums_ = nullptr;  // part sums of ScanParted (made on first use)
+  void ThrowDeviceError(int err, const char* what);
+  void ScanParted(uint64_t* a, int64_t n, const uint64_t* n_ptr);
   void* stage_ = nullptr;
   size_t stage_bytes_ = 0;
   std::shared_ptr<HostBlockPool> host_blocks_;
