@@ -15,7 +15,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 SOURCES = ["kernels.cu", "batch.cu", "engine.cc", "codegen.cc", "capi.cc", "server.cc", "join_prior.cu",
            "operators.cu", "capi_ops.cc"]
 HEADERS = ["engine.h", "plan.h", "json.h", "host_result.h", "capi_internal.h", "join_prior.h", "device_runtime.cuh",
-           "operators.h"]
+           "operators.h", "first_rows.cuh"]
 
 
 def _embed_runtime():

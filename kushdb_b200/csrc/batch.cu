@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "capi_internal.h"
+#include "first_rows.cuh"
 
 namespace kdb {
 namespace {
@@ -97,16 +98,6 @@ struct Acc {
   unsigned long long first_inv;
 };
 static_assert(sizeof(Acc) == 16, "Acc layout");
-
-// One word of a query's first-row bitmap: the bits of 32 fact rows, and the
-// groups whose first row lies before them.
-struct FirstWord {
-  uint32_t bits;
-  uint32_t before;
-};
-static_assert(sizeof(FirstWord) == 8, "FirstWord layout");
-constexpr int kOrderThreads = 256;
-constexpr int kOrderWords = 4 * kOrderThreads;  // bitmap words per CTA of the order phase
 
 // 64-bit mix of the key: the top bits choose the sub-table, the low 32 bits
 // the home slot inside it, so the two are independent.
@@ -269,7 +260,7 @@ __global__ void BatchMark(const QueryDesc* __restrict__ qs, int nq, const Acc* _
       if (inv[j] == 0) continue;
       const unsigned long long f = ~inv[j];
       atomicOr(&first[q.bit_base + static_cast<int64_t>(f >> 5)].bits, 1u << (f & 31));
-      const int c = static_cast<int>(f / (32 * kOrderWords));
+      const int c = static_cast<int>(f / kOrderRows);
       if (in_shared) atomicAdd(&groups[c], 1u);
       else atomicAdd(&chunk_groups[q.order_block0 + c], 1u);
     }
@@ -289,38 +280,12 @@ __global__ void __launch_bounds__(kOrderThreads) BatchOrder(const QueryDesc* __r
                                                             FirstWord* __restrict__ first,
                                                             unsigned long long* __restrict__ out_count) {
   __shared__ int sq;
-  __shared__ uint32_t earlier[kOrderThreads / 32], wsum[kOrderThreads / 32];
   if (threadIdx.x == 0) sq = FindQuery<3>(qs, nq, blockIdx.x);
   __syncthreads();
   const QueryDesc& q = qs[sq];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t e = 0;
-  for (int c = q.order_block0 + threadIdx.x; c < static_cast<int>(blockIdx.x); c += kOrderThreads) e += chunk_groups[c];
-  FirstWord* w = first + q.bit_base + static_cast<int64_t>(blockIdx.x - q.order_block0) * kOrderWords + 4 * threadIdx.x;
-  uint4* v = reinterpret_cast<uint4*>(w);  // two words each
-  uint4 a = v[0], b = v[1];
-  const uint32_t c0 = __popc(a.x), c1 = __popc(a.z), c2 = __popc(b.x), c3 = __popc(b.z);
-  const uint32_t mine = c0 + c1 + c2 + c3;
-  uint32_t incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-    e += __shfl_xor_sync(0xffffffffu, e, o);
-  }
-  if (lane == 31) wsum[warp] = incl;
-  if (lane == 0) earlier[warp] = e;
-  __syncthreads();
-  uint32_t run = incl - mine;
-  for (int k = 0; k < kOrderThreads / 32; k++) run += earlier[k] + (k < warp ? wsum[k] : 0u);
-  a.y = run;
-  a.w = run + c0;
-  b.y = run + c0 + c1;
-  b.w = run + c0 + c1 + c2;
-  v[0] = a;
-  v[1] = b;
-  if (threadIdx.x == kOrderThreads - 1 && static_cast<int>(blockIdx.x) == q.order_block0 + q.order_blocks - 1)
-    out_count[sq] = run + mine;
+  const int chunk = static_cast<int>(blockIdx.x);
+  const uint32_t upto = OrderChunk(first + q.bit_base, chunk_groups, q.order_block0, chunk);
+  if (threadIdx.x == kOrderThreads - 1 && chunk == q.order_block0 + q.order_blocks - 1) out_count[sq] = upto;
 }
 
 // Every group to its place among its query's groups.
@@ -391,7 +356,7 @@ class Batch {
       ob += q.out_blocks;
       q.order_block0 = static_cast<int32_t>(rb);
       q.order_blocks = static_cast<int32_t>(
-          std::max<int64_t>(1, (q.nf + 32 * kOrderWords - 1) / (32 * static_cast<int64_t>(kOrderWords))));
+          std::max<int64_t>(1, (q.nf + kOrderRows - 1) / kOrderRows));
       q.bit_base = rb * kOrderWords;
       rb += q.order_blocks;
       if (bb > INT_MAX || pb > INT_MAX) throw Error(KDB_ERR_CAPACITY, "batch too large");

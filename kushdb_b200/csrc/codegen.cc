@@ -708,6 +708,21 @@ class Executor {
       }
     }
   }
+  // When a stream's positions are distinct numbers below some bound (rows of
+  // a scan or of a buffer in stream order): that bound, else -1.
+  int64_t PosBound(const Operator& o) {
+    switch (o.kind) {
+      case OpKind::SCAN:
+      case OpKind::SCAN_SELECT: return RowBound(o);
+      case OpKind::SELECT: return PosBound(o.child());
+      case OpKind::HASH_JOIN:
+      case OpKind::CROSS_PRODUCT: return -1;
+      default: {
+        auto it = mats_.find(&o);
+        return it != mats_.end() && it->second.pos_is_index ? it->second.rows : -1;
+      }
+    }
+  }
   static bool Streamable(const Operator& op) {
     return op.kind == OpKind::SCAN || op.kind == OpKind::SCAN_SELECT || op.kind == OpKind::SELECT ||
            op.kind == OpKind::HASH_JOIN || op.kind == OpKind::CROSS_PRODUCT;
@@ -3232,7 +3247,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
   }
 
   // capacity: exact for small key domains; otherwise twice the input-row
-  // bound capped at 2^20 slots (regrown on overflow)
+  // bound capped at 2^20 records (regrown on overflow)
   uint64_t cap = 1024;
   if (kl.small_domain) {
     while (cap < 2 * kl.domain) cap <<= 1;
@@ -3241,68 +3256,160 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
                                        1ULL << 20);
     while (cap < want) cap <<= 1;
   }
+  // A group is a record of R words next to each other (a row's updates then
+  // touch one or two sectors, not one per word): the key (packed keys and a
+  // single BIGINT; other keys live in arrays beside a table of hashes), the
+  // complement of its first position, and the aggregates' states.  Minimum
+  // words are kept complemented too, so that every word starts as zero.
+  const bool wide = !kl.packed && nk == 1 && op.group_by[0]->type.id == TypeId::BIGINT && !kl.nullable[0];
+  const bool keyed = kl.packed || wide;
+  const int fw = keyed ? 1 : 0;  // the first position's word
+  bool any_text = false;
+  for (const auto& p : plans) any_text |= p.kind == StateKind::MinMaxText;
+  // groups of a plain stream are ordered by a bitmap of their first rows
+  const int64_t row_bound = PosBound(op.child());
+  const bool rank_rows = row_bound >= 0 && row_bound < (int64_t(1) << 38);
   for (int attempt = 0; attempt < 8; attempt++) {
     const auto mark = ctx_.RecordMark();
-    uint64_t mask = cap - 1;
-    uint64_t* slots = arena_.AllocT<uint64_t>(cap);
-    uint64_t* first = arena_.AllocT<uint64_t>(cap);
-    std::vector<uint64_t*> kw(nk), sv(plans.size()), sc(plans.size());
+    const uint64_t mask = cap - 1;
+    const uint64_t nrec = cap + (wide ? 1 : 0);  // BIGINT key 0 has the last record
+    uint64_t* slots = nullptr;
+    std::vector<uint64_t*> kw(nk);
     std::vector<int32_t*> klen(nk);
     std::vector<int8_t*> kn(nk);
-    if (!kl.packed)
+    if (!keyed) {
+      slots = arena_.AllocT<uint64_t>(cap);
+      ctx_.Memset(slots, 0, cap * sizeof(uint64_t));
       for (size_t k = 0; k < nk; k++) {
         kw[k] = arena_.AllocT<uint64_t>(cap);
         klen[k] = arena_.AllocT<int32_t>(cap);
         kn[k] = arena_.AllocT<int8_t>(cap);
       }
-    for (size_t j = 0; j < plans.size(); j++) {
-      sv[j] = arena_.AllocT<uint64_t>(cap);
-      sc[j] = arena_.AllocT<uint64_t>(cap);
     }
-    // init kernel
-    {
-      KernelSource ks;
-      std::string S = ks.Ptr(slots, "uint64_t"), F = ks.Ptr(first, "uint64_t");
-      std::string C = ks.Word(cap);
-      ks.Open("for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)" + C +
-              "; i += (int64_t)gridDim.x * blockDim.x)");
-      ks.L(S + "[i] = 0; " + F + "[i] = ~0ULL;");
-      for (size_t j = 0; j < plans.size(); j++) {
-        std::string V = ks.Ptr(sv[j], "uint64_t"), N = ks.Ptr(sc[j], "uint64_t");
-        bool min_init = plans[j].kind == StateKind::MinMaxKey && plans[j].is_min;
-        ks.L(V + "[i] = " + (min_init ? "~0ULL" : "0ULL") + "; " + N + "[i] = 0;");
-      }
-      ks.Close();
-      LaunchPipeline(ks, static_cast<int64_t>(cap), "group init");
-    }
+    // word offsets of each aggregate's value and count, fixed when the
+    // pipeline is emitted (whether a count is kept depends on the input)
+    std::vector<int> vw(plans.size(), -1), cw(plans.size(), -1);
+    int R = 0;
+    uint64_t* rec = nullptr;
     // aggregation pipeline
     {
       KernelSource ks;
       ExprGen eg(ctx_, ks);
-      std::string S = ks.Ptr(slots, "uint64_t"), F = ks.Ptr(first, "uint64_t");
+      const int w_rec = ks.Arg(0);
+      ks.pre << "  uint64_t* __restrict__ rec = (uint64_t*)a.w[" << w_rec << "];\n";
+      std::string S = keyed ? "" : ks.Ptr(slots, "uint64_t");
       std::string M = "(uint64_t)" + ks.Word(mask);
       std::string ERR = ks.Ptr(ctx_.d_err, "int");
-      std::vector<std::string> KW(nk), KL(nk), KN(nk), SV(plans.size()), SC(plans.size());
-      if (!kl.packed)
+      std::vector<std::string> KW(nk), KL(nk), KN(nk);
+      if (!keyed)
         for (size_t k = 0; k < nk; k++) {
           KW[k] = ks.Ptr(kw[k], "uint64_t");
           KL[k] = ks.Ptr(klen[k], "int32_t");
           KN[k] = ks.Ptr(kn[k], "int8_t");
         }
-      for (size_t j = 0; j < plans.size(); j++) {
-        SV[j] = ks.Ptr(sv[j], "uint64_t");
-        SC[j] = ks.Ptr(sc[j], "uint64_t");
-      }
+      const std::string find_tail = std::string(", KDB_R, ") + M + ", ";
+      // A block keeps the states of the keys it met first in shared memory
+      // and adds them to the table once at its end: a skewed key's rows would
+      // otherwise queue on its record (224k of 3M rows on one record: 450 us).
+      // A thread whose first 64 rows hit less than one time in eight (many
+      // keys, no skew) leaves the cache alone from then on.
+      int entry = 16;  // bytes per cached key: key, first position, states
+      for (const auto& p : plans) entry += (p.kind == StateKind::Count ? 0 : 8) + 4;
+      const int C = entry <= 44 ? 1024 : (entry <= 88 ? 512 : 256);
+      const bool cache = keyed && !any_text && entry * C <= 46 * 1024;
+      const std::string CN = std::to_string(C);
+      auto inverted = [&](size_t j) { return plans[j].kind == StateKind::MinMaxKey && plans[j].is_min; };
+      auto is_float = [&](size_t j) {
+        return plans[j].kind == StateKind::SumF64 || plans[j].kind == StateKind::AvgF64;
+      };
+      auto V = [](size_t j) { return "gv" + std::to_string(j); };
+      auto N = [](size_t j) { return "gn" + std::to_string(j); };
+      // adds values gv*, counts gn*, position gf to the record at `g`
+      auto to_record = [&](const std::string& g) {
+        for (size_t j = 0; j < plans.size(); j++) {
+          const std::string w = "rec[" + g + " + " + std::to_string(vw[j]) + "]";
+          if (is_float(j)) {
+            ks.L("if (" + N(j) + ") atomicAdd((double*)&" + w + ", " + V(j) + ");");
+          } else if (plans[j].kind == StateKind::SumI64) {
+            ks.L("if (" + N(j) + ") atomicAdd((unsigned long long*)&" + w + ", " + V(j) + ");");
+          } else if (plans[j].kind == StateKind::MinMaxKey) {
+            // a read first: the value rarely improves
+            ks.L("if (" + N(j) + " && " + V(j) + " > __ldcg((const unsigned long long*)&" + w +
+                 ")) atomicMax((unsigned long long*)&" + w + ", " + V(j) + ");");
+          }
+          if (cw[j] >= 0)
+            ks.L("if (" + N(j) + ") atomicAdd((unsigned long long*)&rec[" + g + " + " + std::to_string(cw[j]) +
+                 "], (unsigned long long)" + N(j) + ");");
+        }
+        const std::string f = "rec[" + g + " + " + std::to_string(fw) + "]";
+        ks.L("if (gf > __ldcg((const unsigned long long*)&" + f + ")) atomicMax((unsigned long long*)&" + f + ", gf);");
+      };
+      // strings are compared in place: one update per row
+      auto text_to_record = [&](const std::vector<CVal>& vals, const std::string& g) {
+        for (size_t j = 0; j < plans.size(); j++)
+          if (plans[j].kind == StateKind::MinMaxText)
+            ks.L("if (" + N(j) + ") kdb_atomic_str_minmax(&rec[" + g + " + " + std::to_string(vw[j]) + "], " + vals[j].v +
+                 ", " + (plans[j].is_min ? "true" : "false") + ");");
+      };
+      // folds the values of the lanes that share `id` into the first of
+      // them (gl); the others' are left as they are
+      auto fold_lanes = [&](const std::string& id) {
+        ks.L("const unsigned gm = __match_any_sync(__activemask(), " + id + ");");
+        ks.L("const int glead = __ffs(gm) - 1;");
+        ks.L("const bool gl = (int)(threadIdx.x & 31) == glead;");
+        ks.Open("for (unsigned rest = gm & (gm - 1); rest; rest &= rest - 1)");
+        ks.L("const int src = __ffs(rest) - 1;");
+        for (size_t j = 0; j < plans.size(); j++) {
+          const std::string J = std::to_string(j);
+          if (is_float(j) || plans[j].kind == StateKind::SumI64) {
+            ks.L("{ const auto x = __shfl_sync(gm, " + V(j) + ", src); if (gl) " + V(j) + " += x; }");
+          } else if (plans[j].kind == StateKind::MinMaxKey) {
+            ks.L("{ const auto x = __shfl_sync(gm, " + V(j) + ", src); if (gl && x > " + V(j) + ") " + V(j) + " = x; }");
+          }
+          ks.L("{ const unsigned x = __shfl_sync(gm, " + N(j) + ", src); if (gl) " + N(j) + " += x; }");
+        }
+        ks.L("{ const auto x = __shfl_sync(gm, gf, src); if (gl && x > gf) gf = x; }");
+        ks.Close();
+      };
       int64_t src_rows = 0;
       auto consume = [&](const std::vector<CVal>& in, const std::string& pos) {
         Scope s;
         s.child.push_back(in);
-        std::vector<CVal> keys;
+        std::vector<CVal> keys, vals;
         for (const auto& g : op.group_by) keys.push_back(eg.Emit(*g, s));
-        std::string g = ks.Fresh("g");
-        if (kl.packed) {
-          std::string pk = "0x8000000000000000ULL";
-          for (size_t k = 0; k < nk; k++) {
+        std::string fl = "0ULL";
+        int words = fw + 1;
+        for (size_t j = 0; j < plans.size(); j++) {
+          CVal c = eg.Emit(plans[j].agg->kid(0), s);
+          if (plans[j].count_flag >= 0)
+            fl += " | ((" + c.n + ") ? " + std::to_string(1 << plans[j].count_flag) + "ULL : 0ULL)";
+          counted[j] = NeedsCount(plans[j], c);
+          if (plans[j].kind != StateKind::Count) vw[j] = words++;
+          if (counted[j]) cw[j] = words++;
+          vals.push_back(c);
+        }
+        R = words;
+        ks.Open("");
+        for (size_t j = 0; j < plans.size(); j++) {
+          const CVal& c = vals[j];
+          ks.L("unsigned " + N(j) + " = (" + c.n + ") ? 0u : 1u;");
+          switch (plans[j].kind) {
+            case StateKind::SumF64:
+            case StateKind::AvgF64: ks.L("double " + V(j) + " = (" + c.n + ") ? 0.0 : (double)" + c.v + ";"); break;
+            case StateKind::SumI64:
+              ks.L("unsigned long long " + V(j) + " = (" + c.n + ") ? 0ULL : (unsigned long long)(int64_t)" + c.v + ";");
+              break;
+            case StateKind::MinMaxKey:
+              ks.L("unsigned long long " + V(j) + " = (" + c.n + ") ? 0ULL : " + (inverted(j) ? "~" : "") +
+                   "(unsigned long long)" + OKey(eg, c) + ";");
+              break;
+            default: break;
+          }
+        }
+        ks.L("unsigned long long gf = ~(((uint64_t)(" + pos + ") << 8) | (" + fl + "));");
+        if (keyed) {
+          std::string pk = wide ? "(uint64_t)" + keys[0].v : "0x8000000000000000ULL";
+          for (size_t k = 0; k < nk && !wide; k++) {
             const CVal& c = keys[k];
             std::string bits;
             switch (c.type.id) {
@@ -3318,7 +3425,43 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             if (kl.nullable[k])
               pk += " | ((" + c.n + ") ? (1ULL << " + std::to_string(kl.offset[k] + kl.width[k]) + ") : 0ULL)";
           }
-          ks.L("int64_t " + g + " = kdb_group_find_packed(" + S + ", " + M + ", " + pk + ", " + ERR + ");");
+          ks.L("const uint64_t gkey = " + pk + ";");
+          ks.L("const uint64_t ghash = kdb_mix64(gkey);");
+          if (cache) {
+            ks.L("bool ghit = false;");
+            // cache places come from other hash bits than the table's
+            ks.L("const uint32_t gc = (uint32_t)(ghash >> 40) & " + std::to_string(C - 1) + "u;");
+            ks.Open(std::string("if (kdb_cache_on") + (wide ? " && gkey != 0" : "") + ")");
+            ks.L("unsigned long long k = kdb_ck[gc];");
+            ks.L("if (k == 0) { k = atomicCAS(&kdb_ck[gc], 0ULL, (unsigned long long)gkey); if (k == 0) k = gkey; }");
+            ks.L("ghit = k == gkey;");
+            ks.L("kdb_seen++; kdb_hits += ghit ? 1u : 0u;");
+            ks.L("if (kdb_seen == 64u && kdb_hits < 8u) kdb_cache_on = false;");
+            ks.Close();
+            ks.Open("if (ghit)");
+            fold_lanes("gc");
+            ks.Open("if (gl)");
+            for (size_t j = 0; j < plans.size(); j++) {
+              const std::string v = "kdb_cv" + std::to_string(j) + "[gc]", n = "kdb_cn" + std::to_string(j) + "[gc]";
+              if (is_float(j) || plans[j].kind == StateKind::SumI64)
+                ks.L("if (" + N(j) + ") atomicAdd(&" + v + ", " + V(j) + ");");
+              else if (plans[j].kind == StateKind::MinMaxKey)
+                ks.L("if (" + N(j) + " && " + V(j) + " > " + v + ") atomicMax(&" + v + ", " + V(j) + ");");
+              ks.L("if (" + N(j) + ") atomicAdd(&" + n + ", " + N(j) + ");");
+            }
+            ks.L("if (gf > kdb_cf[gc]) atomicMax(&kdb_cf[gc], gf);");
+            ks.Close();
+            ks.Close();
+            ks.Open("else");
+          }
+          ks.L(std::string("const int64_t g = ") + (wide ? "gkey == 0 ? (int64_t)(" + M + " + 1) * KDB_R : " : "") +
+               "kdb_group_find_rec(rec" + find_tail + "gkey, ghash, " + ERR + ");");
+          if (wide) ks.L("if (gkey == 0) rec[g] = 1ULL;  // occupied (a BIGINT key 0)");
+          ks.Open("if (g >= 0)");
+          text_to_record(vals, "g");
+          to_record("g");
+          ks.Close();
+          if (cache) ks.Close();
         } else {
           std::string h = "0x2545f4914f6cdd1dULL";
           for (size_t k = 0; k < nk; k++)
@@ -3350,28 +3493,105 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             init += KN[k] + "[i] = (" + c.n + ") ? 1 : 0; ";
             eq += " && (" + stored_null + " == (" + c.n + ")) && ((" + c.n + ") || " + veq + ")";
           }
-          ks.L("int64_t " + g + " = kdb_group_find(" + S + ", " + M + ", (" + h +
+          ks.L("const int64_t g = kdb_group_find(" + S + ", " + M + ", (" + h +
                ") | 0x8000000000000000ULL, [&](uint64_t i) { return " + eq + "; }, [&](uint64_t i) { " + init +
                "}, " + ERR + ");");
+          ks.Open("if (g >= 0)");
+          if (any_text) {
+            text_to_record(vals, "g * KDB_R");
+            to_record("g * KDB_R");
+          } else {
+            fold_lanes("(unsigned)g");
+            ks.Open("if (gl)");
+            to_record("g * KDB_R");
+            ks.Close();
+          }
+          ks.Close();
         }
-        ks.Open("if (" + g + " >= 0)");
-        std::string fl = "0ULL";
-        for (size_t j = 0; j < plans.size(); j++) {
-          CVal c = eg.Emit(plans[j].agg->kid(0), s);
-          if (plans[j].count_flag >= 0)
-            fl += " | ((" + c.n + ") ? " + std::to_string(1 << plans[j].count_flag) + "ULL : 0ULL)";
-          counted[j] = NeedsCount(plans[j], c);
-          EmitGroupUpdate(ks, eg, plans[j], c, SV[j], SC[j], g, counted[j]);
-        }
-        ks.L("kdb_atomic_min_u64(&" + F + "[" + g + "], ((uint64_t)(" + pos + ") << 8) | (" + fl + "));");
         ks.Close();
       };
+      if (cache) ks.L("bool kdb_cache_on = true; unsigned kdb_seen = 0, kdb_hits = 0;");
       if (Streamable(op.child())) EmitStream(ks, eg, op.child(), consume, src_rows);
       else EmitMatScan(ks, mats_.at(&op.child()), nullptr, consume, src_rows);
-      LaunchPipeline(ks, src_rows, "group by");
+      ks.globals << "#define KDB_R " << R << "\n";
+      rec = arena_.AllocT<uint64_t>(nrec * R);
+      ctx_.Memset(rec, 0, nrec * R * sizeof(uint64_t));
+      ks.args[w_rec] = reinterpret_cast<uint64_t>(rec);
+      if (cache) {
+        std::ostringstream& pre = ks.pre;
+        pre << "  __shared__ unsigned long long kdb_ck[" << C << "], kdb_cf[" << C << "];\n";
+        std::string zero = "kdb_ck[i] = 0; kdb_cf[i] = 0;";
+        for (size_t j = 0; j < plans.size(); j++) {
+          if (plans[j].kind != StateKind::Count) {
+            pre << "  __shared__ " << (is_float(j) ? "double" : "unsigned long long") << " kdb_cv" << j << "[" << C << "];\n";
+            zero += " kdb_cv" + std::to_string(j) + "[i] = 0;";
+          }
+          pre << "  __shared__ unsigned kdb_cn" << j << "[" << C << "];\n";
+          zero += " kdb_cn" + std::to_string(j) + "[i] = 0;";
+        }
+        pre << "  for (int i = threadIdx.x; i < " << C << "; i += blockDim.x) { " << zero << " }\n  __syncthreads();\n";
+        // the cached keys' states into the table
+        ks.L("__syncthreads();");
+        ks.Open("for (int i = threadIdx.x; i < " + CN + "; i += blockDim.x)");
+        ks.L("const uint64_t gkey = kdb_ck[i];");
+        ks.L("if (gkey == 0) continue;");
+        ks.L("const int64_t g = kdb_group_find_rec(rec" + find_tail + "gkey, kdb_mix64(gkey), " + ERR + ");");
+        ks.L("if (g < 0) continue;");
+        for (size_t j = 0; j < plans.size(); j++) {
+          ks.L("const unsigned " + N(j) + " = kdb_cn" + std::to_string(j) + "[i];");
+          if (plans[j].kind != StateKind::Count) ks.L("const auto " + V(j) + " = kdb_cv" + std::to_string(j) + "[i];");
+        }
+        ks.L("const unsigned long long gf = kdb_cf[i];");
+        to_record("g");
+        ks.Close();
+        // few, large blocks: every block flushes its cache at the end
+        const int block = 512;
+        const int grid = std::min(ctx_.GridFor(std::max<int64_t>(src_rows, 1), block), 2 * ctx_.num_sms);
+        const std::string name = KernelName("group by");
+        ctx_.Launch(ctx_.Kernel(ks.Kernel(name, block, 2), name), grid, block, ks.Args(), 0, "group by");
+      } else {
+        LaunchPipeline(ks, src_rows, "group by");
+      }
     }
+    // the groups' order: a bitmap of their first rows, or (positions that
+    // are not row numbers) their first positions, compacted and sorted
+    const int64_t nwords = rank_rows ? Context::OrderWordsFor(row_bound) : 0;
+    uint2* first_rows = rank_rows ? arena_.AllocT<uint2>(static_cast<size_t>(nwords)) : nullptr;
+    uint64_t* keys = rank_rows ? nullptr : arena_.AllocT<uint64_t>(cap + 1);
+    uint32_t* vals = rank_rows ? nullptr : arena_.AllocT<uint32_t>(cap + 1);
+    uint64_t* ngroups = arena_.AllocT<uint64_t>(1);
+    if (rank_rows) ctx_.Memset(first_rows, 0, sizeof(uint2) * nwords);
+    else ctx_.Memset(ngroups, 0, sizeof(uint64_t));
+    const std::string Rs = std::to_string(R);
+    auto open_groups = [&](KernelSource& ks, const std::string& REC) {
+      const std::string S = keyed ? "" : ks.Ptr(slots, "uint64_t", true);
+      ks.Open("for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)" + ks.Word(nrec) +
+              "; i += (int64_t)gridDim.x * blockDim.x)");
+      ks.L("const uint64_t* __restrict__ r0 = " + REC + " + i * " + Rs + ";");
+      ks.L(std::string("if (") + (keyed ? "r0[0] == 0" : S + "[i] < 2") + ") continue;");
+      ks.L("const uint64_t fst = ~r0[" + std::to_string(fw) + "];");
+    };
+    {
+      KernelSource ks;
+      const std::string REC = ks.Ptr(rec, "uint64_t", true);
+      if (rank_rows) {
+        const std::string FR = ks.Ptr(first_rows, "uint2");
+        open_groups(ks, REC);
+        ks.L("atomicOr(&" + FR + "[fst >> 13].x, 1u << ((fst >> 8) & 31));");
+      } else {
+        const std::string K = ks.Ptr(keys, "uint64_t"), V = ks.Ptr(vals, "uint32_t");
+        const std::string NG = ks.Ptr(ngroups, "unsigned long long");
+        open_groups(ks, REC);
+        ks.L("uint64_t o = kdb_alloc_slot(" + NG + ");");
+        ks.L(K + "[o] = fst; " + V + "[o] = (uint32_t)i;");
+      }
+      ks.Close();
+      LaunchPipeline(ks, static_cast<int64_t>(nrec), "group compact");
+    }
+    if (rank_rows) ctx_.OrderFirstRows(first_rows, row_bound, ngroups, arena_);
+    int64_t ng = 0;
     try {
-      ctx_.CheckDeviceError("group by");
+      ng = ReadU64Checked(ngroups, "group by");
     } catch (const Error& e) {
       if (e.code == -4 && !kl.small_domain) {
         cap <<= 3;
@@ -3380,64 +3600,50 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       }
       throw;
     }
-    // compact occupied slots: (first position, slot)
-    uint64_t* keys = arena_.AllocT<uint64_t>(cap);
-    uint32_t* vals = arena_.AllocT<uint32_t>(cap);
-    uint64_t* ngroups = arena_.AllocT<uint64_t>(1);
-    ctx_.Memset(ngroups, 0, sizeof(uint64_t));
-    {
-      KernelSource ks;
-      std::string S = ks.Ptr(slots, "uint64_t", true), F = ks.Ptr(first, "uint64_t", true);
-      std::string K = ks.Ptr(keys, "uint64_t"), V = ks.Ptr(vals, "uint32_t");
-      std::string NG = ks.Ptr(ngroups, "unsigned long long");
-      std::string C = ks.Word(cap);
-      ks.Open("for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)" + C +
-              "; i += (int64_t)gridDim.x * blockDim.x)");
-      ks.Open("if (" + S + "[i] >= 2)");
-      ks.L("uint64_t o = kdb_alloc_slot(" + NG + ");");
-      ks.L(K + "[o] = " + F + "[i]; " + V + "[o] = (uint32_t)i;");
-      ks.Close();
-      ks.Close();
-      LaunchPipeline(ks, static_cast<int64_t>(cap), "group compact");
-    }
-    int64_t ng = ReadU64(ngroups);
-    if (!any_order) ctx_.RadixSortPairs(keys, vals, ng, arena_, 64);
+    const bool sorted = rank_rows || !any_order;
+    if (!rank_rows && !any_order) ctx_.RadixSortPairs(keys, vals, ng, arena_, 64);
     // output kernel
     MatBuffer out = AllocMat(op.output, ng);
     if (ng > 0) {
       KernelSource ks;
       ExprGen eg(ctx_, ks);
-      std::string S = ks.Ptr(slots, "uint64_t", true), F = ks.Ptr(first, "uint64_t", true);
-      std::string V = ks.Ptr(vals, "uint32_t", true);
-      std::string FK = any_order ? ks.Ptr(keys, "uint64_t", true) : "";
-      std::string NGW = ks.Word(static_cast<uint64_t>(ng));
-      std::vector<std::string> KW(nk), KL(nk), KN(nk), SV(plans.size()), SC(plans.size());
-      if (!kl.packed)
+      const std::string REC = ks.Ptr(rec, "uint64_t", true);
+      std::vector<std::string> KW(nk), KL(nk), KN(nk);
+      if (!keyed)
         for (size_t k = 0; k < nk; k++) {
           KW[k] = ks.Ptr(kw[k], "uint64_t", true);
           KL[k] = ks.Ptr(klen[k], "int32_t", true);
           KN[k] = ks.Ptr(kn[k], "int8_t", true);
         }
-      for (size_t j = 0; j < plans.size(); j++) {
-        SV[j] = ks.Ptr(sv[j], "uint64_t", true);
-        SC[j] = ks.Ptr(sc[j], "uint64_t", true);
-      }
       std::vector<std::string> optr, onull;
       for (const auto& c : out.cols) {
         optr.push_back(ks.Ptr(c.data, StoreType(c.type.id)));
         onull.push_back(c.nullable ? ks.Ptr(c.nulls, "int8_t") : "");
       }
       std::string posp = ks.Ptr(out.pos, "uint64_t");
-      ks.Open("for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < (int64_t)" + NGW +
-              "; r += (int64_t)gridDim.x * blockDim.x)");
-      ks.L("uint64_t i = " + V + "[r];");
-      ks.L("uint64_t fst = " + F + "[i];");
+      int64_t rows = static_cast<int64_t>(nrec);
+      if (rank_rows) {
+        const std::string FR = ks.Ptr(first_rows, "uint2", true);
+        open_groups(ks, REC);
+        ks.L("const uint2 fwd = " + FR + "[fst >> 13];");
+        ks.L("const int64_t r = (int64_t)fwd.y + __popc(fwd.x & ((1u << ((fst >> 8) & 31)) - 1));");
+      } else {
+        rows = ng;
+        const std::string Vp = ks.Ptr(vals, "uint32_t", true);
+        ks.Open("for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < (int64_t)" +
+                ks.Word(static_cast<uint64_t>(ng)) + "; r += (int64_t)gridDim.x * blockDim.x)");
+        ks.L("const int64_t i = (int64_t)" + Vp + "[r];");
+        ks.L("const uint64_t* __restrict__ r0 = " + REC + " + i * " + Rs + ";");
+        ks.L("const uint64_t fst = ~r0[" + std::to_string(fw) + "];");
+      }
       std::vector<CVal> virt;
       for (size_t k = 0; k < nk; k++) {
         const Type& t = op.group_by[k]->type;
-        if (kl.packed) {
+        if (wide) {
+          virt.push_back(eg.Bind(t, "i == (int64_t)" + ks.Word(cap) + " ? (int64_t)0 : (int64_t)r0[0]", "false"));
+        } else if (kl.packed) {
           uint64_t m = kl.width[k] >= 64 ? ~0ULL : ((1ULL << kl.width[k]) - 1);
-          std::string bits = "((" + S + "[i] >> " + std::to_string(kl.offset[k]) + ") & " + std::to_string(m) + "ULL)";
+          std::string bits = "((r0[0] >> " + std::to_string(kl.offset[k]) + ") & " + std::to_string(m) + "ULL)";
           std::string v;
           switch (t.id) {
             case TypeId::REAL: v = "__longlong_as_double((long long)" + bits + ")"; break;
@@ -3447,7 +3653,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             default: v = "(int32_t)(uint32_t)" + bits; break;
           }
           std::string n = kl.nullable[k]
-                              ? "(((" + S + "[i] >> " + std::to_string(kl.offset[k] + kl.width[k]) + ") & 1ULL) != 0)"
+                              ? "(((r0[0] >> " + std::to_string(kl.offset[k] + kl.width[k]) + ") & 1ULL) != 0)"
                               : "false";
           virt.push_back(eg.Bind(t, v, n));
         } else {
@@ -3462,8 +3668,15 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
           virt.push_back(eg.Bind(t, v, "(" + KN[k] + "[i] != 0)"));
         }
       }
-      for (size_t j = 0; j < plans.size(); j++)
-        virt.push_back(GroupResult(eg, plans[j], SV[j], SC[j], "i", "fst", counted[j] != 0));
+      for (size_t j = 0; j < plans.size(); j++) {
+        const std::string J = std::to_string(j);
+        const bool inv = plans[j].kind == StateKind::MinMaxKey && plans[j].is_min;
+        ks.L("const uint64_t gsv" + J + "[1] = {" +
+             (vw[j] >= 0 ? std::string(inv ? "~" : "") + "r0[" + std::to_string(vw[j]) + "]" : std::string("0")) + "};");
+        ks.L("const uint64_t gsc" + J + "[1] = {" +
+             (cw[j] >= 0 ? "r0[" + std::to_string(cw[j]) + "]" : std::string("0")) + "};");
+        virt.push_back(GroupResult(eg, plans[j], "gsv" + J, "gsc" + J, "0", "fst", counted[j] != 0));
+      }
       Scope s;
       s.virt = virt;
       for (size_t c = 0; c < op.output.size(); c++) {
@@ -3472,13 +3685,12 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         ks.L(optr[c] + "[r] = " + val + ";");
         if (!onull[c].empty()) ks.L(onull[c] + "[r] = (" + v.n + ") ? 1 : 0;");
       }
-      ks.L(posp + "[r] = " + (any_order ? FK + "[r]" : std::string("(uint64_t)r")) + ";");
+      ks.L(posp + "[r] = " + (sorted ? std::string("(uint64_t)r") : std::string("fst")) + ";");
       ks.Close();
-      LaunchPipeline(ks, ng, "group output");
+      LaunchPipeline(ks, rows, "group output");
     }
-    ctx_.CheckDeviceError("group output");
     out.rows = ng;
-    out.pos_is_index = !any_order;
+    out.pos_is_index = sorted;
     return out;
   }
   throw Error(-4, "group table did not fit");

@@ -422,8 +422,9 @@ KDB_DEV void kdb_join_insert(uint64_t* slots, uint64_t mask, uint32_t h, uint32_
 }
 
 // ---- group tables ------------------------------------------------------------
-// Packed keys: the whole group key fits in 63 bits; the slot word holds
-// key | 1<<63 and is claimed by a single CAS (no wait on other threads).
+// Packed keys: the whole group key fits in 63 bits; the key word holds
+// key | 1<<63 and is claimed by a single CAS (no wait on other threads).  A
+// single 64-bit key is stored as it is; its value 0 has a record of its own.
 // Overflow detection: tables are sized at most half full from the expected
 // group count, where a probe run averages about two slots; a run longer than
 // KDB_MAX_PROBE slots therefore means the estimate was wrong, and the lookup
@@ -431,15 +432,16 @@ KDB_DEV void kdb_join_insert(uint64_t* slots, uint64_t mask, uint32_t h, uint32_
 // shared counter is touched on the hot path.
 #define KDB_MAX_PROBE 256
 
-KDB_DEV int64_t kdb_group_find_packed(uint64_t* slots, uint64_t mask, uint64_t key, int* err) {
-  uint64_t i = kdb_mix64(key) & mask;
+// The table is an array of records of `stride` words whose first word is the
+// key (0: empty; the record's other words start as zeros); returns the word
+// offset of the key's record.
+KDB_DEV int64_t kdb_group_find_rec(uint64_t* rec, int stride, uint64_t mask, uint64_t key, uint64_t hash, int* err) {
+  uint64_t i = hash & mask;
   for (uint64_t k = 0; k <= mask && k < KDB_MAX_PROBE; k++) {
-    uint64_t s = *(volatile uint64_t*)&slots[i];
-    if (s == key) return (int64_t)i;
-    if (s == 0) {
-      uint64_t prev = atomicCAS((unsigned long long*)&slots[i], 0ULL, (unsigned long long)key);
-      if (prev == 0 || prev == key) return (int64_t)i;
-    }
+    unsigned long long* p = (unsigned long long*)(rec + i * stride);
+    unsigned long long s = __ldcg(p);
+    if (s == 0) s = atomicCAS(p, 0ULL, (unsigned long long)key);
+    if (s == 0 || s == key) return (int64_t)(i * stride);
     i = (i + 1) & mask;
   }
   kdb_set_error(err, KDB_DEV_ERR_CAPACITY);

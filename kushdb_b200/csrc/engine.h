@@ -392,6 +392,10 @@ class Context {
   // device), no pass computes it.
   bool RangeSortItems(void* items, int64_t n, Arena& arena, unsigned long long* ties = nullptr,
                       uint32_t tie_mask = 0, const unsigned long long* key_range = nullptr);
+  // fills the places of a bitmap of groups' first rows (first_rows.cuh;
+  // OrderWordsFor(rows) words) and writes the number of groups to *count
+  void OrderFirstRows(void* words, int64_t rows, uint64_t* count, Arena& arena);
+  static int64_t OrderWordsFor(int64_t rows);
   // lays out the groups counted in every index of `b` and fills their rows
   void GroupIndexRows(const IndexBatch& b);
   // exclusive prefix sum of a[0..n) in place, the total into a[n]

@@ -19,6 +19,7 @@
 
 #include "../../include/kdb_b200.h"
 #include "engine.h"
+#include "first_rows.cuh"
 
 namespace kdb {
 namespace {
@@ -700,6 +701,54 @@ __global__ void __launch_bounds__(256) FillIndexRows(const __grid_constant__ Ind
 }
 
 }  // namespace
+
+namespace {
+
+// bits set in every chunk of a first-row bitmap
+__global__ void __launch_bounds__(kOrderThreads) FirstRowCounts(const FirstWord* __restrict__ w,
+                                                                uint32_t* __restrict__ groups) {
+  const uint4* v = reinterpret_cast<const uint4*>(w + blockIdx.x * static_cast<int64_t>(kOrderWords) + 4 * threadIdx.x);
+  const uint4 a = v[0], b = v[1];
+  const unsigned n = __reduce_add_sync(0xffffffffu, __popc(a.x) + __popc(a.z) + __popc(b.x) + __popc(b.z));
+  __shared__ unsigned ws[kOrderThreads / 32];
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = n;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned t = 0;
+    for (int k = 0; k < kOrderThreads / 32; k++) t += ws[k];
+    groups[blockIdx.x] = t;
+  }
+}
+
+__global__ void __launch_bounds__(kOrderThreads) FirstRowOrder(FirstWord* __restrict__ w,
+                                                               const uint32_t* __restrict__ groups,
+                                                               unsigned long long* __restrict__ count) {
+  const uint32_t upto = OrderChunk(w, groups, 0, static_cast<int>(blockIdx.x));
+  if (threadIdx.x == kOrderThreads - 1 && blockIdx.x == gridDim.x - 1) *count = upto;
+}
+
+}  // namespace
+
+int64_t Context::OrderWordsFor(int64_t rows) {
+  return std::max<int64_t>(1, (rows + kOrderRows - 1) / kOrderRows) * kOrderWords;
+}
+
+void Context::OrderFirstRows(void* words, int64_t rows, uint64_t* count, Arena& arena) {
+  const int64_t chunks = OrderWordsFor(rows) / kOrderWords;
+  uint32_t* groups = arena.AllocT<uint32_t>(static_cast<size_t>(chunks));
+  if (dry) return;
+  FirstWord* w = static_cast<FirstWord*>(words);
+  const unsigned grid = static_cast<unsigned>(chunks);
+  TimedStart("group order");
+  Issue([=](cudaStream_t s) { FirstRowCounts<<<grid, kOrderThreads, 0, s>>>(w, groups); });
+  TimedStop();
+  TimedStart("group order");
+  Issue([=](cudaStream_t s) {
+    FirstRowOrder<<<grid, kOrderThreads, 0, s>>>(w, groups, reinterpret_cast<unsigned long long*>(count));
+  });
+  TimedStop();
+  KDB_CUDA(cudaGetLastError());
+}
 
 void Context::GroupIndexRows(const IndexBatch& b) {
   if (dry) return;
