@@ -30,6 +30,7 @@ struct HashTable {
   std::string table;
   plan::TypeId key_type = plan::TypeId::INT;
   bool wide = false;  // 64-bit keys: 16-byte slots
+  bool unique = false;  // no two build rows share a key (never known of 64-bit keys)
   int bits = 0;
   void* slots = nullptr;
   unsigned long long* slot_off = nullptr;  // device, 2^bits + 1 sub-table offsets (slots)

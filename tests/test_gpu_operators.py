@@ -161,6 +161,30 @@ def test_hash_join_matches_numpy(engine, fanout, nb, np_, dup):
     np.testing.assert_array_equal(ub[o], want_b)
 
 
+# unique build keys: ordered probes compact one match per row; around a
+# compaction tile (4096 rows) and a warp, with NULL keys on both sides
+@pytest.mark.parametrize("fanout", [1, 64])
+@pytest.mark.parametrize("np_", [1, 31, 33, 4095, 4096, 4097, 100_003])
+def test_hash_join_unique_keys_matches_numpy(engine, fanout, np_):
+    from kushdb_b200.operators import HashTable
+    rng = np.random.default_rng(np_)
+    nb = 20_011
+    bkeys = rng.permutation(nb).astype(np.int32)
+    bnull = (rng.random(nb) < 0.05).astype(np.int8)
+    pkeys = rng.integers(-10, nb + 4000, np_).astype(np.int32)
+    pnull = (rng.random(np_) < 0.1).astype(np.int8)
+    b = _key_table(f"ops_ub_{fanout}_{np_}", bkeys, bnull)
+    p = _key_table(f"ops_up_{fanout}_{np_}", pkeys, pnull)
+    engine.register_table(b)
+    engine.register_table(p)
+    ht = HashTable(engine, b.name, "k", fanout=fanout)
+    want_p, want_b = _join_pairs(bkeys, bnull, None, pkeys, pnull, None)
+    for _ in range(2):
+        got_p, got_b = ht.probe(p.name, "k")
+        np.testing.assert_array_equal(got_p, want_p)
+        np.testing.assert_array_equal(got_b, want_b)
+
+
 def test_hash_join_with_selections_and_bigint(engine):
     from kushdb_b200.operators import HashTable, scan_select
     rng = np.random.default_rng(11)
