@@ -428,6 +428,16 @@ int kdb_result_col_type(const kdb_result* r, int32_t col, char* buf, int32_t cap
 int kdb_result_get_i64(const kdb_result* r, int32_t col, int64_t* out);
 int kdb_result_get_f64(const kdb_result* r, int32_t col, double* out);
 int kdb_result_get_nulls(const kdb_result* r, int32_t col, int8_t* out);
+/* A result's shape in one call: its number of columns is returned, its rows
+ * go to *rows, and of the first `cap` columns the type goes to types[2c] (0
+ * SMALLINT, 1 INT, 2 BIGINT, 3 REAL, 4 DATE, 5 TEXT, 6 BOOLEAN, 7 ENUM) and
+ * the enum id to types[2c + 1]. */
+int32_t kdb_result_describe(const kdb_result* r, int64_t* rows, int32_t* types, int32_t cap);
+/* Every column in one call: column c's values to values[c] (double for REAL,
+ * int64_t for the others; TEXT columns are left out) and its NULL flags to
+ * nulls[c]; a null pointer skips that array.  Large results are copied by
+ * several host threads. */
+int kdb_result_read(const kdb_result* r, void* const* values, int8_t* const* nulls);
 int64_t kdb_result_get_text(const kdb_result* r, int32_t col, int64_t row, char* buf, int64_t cap);
 /* Whole result in the reference printer format ("v|v|...|\n" per row);
  * returns the size needed including the terminating NUL. */

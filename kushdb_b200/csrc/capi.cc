@@ -1,7 +1,10 @@
 // extern "C" boundary (include/kdb_b200.h): no exceptions cross it.
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <fstream>
 #include <sstream>
+#include <thread>
 #include <unordered_map>
 
 #include "capi_internal.h"
@@ -50,6 +53,46 @@ std::vector<char> ReadFile(const std::string& path) {
 
 namespace {
 void RunPlan(kdb_ctx* ctx, const char* plan_json, kdb_result** out);
+}  // namespace
+
+namespace {
+
+// Copies every column's values and NULL flags out of a result.  The arrays a
+// caller hands in for a large one are fresh memory, so the copy is bound by
+// page faults and one core's stores; pieces of it go to several threads,
+// which live for the call only.  Starting them and giving back memory that
+// several cores have touched costs more than it saves below about 16 MB: a
+// query returning 3 columns of 1M rows (27 MB) takes 2.5 ms with one thread
+// and 1.5 ms with several, one of 2 columns of 137k rows 362 and 590 us.
+void ReadResult(const kdb::HostResult& r, void* const* values, int8_t* const* nulls) {
+  constexpr int64_t kPieceRows = 1 << 14;
+  constexpr int64_t kManyThreads = int64_t(16) << 20, kThreadBytes = int64_t(3) << 20;
+  const int64_t pieces_per_col = (r.rows + kPieceRows - 1) / kPieceRows;
+  const int64_t pieces = pieces_per_col * static_cast<int64_t>(r.cols.size());
+  auto piece = [&](int64_t p) {
+    const size_t c = static_cast<size_t>(p / pieces_per_col);
+    const int64_t b = p % pieces_per_col * kPieceRows, e = std::min(b + kPieceRows, r.rows);
+    const bool text = r.cols[c].type.id == kdb::plan::TypeId::TEXT;
+    r.cols[c].CopyRange(b, e, values && !text ? static_cast<uint64_t*>(values[c]) : nullptr, nulls ? nulls[c] : nullptr);
+  };
+  const int64_t bytes = r.rows * 9 * static_cast<int64_t>(r.cols.size());
+  const int64_t cores = std::max<int64_t>(1, std::thread::hardware_concurrency());
+  const int threads =
+      bytes < kManyThreads ? 1 : static_cast<int>(std::min<int64_t>({bytes / kThreadBytes, cores, pieces, 8}));
+  std::atomic<int64_t> next{0};
+  auto work = [&] {
+    for (int64_t p; (p = next.fetch_add(1)) < pieces;) piece(p);
+  };
+  std::vector<std::thread> others;
+  try {
+    for (int t = 1; t < threads; t++) others.emplace_back(work);
+  } catch (...) {
+    // no more threads to be had: the ones there are do it
+  }
+  work();
+  for (auto& t : others) t.join();
+}
+
 }  // namespace
 
 kdb::Context* kdb_ctx_context(kdb_ctx* ctx) { return ctx->c.get(); }
@@ -371,6 +414,27 @@ int kdb_result_get_nulls(const kdb_result* r, int32_t col, int8_t* out) {
   if (!r || col < 0 || col >= static_cast<int32_t>(r->r.cols.size())) return KDB_ERR_INVALID;
   r->r.cols[col].CopyNulls(r->r.rows, out);
   return KDB_OK;
+}
+
+int32_t kdb_result_describe(const kdb_result* r, int64_t* rows, int32_t* types, int32_t cap) {
+  if (!r) return -1;
+  if (rows) *rows = r->r.rows;
+  const int32_t n = static_cast<int32_t>(r->r.cols.size());
+  for (int32_t c = 0; types && c < std::min(n, cap); c++) {
+    types[2 * c] = static_cast<int32_t>(r->r.cols[c].type.id);
+    types[2 * c + 1] = r->r.cols[c].type.enum_id;
+  }
+  return n;
+}
+
+int kdb_result_read(const kdb_result* r, void* const* values, int8_t* const* nulls) {
+  if (!r) return KDB_ERR_INVALID;
+  try {
+    ReadResult(r->r, values, nulls);
+    return KDB_OK;
+  } catch (...) {
+    return KDB_ERR_INVALID;
+  }
 }
 
 int64_t kdb_result_get_text(const kdb_result* r, int32_t col, int64_t row, char* buf, int64_t cap) {

@@ -88,6 +88,37 @@ struct HostColumn {
   }
   double RealAt(int64_t r) const { return packed ? reinterpret_cast<const double*>(data)[r] : f[r]; }
 
+  // Rows [b, e) as 64-bit values (the bits of doubles for REAL) and NULL
+  // flags, from the column's start at `out` / `flags`.
+  void CopyRange(int64_t b, int64_t e, uint64_t* out, int8_t* flags) const {
+    if (out) {
+      if (!packed) {
+        const bool real = type.id == plan::TypeId::REAL;
+        const size_t have = real ? f.size() : i.size();
+        if (have < static_cast<size_t>(e)) std::memset(out + b, 0, 8 * (e - b));
+        else if (real) std::memcpy(out + b, f.data() + b, sizeof(double) * (e - b));
+        else std::memcpy(out + b, i.data() + b, sizeof(int64_t) * (e - b));
+      } else {
+        auto widen = [&](auto tag) {
+          using T = decltype(tag);
+          const T* v = reinterpret_cast<const T*>(data);
+          for (int64_t r = b; r < e; r++) out[r] = static_cast<uint64_t>(static_cast<int64_t>(v[r]));
+        };
+        switch (width) {
+          case 1: widen(int8_t{}); break;
+          case 2: widen(int16_t{}); break;
+          case 4: widen(int32_t{}); break;
+          default: std::memcpy(out + b, data + 8 * b, 8 * (e - b)); break;
+        }
+      }
+    }
+    if (flags) {
+      const int8_t* src = packed ? nulls : (null.empty() ? nullptr : null.data());
+      if (src) std::memcpy(flags + b, src + b, e - b);
+      else std::memset(flags + b, 0, e - b);
+    }
+  }
+
   // Whole-column copies (the C interface); false when the column has no
   // values of that kind (integers of a REAL or TEXT column, reals of a
   // non-REAL column).

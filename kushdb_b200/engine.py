@@ -29,6 +29,7 @@ EXPORTS = [
     "kdb_enum_open_kdbenum", "kdb_query_execute", "kdb_last_query_device_ms",
     "kdb_result_num_rows", "kdb_result_num_cols", "kdb_result_col_type", "kdb_result_get_i64",
     "kdb_result_get_f64", "kdb_result_get_nulls", "kdb_result_get_text", "kdb_result_format",
+    "kdb_result_describe", "kdb_result_read",
     "kdb_result_free", "kdb_sort_pairs", "kdb_ctx_set_skinner", "kdb_last_skinner_episodes",
     "kdb_batch_create", "kdb_batch_configure", "kdb_batch_tune", "kdb_batch_config", "kdb_batch_run",
     "kdb_batch_run_timed", "kdb_batch_result", "kdb_batch_free", "kdb_sort_pairs_noalloc",
@@ -174,6 +175,9 @@ def load_library(path: str = LIB_PATH):
     L.kdb_ctx_get_option.restype = I64
     L.kdb_ctx_get_option.argtypes = [P, CP, ctypes.c_char_p, I64]
     declare_result_api(L, "kdb_")
+    L.kdb_result_describe.restype = I32
+    L.kdb_result_describe.argtypes = [P, P, P, I32]
+    L.kdb_result_read.argtypes = [P, P, P]
     _lib = L
     return L
 
@@ -202,6 +206,7 @@ class Engine:
         self.ctx = h
         self.device = device
         self._enums_sent: Dict[int, int] = {}
+        self._enums_version = -1
 
     def close(self):
         if self.ctx:
@@ -225,6 +230,9 @@ class Engine:
             raise KdbError(rc, self.lib.kdb_last_error(self.ctx).decode())
 
     def register_enums(self) -> None:
+        version = EnumRegistry.version()
+        if version == self._enums_version:
+            return
         for k, vals in EnumRegistry.all().items():
             key = tuple(vals)
             if self._enums_sent.get(k) == key:
@@ -235,6 +243,7 @@ class Engine:
             off[1:] = np.cumsum([len(b) for b in enc])
             chars = np.frombuffer(b"".join(enc) or b"\0", np.uint8)
             self._check(self.lib.kdb_enum_register(self.ctx, k, _ptr(off), _ptr(chars), len(enc)))
+        self._enums_version = version
 
     def register_table(self, table: HostTable, name: Optional[str] = None) -> None:
         name = (name or table.name).encode()

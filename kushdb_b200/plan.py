@@ -140,10 +140,16 @@ class EnumRegistry:
     """
 
     _dicts: Dict[int, List[str]] = {}
+    _version = 0  # changes with every registration
 
     @classmethod
     def register(cls, enum_id: int, values: Sequence[str]) -> None:
         cls._dicts[enum_id] = list(values)
+        cls._version += 1
+
+    @classmethod
+    def version(cls) -> int:
+        return cls._version
 
     @classmethod
     def values(cls, enum_id: int) -> List[str]:

@@ -13,7 +13,14 @@ from typing import List, Optional
 import numpy as np
 
 from .data import parse_type
-from .plan import Type
+from .plan import TYPE_IDS, Type
+
+_TYPES = [Type(t) for t in TYPE_IDS]
+_REAL, _TEXT, _ENUM = (TYPE_IDS.index(t) for t in ("REAL", "TEXT", "ENUM"))
+# Bytes of a result whose columns share one array: one block is reused by
+# the next result of the size, where several are given back to the system and
+# faulted in again, page by page.
+_ONE_BLOCK = 24 << 20
 
 
 @dataclass
@@ -77,8 +84,60 @@ class Result:
         except Exception:
             pass
 
+    def _read_at_once(self, lib, handle) -> List[ResultColumn]:
+        """Every column through one library call."""
+        rows = ctypes.c_int64()
+        types = (ctypes.c_int32 * 64)()
+        n = lib.kdb_result_describe(handle, ctypes.byref(rows), types, 32)
+        if n > 32:
+            types = (ctypes.c_int32 * (2 * n))()
+            lib.kdb_result_describe(handle, ctypes.byref(rows), types, n)
+        nrows = rows.value
+        if 9 * n * nrows <= _ONE_BLOCK:
+            block = np.empty(9 * n * nrows, np.int8)
+            v0 = block.__array_interface__["data"][0]
+            n0 = v0 + 8 * n * nrows
+            values = block[:8 * n * nrows].view(np.int64).reshape(n, nrows)
+            nulls = block[8 * n * nrows:].reshape(n, nrows)
+            vp = [v0 + 8 * nrows * c for c in range(n)]
+            np_ = [n0 + nrows * c for c in range(n)]
+        else:
+            values = [np.empty(nrows, np.int64) for _ in range(n)]
+            nulls = [np.empty(nrows, np.int8) for _ in range(n)]
+            vp = [a.__array_interface__["data"][0] for a in values]
+            np_ = [a.__array_interface__["data"][0] for a in nulls]
+        ptrs = ctypes.c_void_p * max(n, 1)
+        if lib.kdb_result_read(handle, ptrs(*vp), ptrs(*np_)) != 0:
+            raise RuntimeError("kdb_result_read failed")
+        cols = []
+        for c in range(n):
+            t = types[2 * c]
+            if t == _TEXT:
+                cols.append(ResultColumn(_TYPES[t], self._read_text(c, nrows), nulls[c]))
+            else:
+                typ = Type.Enum(types[2 * c + 1]) if t == _ENUM else _TYPES[t]
+                cols.append(ResultColumn(typ, values[c].view(np.float64) if t == _REAL else values[c], nulls[c]))
+        return cols
+
+    def _read_text(self, c: int, nrows: int) -> List[str]:
+        lib, prefix, _ctx, handle = self._src
+        get = getattr(lib, prefix + "result_get_text")
+        vals = []
+        tb = ctypes.create_string_buffer(256)
+        for r in range(nrows):
+            n = get(handle, c, r, tb, 256)
+            if n > 256:
+                tb2 = ctypes.create_string_buffer(int(n))
+                get(handle, c, r, tb2, n)
+                vals.append(tb2.raw[:n].decode())
+            else:
+                vals.append(tb.raw[:n].decode())
+        return vals
+
     def _read_columns(self) -> List[ResultColumn]:
         lib, prefix, _ctx, handle = self._src
+        if prefix == "kdb_":
+            return self._read_at_once(lib, handle)
         f = lambda n: getattr(lib, prefix + n)  # noqa: E731
         nrows = f("result_num_rows")(handle)
         ncols = f("result_num_cols")(handle)
@@ -94,16 +153,7 @@ class Result:
                 vals = np.zeros(nrows, np.float64)
                 f("result_get_f64")(handle, c, vals.ctypes.data_as(ctypes.c_void_p))
             elif t.type_id == "TEXT":
-                vals = []
-                tb = ctypes.create_string_buffer(256)
-                for r in range(nrows):
-                    n = f("result_get_text")(handle, c, r, tb, 256)
-                    if n > 256:
-                        tb2 = ctypes.create_string_buffer(int(n))
-                        f("result_get_text")(handle, c, r, tb2, n)
-                        vals.append(tb2.raw[:n].decode())
-                    else:
-                        vals.append(tb.raw[:n].decode())
+                vals = self._read_text(c, nrows)
             else:
                 vals = np.zeros(nrows, np.int64)
                 f("result_get_i64")(handle, c, vals.ctypes.data_as(ctypes.c_void_p))
