@@ -1,9 +1,8 @@
-// Kernels of the learned join-order prior (join_prior.h): fused forward over
-// all layers, fused backward with deterministic per-CTA gradient partials,
-// and a reduce + Adam update.  The MLP is tiny (41,473 fp32 parameters), so
-// the kernels run on CUDA cores: each CTA of 128 threads owns a tile of 16
-// rows, thread j computes hidden unit j for every row of the tile, and the
-// activations of the tile stay in shared memory between layers.
+// Kernels of the learned join-order prior (join_prior.h): one forward (and
+// back to every layer's deltas) of all layers, and one weight gradient + Adam
+// update.  The MLP is tiny (41,473 fp32 parameters) and stays in fp32, so it
+// runs on CUDA cores, bound by latency: what matters is how many SMs and
+// warps share a batch and how many dependent steps each takes.
 #include "join_prior.h"
 
 #include <algorithm>
@@ -17,32 +16,27 @@ namespace {
 
 constexpr int kIn = JoinPrior::kIn;
 constexpr int kHid = JoinPrior::kHid;
-constexpr int kRows = 16;      // rows per CTA
-constexpr int kThreads = kHid;  // one thread per hidden unit
+constexpr int kPassThreads = 256;  // forward / deltas: 8 warps
+constexpr int kPassWarps = kPassThreads / 32;
+constexpr int kPitch = kHid + 4;   // floats per weight row in shared memory: rows four banks apart
+constexpr int kMaxTileRows = 8;
+constexpr int kGradThreads = 512;
+constexpr int kGradWarps = kGradThreads / 32;
 constexpr int64_t kParams = JoinPrior::kParams;
 
-// out[r][j] = relu(b[j] + sum_k in[r][k] * W[k][j]) for the tile; saved to
-// global for the backward pass.
-template <int K>
-__device__ __forceinline__ void Dense(const float* __restrict__ W, const float* __restrict__ b, const float* in,
-                                      float* out, float* __restrict__ save, int64_t row0, int64_t n) {
-  const int j = threadIdx.x;
-  float acc[kRows];
-  const float bj = b[j];
-#pragma unroll
-  for (int r = 0; r < kRows; r++) acc[r] = bj;
-  for (int k = 0; k < K; k++) {
-    const float w = W[k * kHid + j];
-#pragma unroll
-    for (int r = 0; r < kRows; r++) acc[r] = fmaf(in[r * K + k], w, acc[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < kRows; r++) {
-    const float v = fmaxf(acc[r], 0.f);
-    out[r * kHid + j] = v;
-    if (row0 + r < n) save[(row0 + r) * kHid + j] = v;
-  }
-}
+// Shared memory of a forward / deltas CTA working on R rows at a time.
+template <int R>
+struct PassSmem {
+  float w[(kIn + 2 * kHid) * kPitch];  // W1, W2, W3
+  float b[3 * kHid];
+  float w4[kHid];
+  float x[R * kIn];
+  float h[3][R * kHid];
+  float d[2][R * kHid];
+  float part[kPassWarps * R * kHid];
+  float dy[R];
+};
+static_assert(sizeof(PassSmem<kMaxTileRows>) <= 227 * 1024, "fits an SM");
 
 __device__ __forceinline__ float WarpSum(float s) {
 #pragma unroll
@@ -50,149 +44,220 @@ __device__ __forceinline__ float WarpSum(float s) {
   return s;
 }
 
-template <int K>
-__device__ __forceinline__ void LoadTile(float* dst, const float* __restrict__ src, int64_t row0, int64_t n) {
-  for (int i = threadIdx.x; i < kRows * K; i += kThreads) {
-    const int r = i / K;
-    dst[i] = row0 + r < n ? src[(row0 + r) * K + i % K] : 0.f;
-  }
+__device__ __forceinline__ void CopyAsync16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+// ROWS weight rows of kHid floats into rows of kPitch floats, as one group
+template <int ROWS>
+__device__ __forceinline__ void CopyRowsAsync(float* dst, const float* src) {
+  for (int i = threadIdx.x; i < ROWS * (kHid / 4); i += kPassThreads)
+    CopyAsync16(dst + (i / (kHid / 4)) * kPitch + 4 * (i % (kHid / 4)), src + 4 * i);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int LEFT>
+__device__ __forceinline__ void WaitCopies() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) PriorForward(const float* __restrict__ P, const float* __restrict__ X,
-                                                         int64_t n, float* __restrict__ Y, float* __restrict__ H) {
-  __shared__ float xs[kRows * kIn];
-  __shared__ float ha[kRows * kHid];
-  __shared__ float hb[kRows * kHid];
-  __shared__ float red[kThreads / 32][kRows];
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows;
-  float* H1 = H;
-  float* H2 = H + static_cast<int64_t>(JoinPrior::kMaxRows) * kHid;
-  float* H3 = H + 2 * static_cast<int64_t>(JoinPrior::kMaxRows) * kHid;
-  LoadTile<kIn>(xs, X, row0, n);
+// Sums the warps' shares of R x kHid outputs in warp order from `first` on,
+// and hands each to done(row, column, sum); ends with a barrier.
+template <int R, typename FIRST, typename DONE>
+__device__ __forceinline__ void SumShares(const float* part, FIRST first, DONE done) {
   __syncthreads();
-  Dense<kIn>(P + JoinPrior::kOffW1, P + JoinPrior::kOffB1, xs, ha, H1, row0, n);
-  __syncthreads();
-  Dense<kHid>(P + JoinPrior::kOffW2, P + JoinPrior::kOffB2, ha, hb, H2, row0, n);
-  __syncthreads();
-  Dense<kHid>(P + JoinPrior::kOffW3, P + JoinPrior::kOffB3, hb, ha, H3, row0, n);
-  __syncthreads();
-  const int j = threadIdx.x;
-  const float w = P[JoinPrior::kOffW4 + j];
 #pragma unroll
-  for (int r = 0; r < kRows; r++) {
-    const float s = WarpSum(ha[r * kHid + j] * w);
-    if ((j & 31) == 0) red[j >> 5][r] = s;
+  for (int o = threadIdx.x; o < R * kHid; o += kPassThreads) {
+    const int r = o / kHid, j = o % kHid;
+    float s = first(j);
+#pragma unroll
+    for (int w = 0; w < kPassWarps; w++) s += part[w * R * kHid + o];
+    done(r, j, s);
   }
   __syncthreads();
-  if (j < kRows && row0 + j < n)
-    Y[row0 + j] = ((red[0][j] + red[1][j]) + (red[2][j] + red[3][j])) + P[JoinPrior::kOffB4];
 }
 
-// outW[k][j] = sum_r in[r][k] * dz[r][j], outB[j] = sum_r dz[r][j]
-template <int K>
-__device__ __forceinline__ void WeightGrad(const float* in, const float* dz, float* __restrict__ outW,
-                                           float* __restrict__ outB) {
-  const int j = threadIdx.x;
-  float d[kRows];
-  float sb = 0.f;
+// Warp w's share of in (R x K) times W (K x kHid): inputs k in [w, w + 1) *
+// K / 8.  A lane owns 4 neighbouring outputs: a weight row is one 16-byte
+// load per lane, an input is the same word for the whole warp.
+template <int R, int K>
+__device__ __forceinline__ void DenseShare(const float* W, const float* in, float* part) {
+  constexpr int kShare = K / kPassWarps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k0 = warp * kShare;
+  float acc[R][4];
 #pragma unroll
-  for (int r = 0; r < kRows; r++) {
-    d[r] = dz[r * kHid + j];
-    sb += d[r];
-  }
-  outB[j] = sb;
-  for (int k = 0; k < K; k++) {
-    float s = 0.f;
+  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
 #pragma unroll
-    for (int r = 0; r < kRows; r++) s = fmaf(in[r * K + k], d[r], s);
-    outW[k * kHid + j] = s;
-  }
-}
-
-// dst[r][k] = (act[r][k] > 0) * sum_j dz[r][j] * W[k][j]  (W is kHid x kHid)
-__device__ __forceinline__ void InputGrad(const float* __restrict__ W, const float* dz, const float* act,
-                                          float* dst) {
-  const int k = threadIdx.x;
-  float s[kRows];
+  for (int k = 0; k < kShare; k += 4) {
+    float4 v[R];
 #pragma unroll
-  for (int r = 0; r < kRows; r++) s[r] = 0.f;
-  const float4* row = reinterpret_cast<const float4*>(W + k * kHid);
-  for (int j4 = 0; j4 < kHid / 4; j4++) {
-    const float4 w = row[j4];
+    for (int r = 0; r < R; r++) v[r] = *reinterpret_cast<const float4*>(in + r * K + k0 + k);
 #pragma unroll
-    for (int r = 0; r < kRows; r++) {
-      const float* z = dz + r * kHid + 4 * j4;
-      s[r] = fmaf(z[0], w.x, s[r]);
-      s[r] = fmaf(z[1], w.y, s[r]);
-      s[r] = fmaf(z[2], w.z, s[r]);
-      s[r] = fmaf(z[3], w.w, s[r]);
+    for (int i = 0; i < 4; i++) {
+      const float4 w = *reinterpret_cast<const float4*>(W + (k0 + k + i) * kPitch + 4 * lane);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const float s = i == 0 ? v[r].x : i == 1 ? v[r].y : i == 2 ? v[r].z : v[r].w;
+        acc[r][0] = fmaf(s, w.x, acc[r][0]);
+        acc[r][1] = fmaf(s, w.y, acc[r][1]);
+        acc[r][2] = fmaf(s, w.z, acc[r][2]);
+        acc[r][3] = fmaf(s, w.w, acc[r][3]);
+      }
     }
   }
 #pragma unroll
-  for (int r = 0; r < kRows; r++) dst[r * kHid + k] = act[r * kHid + k] > 0.f ? s[r] : 0.f;
+  for (int r = 0; r < R; r++)
+    *reinterpret_cast<float4*>(part + (warp * R + r) * kHid + 4 * lane) =
+        make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
 }
 
-// Gradient of mean((y - t)^2) for this CTA's rows into partial[blockIdx.x].
-__global__ void __launch_bounds__(kThreads) PriorBackward(const float* __restrict__ P, const float* __restrict__ X,
-                                                          const float* __restrict__ H, const float* __restrict__ Y,
-                                                          const float* __restrict__ T, int64_t n,
-                                                          float* __restrict__ partial) {
-  __shared__ float dy[kRows];
-  __shared__ float ga[kRows * kHid];
-  __shared__ float gb[kRows * kHid];
-  __shared__ float hs[kRows * kHid];
-  __shared__ float xs[kRows * kIn];
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows;
-  const float* H1 = H;
-  const float* H2 = H + static_cast<int64_t>(JoinPrior::kMaxRows) * kHid;
-  const float* H3 = H + 2 * static_cast<int64_t>(JoinPrior::kMaxRows) * kHid;
-  float* out = partial + static_cast<int64_t>(blockIdx.x) * kParams;
-  const int j = threadIdx.x;
-  if (j < kRows) dy[j] = row0 + j < n ? 2.f * (Y[row0 + j] - T[row0 + j]) / static_cast<float>(n) : 0.f;
-  LoadTile<kHid>(hs, H3, row0, n);
-  __syncthreads();
-  // head: y = w4 . h3 + b4
-  {
-    float g = 0.f, sb = 0.f;
+// Warp w's share of dz (R x kHid) times W transposed: columns j in [w, w + 1)
+// * 16.  A lane owns outputs lane + 32 i, whose weight rows lie four banks
+// apart.
+template <int R>
+__device__ __forceinline__ void DeltaShare(const float* W, const float* dz, float* part) {
+  constexpr int kShare = kHid / kPassWarps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = warp * kShare;
+  float acc[R][4];
 #pragma unroll
-    for (int r = 0; r < kRows; r++) {
-      g = fmaf(dy[r], hs[r * kHid + j], g);
-      sb += dy[r];
+  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+#pragma unroll
+  for (int j = 0; j < kShare; j += 4) {
+    float4 v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = *reinterpret_cast<const float4*>(dz + r * kHid + j0 + j);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float4 w = *reinterpret_cast<const float4*>(W + (lane + 32 * i) * kPitch + j0 + j);
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        acc[r][i] = fmaf(v[r].w, w.w, fmaf(v[r].z, w.z, fmaf(v[r].y, w.y, fmaf(v[r].x, w.x, acc[r][i]))));
     }
-    out[JoinPrior::kOffW4 + j] = g;
-    if (j == 0) out[JoinPrior::kOffB4] = sb;
-    const float w4 = P[JoinPrior::kOffW4 + j];
-#pragma unroll
-    for (int r = 0; r < kRows; r++) ga[r * kHid + j] = hs[r * kHid + j] > 0.f ? dy[r] * w4 : 0.f;
   }
-  __syncthreads();
-  // layer 3 (input H2, pre-activation delta ga)
-  LoadTile<kHid>(hs, H2, row0, n);
-  __syncthreads();
-  WeightGrad<kHid>(hs, ga, out + JoinPrior::kOffW3, out + JoinPrior::kOffB3);
-  InputGrad(P + JoinPrior::kOffW3, ga, hs, gb);
-  __syncthreads();
-  // layer 2 (input H1, delta gb)
-  LoadTile<kHid>(hs, H1, row0, n);
-  __syncthreads();
-  WeightGrad<kHid>(hs, gb, out + JoinPrior::kOffW2, out + JoinPrior::kOffB2);
-  InputGrad(P + JoinPrior::kOffW2, gb, hs, ga);
-  __syncthreads();
-  // layer 1 (input X, delta ga)
-  LoadTile<kIn>(xs, X, row0, n);
-  __syncthreads();
-  WeightGrad<kIn>(xs, ga, out + JoinPrior::kOffW1, out + JoinPrior::kOffB1);
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) part[(warp * R + r) * kHid + lane + 32 * i] = acc[r][i];
 }
 
-// grad = sum of the CTA partials (fixed order); optional Adam step
-// (Kingma & Ba, beta1 0.9, beta2 0.999, eps 1e-8).
-__global__ void PriorAdam(float* __restrict__ P, const float* __restrict__ partial, int nblk, float* __restrict__ m,
-                          float* __restrict__ v, float* __restrict__ grad, float lr, float c1, float c2) {
-  for (int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; p < kParams;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    float g = 0.f;
-    for (int b = 0; b < nblk; b++) g += partial[b * kParams + p];
-    grad[p] = g;
+// Forward of every layer for tiles of R rows and, with targets, back to
+// every layer's pre-activation deltas.  Each CTA brings all weights into its
+// shared memory once (in the order the layers need them) and walks its
+// tiles; the 8 warps split each layer's inputs.  X, T and Y are host memory
+// mapped into the device (a batch is read and its outputs written once, over
+// the link, without separate copies).  For the weight gradients the inputs,
+// the activations and the deltas go to `keep`.
+template <int R>
+__global__ void __launch_bounds__(kPassThreads, 1)
+    PriorPass(const float* __restrict__ P, const float* __restrict__ X, const float* __restrict__ T, int64_t n,
+              float* __restrict__ Y, const PriorKeep keep) {
+  extern __shared__ __align__(16) unsigned char prior_smem[];
+  PassSmem<R>& s = *reinterpret_cast<PassSmem<R>*>(prior_smem);
+  float* const W1 = s.w;
+  float* const W2 = s.w + kIn * kPitch;
+  float* const W3 = W2 + kHid * kPitch;
+  CopyRowsAsync<kIn>(W1, P + JoinPrior::kOffW1);
+  CopyRowsAsync<kHid>(W2, P + JoinPrior::kOffW2);
+  CopyRowsAsync<kHid>(W3, P + JoinPrior::kOffW3);
+  for (int j = threadIdx.x; j < kHid; j += kPassThreads) {
+    s.b[j] = P[JoinPrior::kOffB1 + j];
+    s.b[kHid + j] = P[JoinPrior::kOffB2 + j];
+    s.b[2 * kHid + j] = P[JoinPrior::kOffB3 + j];
+    s.w4[j] = P[JoinPrior::kOffW4 + j];
+  }
+  const float b4 = P[JoinPrior::kOffB4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tiles = (n + R - 1) / R;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t row0 = tile * R;
+    for (int i = threadIdx.x; i < R * (kIn / 4); i += kPassThreads) {
+      const int64_t row = row0 + i / (kIn / 4);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row < n) {
+        v = reinterpret_cast<const float4*>(X)[row0 * (kIn / 4) + i];
+        if (T) reinterpret_cast<float4*>(keep.x)[row0 * (kIn / 4) + i] = v;
+      }
+      reinterpret_cast<float4*>(s.x)[i] = v;
+    }
+    // layer l's activations: to shared memory, and kept when training
+    auto relu = [&](int l) {
+      return [&, l](int r, int j, float v) {
+        v = fmaxf(v, 0.f);
+        s.h[l][r * kHid + j] = v;
+        if (T && row0 + r < n) keep.h[l][(row0 + r) * kHid + j] = v;
+      };
+    };
+    WaitCopies<2>();
+    DenseShare<R, kIn>(W1, s.x, s.part);
+    SumShares<R>(s.part, [&](int j) { return s.b[j]; }, relu(0));
+    WaitCopies<1>();
+    DenseShare<R, kHid>(W2, s.h[0], s.part);
+    SumShares<R>(s.part, [&](int j) { return s.b[kHid + j]; }, relu(1));
+    WaitCopies<0>();
+    DenseShare<R, kHid>(W3, s.h[1], s.part);
+    SumShares<R>(s.part, [&](int j) { return s.b[2 * kHid + j]; }, relu(2));
+    // head: one warp per row
+    for (int r = warp; r < R; r += kPassWarps) {
+      const float4 h = *reinterpret_cast<const float4*>(s.h[2] + r * kHid + 4 * lane);
+      const float4 w = *reinterpret_cast<const float4*>(s.w4 + 4 * lane);
+      const float y = WarpSum((h.x * w.x + h.y * w.y) + (h.z * w.z + h.w * w.w)) + b4;
+      if (lane == 0) {
+        float dy = 0.f;
+        if (row0 + r < n) {
+          Y[row0 + r] = y;
+          if (T) {
+            dy = 2.f * (y - T[row0 + r]) / static_cast<float>(n);
+            keep.dy[row0 + r] = dy;
+          }
+        }
+        s.dy[r] = dy;
+      }
+    }
+    if (!T) {
+      __syncthreads();  // the next tile overwrites x
+      continue;
+    }
+    __syncthreads();
+    auto delta = [&](int l, float* to) {
+      return [&, l, to](int r, int j, float v) {
+        v = s.h[l][r * kHid + j] > 0.f ? v : 0.f;
+        to[r * kHid + j] = v;
+        if (row0 + r < n) keep.d[l][(row0 + r) * kHid + j] = v;
+      };
+    };
+    for (int o = threadIdx.x; o < R * kHid; o += kPassThreads)
+      delta(2, s.d[0])(o / kHid, o % kHid, s.dy[o / kHid] * s.w4[o % kHid]);
+    __syncthreads();
+    auto zero = [](int) { return 0.f; };
+    DeltaShare<R>(W3, s.d[0], s.part);
+    SumShares<R>(s.part, zero, delta(1, s.d[1]));
+    DeltaShare<R>(W2, s.d[1], s.part);
+    SumShares<R>(s.part, zero, delta(0, s.d[0]));
+  }
+}
+
+// Gradient of mean((y - t)^2) over the batch and, with lr > 0, the Adam step
+// (Kingma & Ba, beta1 0.9, beta2 0.999, eps 1e-8).  A CTA owns 16 x 32 weights
+// of one layer over all rows: its 16 warps take every 16th row, eight rows'
+// loads in flight, and their sums meet in shared memory in warp order, so the
+// result is the same on every run and no per-CTA partials are written.
+// Four more CTAs own the biases and the head.
+constexpr int kGradK = 16, kGradJ = 32, kGradAhead = 8;
+constexpr int kGradTiles1 = (kIn / kGradK) * (kHid / kGradJ);
+constexpr int kGradTiles = (kHid / kGradK) * (kHid / kGradJ);
+constexpr int kGradBlocks = kGradTiles1 + 2 * kGradTiles + 4;
+static_assert(kGradK * kGradJ == kGradThreads, "one weight per thread");
+
+__global__ void __launch_bounds__(kGradThreads)
+    PriorGrad(float* __restrict__ P, const PriorKeep keep, int64_t n, float* __restrict__ m, float* __restrict__ v,
+              float* __restrict__ grad, float lr, float c1, float c2) {
+  __shared__ float part[kGradWarps * kGradThreads];
+  __shared__ float head[kGradWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto update = [&](int64_t p, float g) {
+    if (grad) grad[p] = g;
     if (lr > 0.f) {
       const float mp = 0.9f * m[p] + 0.1f * g;
       const float vp = 0.999f * v[p] + 0.001f * g * g;
@@ -200,7 +265,108 @@ __global__ void PriorAdam(float* __restrict__ P, const float* __restrict__ parti
       v[p] = vp;
       P[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + 1e-8f);
     }
+  };
+  int b = blockIdx.x;
+  if (b < kGradTiles1 + 2 * kGradTiles) {
+    int l = 0;
+    if (b >= kGradTiles1) {
+      b -= kGradTiles1;
+      l = 1 + b / kGradTiles;
+      b %= kGradTiles;
+    }
+    const int k0 = b / (kHid / kGradJ) * kGradK, j0 = b % (kHid / kGradJ) * kGradJ;
+    const int width = l == 0 ? kIn : kHid;
+    const float* in = (l == 0 ? keep.x : keep.h[l - 1]) + k0 + 4 * (lane >> 3);
+    const float* dz = keep.d[l] + j0 + 4 * (lane & 7);
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int64_t r0 = warp; r0 < n; r0 += kGradWarps * kGradAhead) {
+      float4 a[kGradAhead], d[kGradAhead];
+#pragma unroll
+      for (int u = 0; u < kGradAhead; u++) {
+        const int64_t r = r0 + u * kGradWarps;
+        a[u] = d[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < n) {
+          a[u] = *reinterpret_cast<const float4*>(in + r * width);
+          d[u] = *reinterpret_cast<const float4*>(dz + r * kHid);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kGradAhead; u++) {
+        const float x[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          acc[i][0] = fmaf(x[i], d[u].x, acc[i][0]);
+          acc[i][1] = fmaf(x[i], d[u].y, acc[i][1]);
+          acc[i][2] = fmaf(x[i], d[u].z, acc[i][2]);
+          acc[i][3] = fmaf(x[i], d[u].w, acc[i][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *reinterpret_cast<float4*>(part + warp * kGradThreads + (4 * (lane >> 3) + i) * kGradJ + 4 * (lane & 7)) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
+    float g = 0.f;
+#pragma unroll
+    for (int w = 0; w < kGradWarps; w++) g += part[w * kGradThreads + threadIdx.x];
+    const int64_t off = l == 0 ? JoinPrior::kOffW1 : l == 1 ? JoinPrior::kOffW2 : JoinPrior::kOffW3;
+    update(off + (k0 + threadIdx.x / kGradJ) * kHid + j0 + threadIdx.x % kGradJ, g);
+    return;
   }
+  // a layer's bias (the column sums of its deltas), or the head (the third
+  // layer's activations weighted by dy, and dy's own sum)
+  const int l = b - (kGradTiles1 + 2 * kGradTiles);
+  const bool is_head = l == 3;
+  const float* rows = (is_head ? keep.h[2] : keep.d[l]) + 4 * lane;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float sum = 0.f;
+  for (int64_t r0 = warp; r0 < n; r0 += kGradWarps * kGradAhead) {
+    float4 x[kGradAhead];
+    float f[kGradAhead];
+#pragma unroll
+    for (int u = 0; u < kGradAhead; u++) {
+      const int64_t r = r0 + u * kGradWarps;
+      x[u] = r < n ? *reinterpret_cast<const float4*>(rows + r * kHid) : make_float4(0.f, 0.f, 0.f, 0.f);
+      f[u] = r < n ? (is_head ? keep.dy[r] : 1.f) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kGradAhead; u++) {
+      acc.x = fmaf(f[u], x[u].x, acc.x);
+      acc.y = fmaf(f[u], x[u].y, acc.y);
+      acc.z = fmaf(f[u], x[u].z, acc.z);
+      acc.w = fmaf(f[u], x[u].w, acc.w);
+      sum += f[u];
+    }
+  }
+  *reinterpret_cast<float4*>(part + warp * kHid + 4 * lane) = acc;
+  if (lane == 0) head[warp] = sum;
+  __syncthreads();
+  if (threadIdx.x < kHid) {
+    float g = 0.f;
+    for (int w = 0; w < kGradWarps; w++) g += part[w * kHid + threadIdx.x];
+    const int64_t off = l == 0   ? JoinPrior::kOffB1
+                        : l == 1 ? JoinPrior::kOffB2
+                        : l == 2 ? JoinPrior::kOffB3
+                                 : JoinPrior::kOffW4;
+    update(off + threadIdx.x, g);
+  } else if (is_head && threadIdx.x == kHid) {
+    float g = 0.f;
+    for (int w = 0; w < kGradWarps; w++) g += head[w];
+    update(JoinPrior::kOffB4, g);
+  }
+}
+
+template <int R>
+void LaunchPass(const float* p, const float* x, const float* t, int64_t n, float* y, const PriorKeep& keep, int sms,
+                cudaStream_t s) {
+  constexpr int kSmem = static_cast<int>(sizeof(PassSmem<R>));
+  KDB_CUDA(cudaFuncSetAttribute(PriorPass<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  const int grid = static_cast<int>(std::min<int64_t>((n + R - 1) / R, sms));
+  PriorPass<R><<<grid, kPassThreads, kSmem, s>>>(p, x, t, n, y, keep);
+  KDB_CUDA(cudaGetLastError());
 }
 
 uint64_t SplitMix(uint64_t& s) {
@@ -215,17 +381,24 @@ uint64_t SplitMix(uint64_t& s) {
 JoinPrior::JoinPrior(int device, uint32_t seed) : device_(device) {
   KDB_CUDA(cudaSetDevice(device));
   KDB_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-  const int64_t nblk = kMaxRows / kRows;
+  KDB_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
   KDB_CUDA(cudaMalloc(&p_, sizeof(float) * kParams));
   KDB_CUDA(cudaMalloc(&m_, sizeof(float) * kParams));
   KDB_CUDA(cudaMalloc(&v_, sizeof(float) * kParams));
-  KDB_CUDA(cudaMalloc(&grad_, sizeof(float) * kParams));
-  KDB_CUDA(cudaMalloc(&x_, sizeof(float) * kMaxRows * kIn));
-  KDB_CUDA(cudaMalloc(&t_, sizeof(float) * kMaxRows));
-  KDB_CUDA(cudaMalloc(&y_, sizeof(float) * kMaxRows));
-  KDB_CUDA(cudaMalloc(&h_, sizeof(float) * 3 * kMaxRows * kHid));
-  KDB_CUDA(cudaMalloc(&partial_, sizeof(float) * nblk * kParams));
-  KDB_CUDA(cudaMallocHost(&pinned_, sizeof(float) * (kMaxRows * (kIn + 2) + kParams)));
+  // inputs, three activations, three deltas and dy of a batch
+  KDB_CUDA(cudaMalloc(&batch_, sizeof(float) * kMaxRows * (kIn + 6 * kHid + 1)));
+  keep_.x = batch_;
+  for (int l = 0; l < 3; l++) {
+    keep_.h[l] = batch_ + kMaxRows * (kIn + l * kHid);
+    keep_.d[l] = batch_ + kMaxRows * (kIn + (3 + l) * kHid);
+  }
+  keep_.dy = batch_ + kMaxRows * (kIn + 6 * kHid);
+  // a batch's inputs, targets and outputs, and the gradient: read and
+  // written by the kernels directly
+  KDB_CUDA(cudaHostAlloc(&pinned_, sizeof(float) * (kMaxRows * (kIn + 2) + kParams), cudaHostAllocMapped));
+  void* mapped = nullptr;
+  KDB_CUDA(cudaHostGetDevicePointer(&mapped, pinned_, 0));
+  mapped_ = static_cast<float*>(mapped);
   // He-uniform initialisation (bound sqrt(6 / fan_in)), zero biases
   std::vector<float> init(kParams, 0.f);
   uint64_t s = 0x6A09E667F3BCC909ULL ^ seed;
@@ -244,7 +417,7 @@ JoinPrior::JoinPrior(int device, uint32_t seed) : device_(device) {
 JoinPrior::~JoinPrior() {
   cudaSetDevice(device_);
   cudaStreamSynchronize(stream_);
-  for (float* p : {p_, m_, v_, grad_, x_, t_, y_, h_, partial_}) cudaFree(p);
+  for (float* p : {p_, m_, v_, batch_}) cudaFree(p);
   cudaFreeHost(pinned_);
   cudaStreamDestroy(stream_);
 }
@@ -273,36 +446,30 @@ double JoinPrior::Run(const float* x, const float* t, int64_t n, float* grad, fl
                                                               std::to_string(kMaxRows) + " rows");
   std::lock_guard<std::mutex> lock(mu_);
   KDB_CUDA(cudaSetDevice(device_));
-  const int nblk = static_cast<int>((n + kRows - 1) / kRows);
-  float* px = pinned_;
-  float* pt = pinned_ + kMaxRows * kIn;
-  float* py = pt + kMaxRows;
-  std::memcpy(px, x, sizeof(float) * n * kIn);
-  KDB_CUDA(cudaMemcpyAsync(x_, px, sizeof(float) * n * kIn, cudaMemcpyHostToDevice, stream_));
+  constexpr int64_t kOffT = kMaxRows * kIn, kOffY = kOffT + kMaxRows, kOffG = kOffY + kMaxRows;
+  const float* py = pinned_ + kOffY;
+  std::memcpy(pinned_, x, sizeof(float) * n * kIn);
+  if (t) std::memcpy(pinned_ + kOffT, t, sizeof(float) * n);
+  // Rows per tile: the fewest that let every tile have its own SM (a tile is
+  // a chain of layers, so a batch is done soonest spread wide), else 8, the
+  // CTAs walking their tiles with the weights in place.
+  const float* mt = t ? mapped_ + kOffT : nullptr;
+  if (n <= 2 * sms_) LaunchPass<2>(p_, mapped_, mt, n, mapped_ + kOffY, keep_, sms_, stream_);
+  else if (n <= 4 * sms_) LaunchPass<4>(p_, mapped_, mt, n, mapped_ + kOffY, keep_, sms_, stream_);
+  else LaunchPass<kMaxTileRows>(p_, mapped_, mt, n, mapped_ + kOffY, keep_, sms_, stream_);
   if (t) {
-    std::memcpy(pt, t, sizeof(float) * n);
-    KDB_CUDA(cudaMemcpyAsync(t_, pt, sizeof(float) * n, cudaMemcpyHostToDevice, stream_));
-  }
-  PriorForward<<<nblk, kThreads, 0, stream_>>>(p_, x_, n, y_, h_);
-  KDB_CUDA(cudaGetLastError());
-  if (t) {
-    PriorBackward<<<nblk, kThreads, 0, stream_>>>(p_, x_, h_, y_, t_, n, partial_);
-    KDB_CUDA(cudaGetLastError());
     float c1 = 1.f, c2 = 1.f;
     if (lr > 0.f) {
       step_++;
       c1 = static_cast<float>(1.0 - std::pow(0.9, static_cast<double>(step_)));
       c2 = static_cast<float>(1.0 - std::pow(0.999, static_cast<double>(step_)));
     }
-    PriorAdam<<<static_cast<int>((kParams + 255) / 256), 256, 0, stream_>>>(p_, partial_, nblk, m_, v_, grad_, lr,
-                                                                              c1, c2);
+    PriorGrad<<<kGradBlocks, kGradThreads, 0, stream_>>>(p_, keep_, n, m_, v_, grad ? mapped_ + kOffG : nullptr, lr, c1,
+                                                         c2);
     KDB_CUDA(cudaGetLastError());
-    if (grad) KDB_CUDA(cudaMemcpyAsync(pinned_ + kMaxRows * (kIn + 2), grad_, sizeof(float) * kParams,
-                                       cudaMemcpyDeviceToHost, stream_));
   }
-  KDB_CUDA(cudaMemcpyAsync(py, y_, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_));
   KDB_CUDA(cudaStreamSynchronize(stream_));
-  if (grad) std::memcpy(grad, pinned_ + kMaxRows * (kIn + 2), sizeof(float) * kParams);
+  if (grad) std::memcpy(grad, pinned_ + kOffG, sizeof(float) * kParams);
   double loss = 0;
   if (t)
     for (int64_t i = 0; i < n; i++) {

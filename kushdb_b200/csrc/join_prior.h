@@ -16,6 +16,15 @@ namespace kdb {
 
 class Context;
 
+// What a training batch's forward pass leaves on the device for the weight
+// gradients: inputs, the layers' activations and deltas, and the output's.
+struct PriorKeep {
+  float* x = nullptr;
+  float* h[3] = {nullptr, nullptr, nullptr};
+  float* d[3] = {nullptr, nullptr, nullptr};
+  float* dy = nullptr;
+};
+
 class JoinPrior {
  public:
   static constexpr int kIn = 64;
@@ -56,13 +65,11 @@ class JoinPrior {
   float* p_ = nullptr;  // parameters
   float* m_ = nullptr;  // Adam moments
   float* v_ = nullptr;
-  float* x_ = nullptr;
-  float* t_ = nullptr;
-  float* y_ = nullptr;
-  float* h_ = nullptr;        // saved activations H1, H2, H3
-  float* partial_ = nullptr;  // per-CTA gradient partials
-  float* grad_ = nullptr;
-  float* pinned_ = nullptr;
+  float* batch_ = nullptr;   // the memory of keep_
+  PriorKeep keep_;
+  float* pinned_ = nullptr;  // x, t, y of a batch and the gradient
+  float* mapped_ = nullptr;  // the same, as the device sees it
+  int sms_ = 148;
   int64_t step_ = 0;
 };
 

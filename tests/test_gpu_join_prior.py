@@ -140,3 +140,21 @@ def test_prior_needs_fewer_episodes_than_uct(engine):
     assert totals["prior"][1] < totals["uct"][1]
     assert totals["prior"][3] < totals["uct"][3]
     model.close()
+
+
+# rows per tile change at 2 and 4 rows per SM (148 of them), and past 8 per SM
+# a CTA walks several tiles; weight gradients take rows 128 at a time
+@pytest.mark.parametrize("rows", [2, 127, 129, 296, 297, 592, 593, 1185])
+def test_gradient_at_tile_edges_matches_oracle(engine, rows):
+    m, p = _random_model(engine, seed=rows)
+    rng = np.random.default_rng(rows)
+    x = rng.normal(0, 1, (rows, m.num_features)).astype(np.float32)
+    t = rng.normal(0, 1, rows).astype(np.float32)
+    ref, ref_loss = jp.gradient(p, x, t)
+    for _ in range(2):
+        g, loss = m.gradient(x, t)
+        assert np.all(np.abs(g - ref) <= 1e-4 * np.max(np.abs(ref)) + 1e-3 * np.abs(ref))
+        assert abs(loss - ref_loss) <= 1e-5 * (1 + ref_loss)
+    y, _ = jp.forward(p, x)
+    assert np.all(np.abs(m.forward(x) - y) <= 1e-4 * (1 + np.abs(y)))
+    m.close()
