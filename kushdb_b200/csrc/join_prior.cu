@@ -16,8 +16,9 @@ namespace {
 
 constexpr int kIn = JoinPrior::kIn;
 constexpr int kHid = JoinPrior::kHid;
-constexpr int kPassThreads = 256;  // forward / deltas: 8 warps
-constexpr int kPassWarps = kPassThreads / 32;
+constexpr int kPassThreads = 512;  // forward / deltas
+constexpr int kShares = 8;         // parts of a layer's inputs; two warps share one, half of the rows each
+static_assert(kPassThreads / 32 == 2 * kShares, "two warps per share");
 constexpr int kPitch = kHid + 4;   // floats per weight row in shared memory: rows four banks apart
 constexpr int kMaxTileRows = 8;
 constexpr int kGradThreads = 512;
@@ -33,7 +34,8 @@ struct PassSmem {
   float x[R * kIn];
   float h[3][R * kHid];
   float d[2][R * kHid];
-  float part[kPassWarps * R * kHid];
+  float part[kShares * R * kHid];
+  float t[R];
   float dy[R];
 };
 static_assert(sizeof(PassSmem<kMaxTileRows>) <= 227 * 1024, "fits an SM");
@@ -63,42 +65,42 @@ __device__ __forceinline__ void WaitCopies() {
   __syncthreads();
 }
 
-// Sums the warps' shares of R x kHid outputs in warp order from `first` on,
+// Sums the shares of R x kHid outputs in their order from `first` on,
 // and hands each to done(row, column, sum); ends with a barrier.
 template <int R, typename FIRST, typename DONE>
 __device__ __forceinline__ void SumShares(const float* part, FIRST first, DONE done) {
   __syncthreads();
-#pragma unroll
   for (int o = threadIdx.x; o < R * kHid; o += kPassThreads) {
     const int r = o / kHid, j = o % kHid;
     float s = first(j);
 #pragma unroll
-    for (int w = 0; w < kPassWarps; w++) s += part[w * R * kHid + o];
+    for (int w = 0; w < kShares; w++) s += part[w * R * kHid + o];
     done(r, j, s);
   }
   __syncthreads();
 }
 
-// Warp w's share of in (R x K) times W (K x kHid): inputs k in [w, w + 1) *
-// K / 8.  A lane owns 4 neighbouring outputs: a weight row is one 16-byte
-// load per lane, an input is the same word for the whole warp.
+// A warp's share of in (R x K) times W (K x kHid): one eighth of the inputs,
+// half of the rows.  A lane owns 4 neighbouring outputs: a weight row is one
+// 16-byte load per lane, an input is the same word for the whole warp.
 template <int R, int K>
 __device__ __forceinline__ void DenseShare(const float* W, const float* in, float* part) {
-  constexpr int kShare = K / kPassWarps;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k0 = warp * kShare;
-  float acc[R][4];
+  constexpr int kShare = K / kShares, H = R / 2;
+  const int lane = threadIdx.x & 31, share = (threadIdx.x >> 5) % kShares, r0 = (threadIdx.x >> 5) / kShares * H;
+  const int k0 = share * kShare;
+  float acc[H][4];
 #pragma unroll
-  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+  for (int r = 0; r < H; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
 #pragma unroll
   for (int k = 0; k < kShare; k += 4) {
-    float4 v[R];
+    float4 v[H];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = *reinterpret_cast<const float4*>(in + r * K + k0 + k);
+    for (int r = 0; r < H; r++) v[r] = *reinterpret_cast<const float4*>(in + (r0 + r) * K + k0 + k);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const float4 w = *reinterpret_cast<const float4*>(W + (k0 + k + i) * kPitch + 4 * lane);
 #pragma unroll
-      for (int r = 0; r < R; r++) {
+      for (int r = 0; r < H; r++) {
         const float s = i == 0 ? v[r].x : i == 1 ? v[r].y : i == 2 ? v[r].z : v[r].w;
         acc[r][0] = fmaf(s, w.x, acc[r][0]);
         acc[r][1] = fmaf(s, w.y, acc[r][1]);
@@ -108,44 +110,45 @@ __device__ __forceinline__ void DenseShare(const float* W, const float* in, floa
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; r++)
-    *reinterpret_cast<float4*>(part + (warp * R + r) * kHid + 4 * lane) =
+  for (int r = 0; r < H; r++)
+    *reinterpret_cast<float4*>(part + (share * R + r0 + r) * kHid + 4 * lane) =
         make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
 }
 
-// Warp w's share of dz (R x kHid) times W transposed: columns j in [w, w + 1)
-// * 16.  A lane owns outputs lane + 32 i, whose weight rows lie four banks
-// apart.
+// A warp's share of dz (R x kHid) times W transposed: one eighth of the
+// columns, half of the rows.  A lane owns outputs lane + 32 i, whose weight
+// rows lie four banks apart.
 template <int R>
 __device__ __forceinline__ void DeltaShare(const float* W, const float* dz, float* part) {
-  constexpr int kShare = kHid / kPassWarps;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = warp * kShare;
-  float acc[R][4];
+  constexpr int kShare = kHid / kShares, H = R / 2;
+  const int lane = threadIdx.x & 31, share = (threadIdx.x >> 5) % kShares, r0 = (threadIdx.x >> 5) / kShares * H;
+  const int j0 = share * kShare;
+  float acc[H][4];
 #pragma unroll
-  for (int r = 0; r < R; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+  for (int r = 0; r < H; r++) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
 #pragma unroll
   for (int j = 0; j < kShare; j += 4) {
-    float4 v[R];
+    float4 v[H];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = *reinterpret_cast<const float4*>(dz + r * kHid + j0 + j);
+    for (int r = 0; r < H; r++) v[r] = *reinterpret_cast<const float4*>(dz + (r0 + r) * kHid + j0 + j);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const float4 w = *reinterpret_cast<const float4*>(W + (lane + 32 * i) * kPitch + j0 + j);
 #pragma unroll
-      for (int r = 0; r < R; r++)
+      for (int r = 0; r < H; r++)
         acc[r][i] = fmaf(v[r].w, w.w, fmaf(v[r].z, w.z, fmaf(v[r].y, w.y, fmaf(v[r].x, w.x, acc[r][i]))));
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; r++)
+  for (int r = 0; r < H; r++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) part[(warp * R + r) * kHid + lane + 32 * i] = acc[r][i];
+    for (int i = 0; i < 4; i++) part[(share * R + r0 + r) * kHid + lane + 32 * i] = acc[r][i];
 }
 
 // Forward of every layer for tiles of R rows and, with targets, back to
 // every layer's pre-activation deltas.  Each CTA brings all weights into its
 // shared memory once (in the order the layers need them) and walks its
-// tiles; the 8 warps split each layer's inputs.  X, T and Y are host memory
+// tiles; the 16 warps split each layer's inputs and rows.  X, T and Y are host memory
 // mapped into the device (a batch is read and its outputs written once, over
 // the link, without separate copies).  For the weight gradients the inputs,
 // the activations and the deltas go to `keep`.
@@ -181,6 +184,11 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       }
       reinterpret_cast<float4*>(s.x)[i] = v;
     }
+    // (with the inputs: a read over the link takes about 2 us)
+    if (T && threadIdx.x >= kPassThreads - R) {
+      const int r = threadIdx.x - (kPassThreads - R);
+      s.t[r] = row0 + r < n ? T[row0 + r] : 0.f;
+    }
     // layer l's activations: to shared memory, and kept when training
     auto relu = [&](int l) {
       return [&, l](int r, int j, float v) {
@@ -199,7 +207,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     DenseShare<R, kHid>(W3, s.h[1], s.part);
     SumShares<R>(s.part, [&](int j) { return s.b[2 * kHid + j]; }, relu(2));
     // head: one warp per row
-    for (int r = warp; r < R; r += kPassWarps) {
+    for (int r = warp; r < R; r += kPassThreads / 32) {
       const float4 h = *reinterpret_cast<const float4*>(s.h[2] + r * kHid + 4 * lane);
       const float4 w = *reinterpret_cast<const float4*>(s.w4 + 4 * lane);
       const float y = WarpSum((h.x * w.x + h.y * w.y) + (h.z * w.z + h.w * w.w)) + b4;
@@ -208,7 +216,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         if (row0 + r < n) {
           Y[row0 + r] = y;
           if (T) {
-            dy = 2.f * (y - T[row0 + r]) / static_cast<float>(n);
+            dy = 2.f * (y - s.t[r]) / static_cast<float>(n);
             keep.dy[row0 + r] = dy;
           }
         }
@@ -281,29 +289,31 @@ __global__ void __launch_bounds__(kGradThreads)
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    for (int64_t r0 = warp; r0 < n; r0 += kGradWarps * kGradAhead) {
+    auto add = [&](const float4& a, const float4& d) {
+      const float x[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        acc[i][0] = fmaf(x[i], d.x, acc[i][0]);
+        acc[i][1] = fmaf(x[i], d.y, acc[i][1]);
+        acc[i][2] = fmaf(x[i], d.z, acc[i][2]);
+        acc[i][3] = fmaf(x[i], d.w, acc[i][3]);
+      }
+    };
+    int64_t r = warp;
+    // (whole batches without a test per row: with one the compiler takes
+    // the rows' loads one after the other, 125 us for 4096 rows)
+    for (; r + (kGradAhead - 1) * kGradWarps < n; r += kGradAhead * kGradWarps) {
       float4 a[kGradAhead], d[kGradAhead];
 #pragma unroll
       for (int u = 0; u < kGradAhead; u++) {
-        const int64_t r = r0 + u * kGradWarps;
-        a[u] = d[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < n) {
-          a[u] = *reinterpret_cast<const float4*>(in + r * width);
-          d[u] = *reinterpret_cast<const float4*>(dz + r * kHid);
-        }
+        a[u] = __ldcg(reinterpret_cast<const float4*>(in + (r + u * kGradWarps) * width));
+        d[u] = __ldcg(reinterpret_cast<const float4*>(dz + (r + u * kGradWarps) * kHid));
       }
 #pragma unroll
-      for (int u = 0; u < kGradAhead; u++) {
-        const float x[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          acc[i][0] = fmaf(x[i], d[u].x, acc[i][0]);
-          acc[i][1] = fmaf(x[i], d[u].y, acc[i][1]);
-          acc[i][2] = fmaf(x[i], d[u].z, acc[i][2]);
-          acc[i][3] = fmaf(x[i], d[u].w, acc[i][3]);
-        }
-      }
+      for (int u = 0; u < kGradAhead; u++) add(a[u], d[u]);
     }
+    for (; r < n; r += kGradWarps)
+      add(*reinterpret_cast<const float4*>(in + r * width), *reinterpret_cast<const float4*>(dz + r * kHid));
 #pragma unroll
     for (int i = 0; i < 4; i++)
       *reinterpret_cast<float4*>(part + warp * kGradThreads + (4 * (lane >> 3) + i) * kGradJ + 4 * (lane & 7)) =
@@ -323,24 +333,27 @@ __global__ void __launch_bounds__(kGradThreads)
   const float* rows = (is_head ? keep.h[2] : keep.d[l]) + 4 * lane;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float sum = 0.f;
-  for (int64_t r0 = warp; r0 < n; r0 += kGradWarps * kGradAhead) {
+  auto add = [&](const float4& x, float f) {
+    acc.x = fmaf(f, x.x, acc.x);
+    acc.y = fmaf(f, x.y, acc.y);
+    acc.z = fmaf(f, x.z, acc.z);
+    acc.w = fmaf(f, x.w, acc.w);
+    sum += f;
+  };
+  int64_t r = warp;
+  for (; r + (kGradAhead - 1) * kGradWarps < n; r += kGradAhead * kGradWarps) {
     float4 x[kGradAhead];
     float f[kGradAhead];
 #pragma unroll
     for (int u = 0; u < kGradAhead; u++) {
-      const int64_t r = r0 + u * kGradWarps;
-      x[u] = r < n ? *reinterpret_cast<const float4*>(rows + r * kHid) : make_float4(0.f, 0.f, 0.f, 0.f);
-      f[u] = r < n ? (is_head ? keep.dy[r] : 1.f) : 0.f;
+      x[u] = __ldcg(reinterpret_cast<const float4*>(rows + (r + u * kGradWarps) * kHid));
+      f[u] = is_head ? __ldcg(keep.dy + r + u * kGradWarps) : 1.f;
     }
 #pragma unroll
-    for (int u = 0; u < kGradAhead; u++) {
-      acc.x = fmaf(f[u], x[u].x, acc.x);
-      acc.y = fmaf(f[u], x[u].y, acc.y);
-      acc.z = fmaf(f[u], x[u].z, acc.z);
-      acc.w = fmaf(f[u], x[u].w, acc.w);
-      sum += f[u];
-    }
+    for (int u = 0; u < kGradAhead; u++) add(x[u], f[u]);
   }
+  for (; r < n; r += kGradWarps)
+    add(*reinterpret_cast<const float4*>(rows + r * kHid), is_head ? keep.dy[r] : 1.f);
   *reinterpret_cast<float4*>(part + warp * kHid + 4 * lane) = acc;
   if (lane == 0) head[warp] = sum;
   __syncthreads();
