@@ -826,16 +826,8 @@ class Executor {
   MatBuffer SmallOrderBy(const Operator& op, MatBuffer& m);
   MatBuffer LargeOrderBy(const Operator& op, MatBuffer& m);
   // Returns true when it also counted ties into *ties (range sort taken).
-  bool SortItems(uint64_t* items, int64_t n, unsigned long long* ties = nullptr, uint32_t tie_mask = 0,
-                 const unsigned long long* key_range = nullptr);
-  // KDB_ORDER_FUSED_RANGE: the kernel that makes the items also reduces
-  // their key range for the range-bucket sort (one 64-bit atomic min and max
-  // per warp).  Measured slower on the Q3 ORDER BY (step 217-219 against
-  // 214-216 us): thousands of warps' atomics queue on the two words, where
-  // the sort's own 32-CTA pass issues 64.
-  bool KeyRangeWanted() const {
-    return ctx_.OptStr("KDB_ORDER_FUSED_RANGE") && !ctx_.OptStr("KDB_ORDER_MERGE") && !ctx_.OptStr("KDB_ORDER_SAMPLE");
-  }
+  bool SortItems(uint64_t* items, int64_t n, const Context::ItemKeys& keys, unsigned long long* ties = nullptr,
+                 uint32_t tie_mask = 0);
   // set while materialising an ORDER BY's output: the sorted items, whose
   // high words hold the rows (read by EmitMatScan instead of an index array)
   const uint64_t* order_items_ = nullptr;
@@ -2030,6 +2022,7 @@ MatBuffer Executor::MaterializeCounted(const Operator& op, const std::function<v
   EmitStream(ks, eg, op, sink, src_rows2);
   LaunchPipeline(ks, src_rows2, "materialize", block);
   out.rows = produced;
+  out.pos_bound = PosBound(op);
   return out;
 }
 
@@ -3818,20 +3811,19 @@ MatBuffer Executor::SmallOrderBy(const Operator& op, MatBuffer& m) {
   return MaterializeStream(op, idx, &m);
 }
 
-// (key, tie) order of 16-byte items: the range-bucket sort (16384
-// equal-width key buckets, each item ranked within its bucket), falling
+// (key, tie) order of 16-byte items: the range-bucket sort (equal-width key
+// buckets of a few items, each item ranked within its bucket), falling
 // back to the block sort plus merge passes when a bucket holds more than
 // 1024 items (many equal keys); KDB_ORDER_MERGE forces the merge passes and
 // KDB_ORDER_SAMPLE a sample sort (splitters from a sorted sample).  On the
 // 134k-item ORDER BY of the Q3-shape query the query steps at 228 us with
 // the range sort against 241 us with the merge passes (198 / 211 us with
 // Zipf keys); the sample sort was slower than both.
-bool Executor::SortItems(uint64_t* items, int64_t n, unsigned long long* ties, uint32_t tie_mask,
-                         const unsigned long long* key_range) {
+bool Executor::SortItems(uint64_t* items, int64_t n, const Context::ItemKeys& keys, unsigned long long* ties,
+                         uint32_t tie_mask) {
   if (ctx_.OptStr("KDB_ORDER_SAMPLE") && ctx_.SampleSortItems(items, n, arena_)) return false;
   if (!ctx_.OptStr("KDB_ORDER_MERGE") && !ctx_.OptStr("KDB_ORDER_SAMPLE") &&
-      ctx_.RangeSortItems(items, n, arena_, ctx_.OptStr("KDB_ORDER_TIE_PASS") ? nullptr : ties, tie_mask,
-                          KeyRangeWanted() ? key_range : nullptr))
+      ctx_.RangeSortItems(items, n, arena_, keys, ctx_.OptStr("KDB_ORDER_TIE_PASS") ? nullptr : ties, tie_mask))
     return ties != nullptr && !ctx_.OptStr("KDB_ORDER_TIE_PASS");
   ctx_.MergeSortItems(items, n, arena_);
   return false;
@@ -3862,6 +3854,10 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
           ks.L(I + "[i] = (uint32_t)i;");
           return std::string("0ULL");
         });
+      } else if (m.pos_bound >= 0) {
+        // positions are distinct row numbers: a row's place is the number
+        // of positions below its own (a bitmap of them), without a sort
+        ctx_.OrderPositions(m.pos, n, m.pos_bound, idx, arena_);
       } else {
         keygen([&](KernelSource& ks, ExprGen&, const std::string& I) {
           std::string P = ks.Ptr(m.pos, "uint64_t", true);
@@ -3890,22 +3886,23 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
       // stream_ties: rows in stream order (idx) with the reference merge
       // sort's tie rank; otherwise rows in buffer order with the row index
       // as a provisional (unique) tie
-      // the items' key range, reduced while they are made (the range-bucket
-      // sort then needs no pass of its own for it)
-      unsigned long long* key_range = KeyRangeWanted() ? arena_.AllocT<unsigned long long>(2) : nullptr;
+      // the items' key range {min key, min complement}, reduced while they
+      // are made: one atomic pair per block (one per warp queues thousands
+      // of warps on the two words, slower than a pass of its own)
+      Context::ItemKeys item_keys;
+      item_keys.range = arena_.AllocT<unsigned long long>(2);
+      item_keys.tie_bits = depth;
+      item_keys.key_bit_in_tie = mc.nullable;
       auto make_items = [&](bool stream_ties) {
         KernelSource ks;
         ExprGen eg(ctx_, ks);
         std::string IT = ks.Ptr(items, "uint64_t"), I = ks.Ptr(idx, "uint32_t", true);
         std::string D = ks.Ptr(mc.data, StoreType(t), true);
         std::string N = ks.Word(static_cast<uint64_t>(n));
-        std::string KR;
-        if (key_range) {
-          ctx_.Memset(key_range, 0xff, sizeof(unsigned long long));
-          ctx_.Memset(key_range + 1, 0, sizeof(unsigned long long));
-          KR = ks.Ptr(key_range, "unsigned long long");
-          ks.L("unsigned long long kdb_klo = ~0ULL, kdb_khi = 0ULL;");
-        }
+        ctx_.Memset(item_keys.range, 0xff, 2 * sizeof(unsigned long long));
+        const std::string KR = ks.Ptr(item_keys.range, "unsigned long long");
+        ks.L("__shared__ uint64_t kdb_range_scratch[32];");
+        ks.L("uint64_t kdb_klo = ~0ULL, kdb_khi = ~0ULL;  // of the keys, of their complements");
         ks.Open("for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)" + N +
                 "; i += (int64_t)gridDim.x * blockDim.x)");
         ks.L(std::string("const uint32_t row = ") + (m.pos_is_index || !stream_ties ? "(uint32_t)i" : I + "[i]") +
@@ -3932,18 +3929,13 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
           ks.L(IT + "[2 * i] = (flag << 63) | (k >> 1);");
           ks.L(IT + "[2 * i + 1] = ((k & 1ULL) << 31) | " + tie + " | ((uint64_t)row << 32);");
         }
-        if (key_range) {
-          ks.L("{ const unsigned long long kk = " + IT + "[2 * i]; kdb_klo = kk < kdb_klo ? kk : kdb_klo; "
-               "kdb_khi = kk > kdb_khi ? kk : kdb_khi; }");
-        }
+        ks.L("{ const uint64_t kk = " + IT + "[2 * i]; kdb_klo = kk < kdb_klo ? kk : kdb_klo; "
+             "kdb_khi = ~kk < kdb_khi ? ~kk : kdb_khi; }");
         ks.Close();
-        if (key_range) {
-          ks.L("for (int o = 16; o > 0; o >>= 1) { const unsigned long long a = __shfl_xor_sync(0xffffffffu, kdb_klo, o), "
-               "b = __shfl_xor_sync(0xffffffffu, kdb_khi, o); kdb_klo = a < kdb_klo ? a : kdb_klo; "
-               "kdb_khi = b > kdb_khi ? b : kdb_khi; }");
-          ks.L("if ((threadIdx.x & 31) == 0 && kdb_klo <= kdb_khi) { atomicMin(&" + KR + "[0], kdb_klo); atomicMax(&" + KR +
-               "[1], kdb_khi); }");
-        }
+        ks.L("kdb_klo = kdb_block_reduce(kdb_klo, KdbMinU64(), kdb_range_scratch);");
+        ks.L("kdb_khi = kdb_block_reduce(kdb_khi, KdbMinU64(), kdb_range_scratch);");
+        ks.L("if (threadIdx.x == 0 && kdb_klo <= ~kdb_khi) { atomicMin(&" + KR + "[0], kdb_klo); atomicMin(&" + KR +
+             "[1], kdb_khi); }");
         LaunchPipeline(ks, n, "order key");
       };
       auto order_rows = [&]() {
@@ -3968,17 +3960,23 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
         order_items_ = nullptr;
         return out;
       };
-      if (!m.pos_is_index && !ctx_.OptStr("KDB_ORDER_TIE_SORT")) {
+      // Integer-like keys mostly tie, and the stream order of rows with known
+      // positions costs four small launches (a date key over 1M rows: 488 us
+      // per query against 1409 when it is sorted twice); a float key rarely
+      // ties, and those launches are then for nothing (50k rows: 87 against
+      // 78 us).
+      const bool likely_ties = t != TypeId::REAL && m.pos_bound >= 0;
+      if (!m.pos_is_index && !likely_ties && !ctx_.OptStr("KDB_ORDER_TIE_SORT")) {
         // Rows not in stream order (groups in table order): sort by the key
         // alone and look for equal neighbours.  Without ties the tie rank
-        // never decides, and the stream-order sort is not needed.
+        // never decides, and the stream order is not needed.
         make_items(false);
         uint64_t* ties = arena_.AllocT<uint64_t>(1);
         ctx_.Memset(ties, 0, sizeof(uint64_t));
         // the range sort counts ties while it ranks (equal keys share a
         // bucket); after the other sorts a pass compares neighbours
-        if (!SortItems(items, n, reinterpret_cast<unsigned long long*>(ties), mc.nullable ? 0x80000000u : 0u,
-                       key_range)) {
+        if (!SortItems(items, n, item_keys, reinterpret_cast<unsigned long long*>(ties),
+                       mc.nullable ? 0x80000000u : 0u)) {
           KernelSource ks;
           std::string IT = ks.Ptr(items, "uint64_t", true), T = ks.Ptr(ties, "unsigned long long");
           std::string N = ks.Word(static_cast<uint64_t>(n));
@@ -3994,7 +3992,7 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
       }
       stream_order();
       make_items(true);
-      SortItems(items, n, nullptr, 0, key_range);
+      SortItems(items, n, item_keys);
       return sorted_output();
     }
     stream_order();

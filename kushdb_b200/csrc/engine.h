@@ -84,6 +84,7 @@ struct MatBuffer {
   std::vector<MatCol> cols;
   uint64_t* pos = nullptr;   // stream position of each row (reference emission order key)
   bool pos_is_index = false;  // pos[r] == r: rows are already in stream order
+  int64_t pos_bound = -1;     // positions are distinct numbers below this (-1: not known)
   int64_t rows = 0;
   int64_t cap = 0;
 };
@@ -384,14 +385,23 @@ class Context {
   // shared-memory sort per bucket); false, with the items untouched, when a
   // bucket came out too large (the caller then merge sorts)
   bool SampleSortItems(void* items, int64_t n, Arena& arena);
+  // What the range-bucket sort has to know of its items: {min key, min
+  // complemented key} on the device, the ties' bits, and whether the tie
+  // word's top bit is the key's lowest bit.
+  struct ItemKeys {
+    unsigned long long* range = nullptr;
+    int tie_bits = 32;
+    bool key_bit_in_tie = false;
+  };
   // (key, tie) order by key-range buckets; false (nothing done) when a
-  // bucket is too large for one CTA's shared memory
-  // With `ties` (zeroed by the caller), also counts the items whose key
-  // (and tie bits under `tie_mask`) another item shares.
-  // With `key_range` (min and max of the items' keys, already on the
-  // device), no pass computes it.
-  bool RangeSortItems(void* items, int64_t n, Arena& arena, unsigned long long* ties = nullptr,
-                      uint32_t tie_mask = 0, const unsigned long long* key_range = nullptr);
+  // bucket holds too many items.  With `ties` (zeroed by the caller), also
+  // counts the items whose key (and tie bits under `tie_mask`) another item
+  // shares.
+  bool RangeSortItems(void* items, int64_t n, Arena& arena, const ItemKeys& keys, unsigned long long* ties = nullptr,
+                      uint32_t tie_mask = 0);
+  // idx[k] = the row with the k-th smallest of n distinct positions below
+  // `bound`
+  void OrderPositions(const uint64_t* pos, int64_t n, int64_t bound, uint32_t* idx, Arena& arena);
   // fills the places of a bitmap of groups' first rows (first_rows.cuh;
   // OrderWordsFor(rows) words) and writes the number of groups to *count
   void OrderFirstRows(void* words, int64_t rows, uint64_t* count, Arena& arena);

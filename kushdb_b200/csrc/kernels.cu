@@ -1014,159 +1014,167 @@ __global__ void SampleBucketSort(const SortItem* __restrict__ src, const unsigne
 
 // ---------------------------------------------------------------------------
 // Range-bucket sort of 16-byte items by (key, tie): the keys' minimum and
-// maximum split the key range into kRangeBuckets equal-width buckets (a
-// bucket index never decreases with the key), one pass counts them, one
-// block scans the counts, one pass scatters every item into its bucket's
-// range, and then every item finds its final slot itself: its bucket's
-// start plus the number of items in the same bucket that order before it.
-// With many narrow buckets each item compares itself with a few dozen
-// others, all in parallel (no per-bucket sort whose largest bucket sets the
-// time).  Equal keys share a bucket, so many ties (or a very skewed range)
-// make a bucket larger than kRangeBucketCap; the caller then uses the merge
-// sort.
+// maximum split the key range into equal-width buckets (a bucket index never
+// decreases with the key), one pass counts them, two scan the counts, one
+// scatters every item into its bucket's range, and then every item finds its
+// final slot itself: its bucket's start plus the number of items in the same
+// bucket that order before it.  An item compares itself with its whole
+// bucket, so the buckets are many: about 4 items each (with 16384 buckets,
+// 61 items each, scattering and ranking 1M items took 208 us, against 52).  Where the
+// keys have fewer distinct values than buckets (dates), a key's buckets
+// divide its items by their ties, which spread evenly.  Equal keys whose ties
+// are not to be divided, or a very skewed range, can make a bucket larger
+// than kRangeBucketCap; the caller then uses the merge sort.
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kRangeBuckets = 16384;
+constexpr int kMinRangeBuckets = 16384, kMaxRangeBuckets = 1 << 21;
 constexpr int kRangeThreads = 1024;
+constexpr int kRangePart = 4 * kRangeThreads;  // buckets per CTA of the offset passes
 constexpr unsigned kRangeBucketCap = 1024;  // items one bucket may hold
 
-__global__ void __launch_bounds__(kRangeThreads) RangeMinMax(const SortItem* __restrict__ items, int64_t n,
-                                                             unsigned long long* __restrict__ mm) {
-  __shared__ unsigned long long slo[kRangeThreads / 32], shi[kRangeThreads / 32];
-  unsigned long long lo = ~0ULL, hi = 0;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const unsigned long long k = items[i].key;
-    lo = k < lo ? k : lo;
-    hi = k > hi ? k : hi;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
-    lo = a < lo ? a : lo;
-    hi = b > hi ? b : hi;
-  }
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    slo[warp] = lo;
-    shi[warp] = hi;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < nw; w++) {
-      lo = slo[w] < lo ? slo[w] : lo;
-      hi = shi[w] > hi ? shi[w] : hi;
-    }
-    atomicMin(&mm[0], lo);
-    atomicMax(&mm[1], hi);
-  }
-}
+// How items map to buckets (the same on every thread that asks).
+struct RangeMap {
+  unsigned long long lo;
+  double scale;      // buckets per key, when a bucket holds whole keys
+  unsigned divide;   // buckets per key, when a key has several (else 0)
+  int buckets, tie_bits;
+  bool key_bit_in_tie;
 
-__device__ __forceinline__ unsigned RangeBucket(unsigned long long k, unsigned long long lo, unsigned long long range) {
-  // (k - lo) / (range + 1) * B in doubles: rounding keeps it monotonic
-  const double f = static_cast<double>(k - lo) / (static_cast<double>(range) + 1.0);
-  const int b = static_cast<int>(f * kRangeBuckets);
-  return b < 0 ? 0u : (b >= kRangeBuckets ? static_cast<unsigned>(kRangeBuckets - 1) : static_cast<unsigned>(b));
+  __device__ RangeMap(const unsigned long long* range, int b, int tb, bool kb, bool divide_keys)
+      : lo(range[0]), buckets(b), tie_bits(tb), key_bit_in_tie(kb) {
+    const unsigned long long span = ~range[1] - range[0];
+    divide = divide_keys && span < static_cast<unsigned long long>(b) / 2 ? b / static_cast<unsigned>(span + 1) : 0u;
+    scale = static_cast<double>(b) / (static_cast<double>(span) + 1.0);
+  }
+  __device__ __forceinline__ unsigned Of(const SortItem& x) const {
+    const unsigned long long k = x.key - lo;
+    if (divide) {
+      // ties are below 2^tie_bits; a key bit in the tie's top bit orders first
+      unsigned sub;
+      if (key_bit_in_tie)
+        sub = (x.tie >> 31) * (divide / 2) +
+              static_cast<unsigned>((static_cast<unsigned long long>(x.tie & 0x7fffffffu) * (divide / 2)) >> tie_bits);
+      else
+        sub = static_cast<unsigned>((static_cast<unsigned long long>(x.tie) * divide) >> tie_bits);
+      return static_cast<unsigned>(k) * divide + sub;
+    }
+    // the conversion and the product round, but never decrease with the key
+    const unsigned b = static_cast<unsigned>(static_cast<double>(k) * scale);
+    return b < static_cast<unsigned>(buckets) ? b : static_cast<unsigned>(buckets - 1);
+  }
+};
+
+struct RangeArgs {
+  const unsigned long long* range;
+  int buckets, tie_bits;
+  bool key_bit_in_tie, divide;
+};
+__device__ __forceinline__ RangeMap MapOf(const RangeArgs& a) {
+  return RangeMap(a.range, a.buckets, a.tie_bits, a.key_bit_in_tie, a.divide);
 }
 
 // bucket counts (global; few items per bucket, so the atomics rarely meet)
-__global__ void RangeCount(const SortItem* __restrict__ items, int64_t n, const unsigned long long* __restrict__ mm,
-                           uint16_t* __restrict__ bucket_of, unsigned* __restrict__ counts) {
-  const unsigned long long lo = mm[0], range = mm[1] - mm[0];
+__global__ void RangeCount(const SortItem* __restrict__ items, int64_t n, const RangeArgs a,
+                           unsigned* __restrict__ counts) {
+  const RangeMap map = MapOf(a);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const unsigned b = RangeBucket(items[i].key, lo, range);
-    bucket_of[i] = static_cast<uint16_t>(b);
-    atomicAdd(&counts[b], 1u);
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    atomicAdd(&counts[map.Of(items[i])], 1u);
+}
+
+// items in every part of kRangePart buckets; the largest bucket into *largest
+__global__ void __launch_bounds__(kRangeThreads) RangePartSums(const unsigned* __restrict__ counts,
+                                                               unsigned* __restrict__ sums,
+                                                               unsigned* __restrict__ largest) {
+  __shared__ unsigned ws[32], wm[32];
+  const uint4 c = reinterpret_cast<const uint4*>(counts)[blockIdx.x * kRangeThreads + threadIdx.x];
+  const unsigned m = __reduce_max_sync(0xffffffffu, max(max(c.x, c.y), max(c.z, c.w)));
+  const unsigned s = __reduce_add_sync(0xffffffffu, c.x + c.y + c.z + c.w);
+  if ((threadIdx.x & 31) == 0) {
+    ws[threadIdx.x >> 5] = s;
+    wm[threadIdx.x >> 5] = m;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const unsigned total = __reduce_add_sync(0xffffffffu, ws[threadIdx.x]);
+    const unsigned most = __reduce_max_sync(0xffffffffu, wm[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      sums[blockIdx.x] = total;
+      atomicMax(largest, most);
+    }
   }
 }
 
-// one block: exclusive bucket offsets (offs[B] = total), each bucket's
-// cursor set to its offset, the largest bucket into *largest
+// exclusive bucket offsets (offs[B] = n) and each bucket's cursor, set to it
 __global__ void __launch_bounds__(kRangeThreads) RangeOffsets(const unsigned* __restrict__ counts,
+                                                              const unsigned* __restrict__ sums,
                                                               unsigned* __restrict__ offs,
-                                                              unsigned* __restrict__ cursor,
-                                                              unsigned* __restrict__ largest) {
-  constexpr int kPer = kRangeBuckets / kRangeThreads;
-  __shared__ unsigned ws[32], wmax[32];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  static_assert(kPer % 4 == 0, "whole 16-byte vectors per thread");
-  unsigned c[kPer], tot = 0, mx = 0;
-  // a thread's buckets as 16-byte vectors (a warp reads 2 KiB contiguously)
+                                                              unsigned* __restrict__ cursor) {
+  static_assert(kMaxRangeBuckets / kRangePart <= kRangeThreads, "one earlier part per thread");
+  __shared__ unsigned ws[32], wb[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned before =
+      __reduce_add_sync(0xffffffffu, threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0u);
+  const int64_t at = blockIdx.x * static_cast<int64_t>(kRangeThreads) + threadIdx.x;
+  const uint4 c = reinterpret_cast<const uint4*>(counts)[at];
+  const unsigned mine = c.x + c.y + c.z + c.w;
+  unsigned incl = mine;
 #pragma unroll
-  for (int q = 0; q < kPer / 4; q++) {
-    const uint4 v = reinterpret_cast<const uint4*>(counts + t * kPer)[q];
-    c[4 * q] = v.x;
-    c[4 * q + 1] = v.y;
-    c[4 * q + 2] = v.z;
-    c[4 * q + 3] = v.w;
-  }
-#pragma unroll
-  for (int q = 0; q < kPer; q++) {
-    tot += c[q];
-    mx = c[q] > mx ? c[q] : mx;
-  }
-  unsigned incl = tot;
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
-    const unsigned z = __shfl_xor_sync(0xffffffffu, mx, o);
-    mx = z > mx ? z : mx;
   }
   if (lane == 31) ws[warp] = incl;
-  if (lane == 0) wmax[warp] = mx;
+  if (lane == 0) wb[warp] = before;
   __syncthreads();
   if (warp == 0) {
-    unsigned v = ws[lane], m = wmax[lane];
+    const unsigned w = ws[lane];
+    unsigned wi = w;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += y;
-      const unsigned z = __shfl_xor_sync(0xffffffffu, m, o);
-      m = z > m ? z : m;
+      const unsigned y = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += y;
     }
-    ws[lane] = v;  // inclusive per warp
-    if (lane == 0) *largest = m;
+    ws[lane] = wi - w + __reduce_add_sync(0xffffffffu, wb[lane]);
   }
   __syncthreads();
-  unsigned run = (warp ? ws[warp - 1] : 0u) + incl - tot;
-#pragma unroll
-  for (int q = 0; q < kPer / 4; q++) {
-    uint4 v;
-    v.x = run;
-    v.y = v.x + c[4 * q];
-    v.z = v.y + c[4 * q + 1];
-    v.w = v.z + c[4 * q + 2];
-    run = v.w + c[4 * q + 3];
-    reinterpret_cast<uint4*>(offs + t * kPer)[q] = v;
-    reinterpret_cast<uint4*>(cursor + t * kPer)[q] = v;
-  }
-  if (t == kRangeThreads - 1) offs[kRangeBuckets] = run;
+  uint4 o;
+  o.x = ws[warp] + incl - mine;
+  o.y = o.x + c.x;
+  o.z = o.y + c.y;
+  o.w = o.z + c.z;
+  reinterpret_cast<uint4*>(offs)[at] = o;
+  reinterpret_cast<uint4*>(cursor)[at] = o;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kRangeThreads - 1)
+    offs[static_cast<int64_t>(gridDim.x) * kRangePart] = o.w + c.w;
 }
 
 // every item into its bucket's range (in any order within the bucket)
-__global__ void RangeScatter(const SortItem* __restrict__ items, int64_t n, const uint16_t* __restrict__ bucket_of,
-                             unsigned* __restrict__ cursor, SortItem* __restrict__ out, uint16_t* __restrict__ out_bucket) {
+__global__ void RangeScatter(const SortItem* __restrict__ items, int64_t n, const RangeArgs a,
+                             unsigned* __restrict__ cursor, SortItem* __restrict__ out) {
+  const RangeMap map = MapOf(a);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const unsigned b = bucket_of[i];
-    const unsigned pos = atomicAdd(&cursor[b], 1u);
-    out[pos] = items[i];
-    out_bucket[pos] = static_cast<uint16_t>(b);
+    const SortItem x = items[i];
+    out[atomicAdd(&cursor[map.Of(x)], 1u)] = x;
   }
 }
 
 // every item to its bucket's start plus the number of its bucket's items
 // that order before it ((key, tie) pairs are unique: distinct slots).  With
-// `ties`, an item whose key another item of its bucket shares (and, under
-// `tie_mask`, the same masked tie bits) counts into *ties: equal keys always
-// share a bucket, so this finds every tie of the sorted sequence.
-__global__ void RangeRank(const SortItem* __restrict__ src, const uint16_t* __restrict__ bucket, int64_t n,
+// `ties` (keys not divided), an item whose key another item of its bucket
+// shares (and, under `tie_mask`, the same masked tie bits) counts into *ties:
+// equal keys then always share a bucket, so this finds every tie of the
+// sorted sequence.
+__global__ void RangeRank(const SortItem* __restrict__ src, int64_t n, const RangeArgs a,
                           const unsigned* __restrict__ offs, SortItem* __restrict__ dst,
                           unsigned long long* __restrict__ ties, uint32_t tie_mask) {
+  const RangeMap map = MapOf(a);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const SortItem x = src[i];
-    const unsigned b = bucket[i], b0 = offs[b], b1 = offs[b + 1];
+    const unsigned b = map.Of(x), b0 = offs[b], b1 = offs[b + 1];
     unsigned r = b0;
     bool tie = false;
     for (unsigned j = b0; j < b1; j++) {
@@ -1179,35 +1187,64 @@ __global__ void RangeRank(const SortItem* __restrict__ src, const uint16_t* __re
   }
 }
 
+__global__ void MarkPositions(const uint64_t* __restrict__ pos, int64_t n, FirstWord* __restrict__ words) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    atomicOr(&words[pos[i] >> 5].bits, 1u << (pos[i] & 31));
+}
+
+__global__ void PlacePositions(const uint64_t* __restrict__ pos, int64_t n, const FirstWord* __restrict__ words,
+                               uint32_t* __restrict__ idx) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const FirstWord w = words[pos[i] >> 5];
+    idx[w.before + __popc(w.bits & ((1u << (pos[i] & 31)) - 1))] = static_cast<uint32_t>(i);
+  }
+}
+
 }  // namespace
 
-bool Context::RangeSortItems(void* items_v, int64_t n, Arena& arena, unsigned long long* ties, uint32_t tie_mask,
-                             const unsigned long long* key_range) {
+void Context::OrderPositions(const uint64_t* pos, int64_t n, int64_t bound, uint32_t* idx, Arena& arena) {
+  const int64_t nwords = OrderWordsFor(bound);
+  FirstWord* words = reinterpret_cast<FirstWord*>(arena.Alloc(sizeof(FirstWord) * nwords));
+  uint64_t* count = arena.AllocT<uint64_t>(1);
+  if (dry || n <= 0) return;
+  Memset(words, 0, sizeof(FirstWord) * nwords);
+  const int grid = GridFor(n, 256);
+  TimedStart("order rows");
+  Issue([=](cudaStream_t s) { MarkPositions<<<grid, 256, 0, s>>>(pos, n, words); });
+  TimedStop();
+  OrderFirstRows(words, bound, count, arena);
+  TimedStart("order rows");
+  Issue([=](cudaStream_t s) { PlacePositions<<<grid, 256, 0, s>>>(pos, n, words, idx); });
+  TimedStop();
+  KDB_CUDA(cudaGetLastError());
+}
+
+bool Context::RangeSortItems(void* items_v, int64_t n, Arena& arena, const ItemKeys& keys, unsigned long long* ties,
+                             uint32_t tie_mask) {
   if (n <= 1 || dry) return true;
   if (n > 0x7fffffffLL) return false;
+  int buckets = kMinRangeBuckets;
+  while (buckets < kMaxRangeBuckets && static_cast<int64_t>(buckets) * 4 < n) buckets <<= 1;
+  const unsigned parts = static_cast<unsigned>(buckets / kRangePart);
   SortItem* items = static_cast<SortItem*>(items_v);
   SortItem* tmp = reinterpret_cast<SortItem*>(arena.Alloc(sizeof(SortItem) * n));
-  uint16_t* bof = reinterpret_cast<uint16_t*>(arena.Alloc(sizeof(uint16_t) * n));
-  uint16_t* tbof = reinterpret_cast<uint16_t*>(arena.Alloc(sizeof(uint16_t) * n));
-  unsigned long long* mm = key_range ? nullptr : arena.AllocT<unsigned long long>(2);
-  const unsigned long long* range = key_range ? key_range : mm;
-  unsigned* counts = arena.AllocT<unsigned>(kRangeBuckets);
-  unsigned* offs = arena.AllocT<unsigned>(kRangeBuckets + 1);
-  unsigned* cursor = arena.AllocT<unsigned>(kRangeBuckets);
-  unsigned* largest = arena.AllocT<unsigned>(1);
+  // counts, then the largest bucket (cleared together)
+  unsigned* counts = arena.AllocT<unsigned>(buckets + 1);
+  unsigned* largest = counts + buckets;
+  unsigned* sums = arena.AllocT<unsigned>(parts);
+  unsigned* offs = arena.AllocT<unsigned>(buckets + 1);
+  unsigned* cursor = arena.AllocT<unsigned>(buckets);
+  const RangeArgs a{keys.range, buckets, keys.tie_bits, keys.key_bit_in_tie, ties == nullptr};
   // a fallback to the merge sort drops these passes from the recording
   const auto mark = RecordMark();
-  if (mm) {
-    Memset(mm, 0xff, sizeof(unsigned long long));
-    Memset(mm + 1, 0, sizeof(unsigned long long));
-  }
-  Memset(counts, 0, sizeof(unsigned) * kRangeBuckets);
-  const int mm_grid = static_cast<int>(std::min<int64_t>((n + kRangeThreads - 1) / kRangeThreads, 32));
+  Memset(counts, 0, sizeof(unsigned) * (buckets + 1));
   const int grid = GridFor(n, 256);
   TimedStart("sort range");
-  if (mm) Issue([=](cudaStream_t s) { RangeMinMax<<<mm_grid, kRangeThreads, 0, s>>>(items, n, mm); });
-  Issue([=](cudaStream_t s) { RangeCount<<<grid, 256, 0, s>>>(items, n, range, bof, counts); });
-  Issue([=](cudaStream_t s) { RangeOffsets<<<1, kRangeThreads, 0, s>>>(counts, offs, cursor, largest); });
+  Issue([=](cudaStream_t s) { RangeCount<<<grid, 256, 0, s>>>(items, n, a, counts); });
+  Issue([=](cudaStream_t s) { RangePartSums<<<parts, kRangeThreads, 0, s>>>(counts, sums, largest); });
+  Issue([=](cudaStream_t s) { RangeOffsets<<<parts, kRangeThreads, 0, s>>>(counts, sums, offs, cursor); });
   TimedStop();
   KDB_CUDA(cudaGetLastError());
   // the bucket sizes decide (at recording; a replay runs on the same data)
@@ -1218,8 +1255,8 @@ bool Context::RangeSortItems(void* items_v, int64_t n, Arena& arena, unsigned lo
     return false;
   }
   TimedStart("sort buckets");
-  Issue([=](cudaStream_t s) { RangeScatter<<<grid, 256, 0, s>>>(items, n, bof, cursor, tmp, tbof); });
-  Issue([=](cudaStream_t s) { RangeRank<<<grid, 256, 0, s>>>(tmp, tbof, n, offs, items, ties, tie_mask); });
+  Issue([=](cudaStream_t s) { RangeScatter<<<grid, 256, 0, s>>>(items, n, a, cursor, tmp); });
+  Issue([=](cudaStream_t s) { RangeRank<<<grid, 256, 0, s>>>(tmp, n, a, offs, items, ties, tie_mask); });
   TimedStop();
   KDB_CUDA(cudaGetLastError());
   return true;
