@@ -467,7 +467,7 @@ void EmitPartialReduce(KernelSource& ks, const std::string& part, const std::str
   ks.Open("for (int64_t b0 = lane; b0 < (int64_t)" + G + "; b0 += 256)");
   ks.L("uint64_t v[8];");
   ks.L("_Pragma(\"unroll\") for (int u = 0; u < 8; u++) { const int64_t b = b0 + 32 * u; v[u] = b < (int64_t)" + G +
-       " ? " + part + "[(int64_t)k * (int64_t)" + G + " + b] : 0ULL; }");
+       " ? __ldcg((const unsigned long long*)&" + part + "[(int64_t)k * (int64_t)" + G + " + b]) : 0ULL; }");
   ks.L("_Pragma(\"unroll\") for (int u = 0; u < 8; u++) if (b0 + 32 * u < (int64_t)" + G +
        ") x = kdb_word_combine(kind, x, v[u]);");
   ks.Close();
@@ -673,7 +673,10 @@ class Executor {
   Executor(Context& ctx, Arena& arena) : ctx_(ctx), arena_(arena) {}
 
   HostResult Run(const Operator& root);
-  MatBuffer MaterializeRoot(const Operator& root) { return Materialize(root); }
+  MatBuffer MaterializeRoot(const Operator& root) {
+    root_result_ = true;
+    return Materialize(root);
+  }
   // the root's rows from the device into a host result
   HostResult Download(const MatBuffer& m, const Operator& root, bool check_error = false);
   int64_t bytes_scanned = 0;
@@ -686,6 +689,8 @@ class Executor {
   // build-cache entries this query reads: kept until the executor (whose
   // query has synchronised by then) is destroyed
   std::vector<std::shared_ptr<BuildEntry>> held_;
+  // set while the operator materialised next makes the query's result
+  bool root_result_ = false;
   std::string ChildSig(const Operator& child, const std::set<int>& index_cols) const;
 
   // --- helpers -----------------------------------------------------------
@@ -758,6 +763,56 @@ class Executor {
     return m;
   }
 
+  // A buffer of a few rows for the query's result, in pinned host memory that
+  // the kernel writing it reaches directly: the download then waits for the
+  // query and has the rows, with no kernel or copy of its own.  The first
+  // word of its block takes the device error word (see EmitHostError).
+  // Without a free block, or with TEXT columns, an ordinary buffer.
+  MatBuffer AllocResult(const std::vector<SchemaCol>& schema, int64_t cap, bool all_nullable) {
+    size_t bytes = 16;
+    bool text = false;
+    for (const auto& c : schema) {
+      bytes += ((StoreWidth(c.expr->type.id) * cap + 15) & ~size_t(15)) + ((static_cast<size_t>(cap) + 15) & ~size_t(15));
+      text |= c.expr->type.id == TypeId::TEXT;
+    }
+    std::shared_ptr<char> block;
+    if (!ctx_.dry && !text && bytes <= Context::kResultSlotBytes && !ctx_.OptStr("KDB_NO_MAPPED_RESULT"))
+      block = ctx_.AcquireResultSlot();
+    MatBuffer m;
+    if (!block) {
+      m = AllocMat(schema, cap);
+    } else {
+      m.cap = cap;
+      m.host = block;
+      m.host_device = ctx_.ResultSlotDevice(block.get());
+      size_t off = 16;
+      for (const auto& c : schema) {
+        MatCol mc;
+        mc.type = c.expr->type;
+        mc.data = m.host_device + off;
+        off += (StoreWidth(mc.type.id) * cap + 15) & ~size_t(15);
+        mc.nullable = c.expr->nullable || all_nullable;
+        if (mc.nullable) {
+          mc.nulls = reinterpret_cast<int8_t*>(m.host_device + off);
+          off += (static_cast<size_t>(cap) + 15) & ~size_t(15);
+        }
+        m.cols.push_back(mc);
+      }
+      m.pos = arena_.AllocT<uint64_t>(cap);
+    }
+    if (all_nullable)
+      for (auto& mc : m.cols)
+        if (!mc.nulls) {
+          mc.nullable = true;
+          mc.nulls = arena_.AllocT<int8_t>(cap);
+        }
+    return m;
+  }
+  // the thread that ends a result's kernel hands the error word over too
+  void EmitHostError(KernelSource& ks, const MatBuffer& m) {
+    if (m.host) ks.L("*" + ks.Ptr(m.host_device, "int") + " = *" + ks.Ptr(ctx_.d_err, "int") + ";");
+  }
+
   // Prepare everything a stream over `op` needs: materialise non-streamable
   // inputs, build hash-join tables and Skinner indexes.
   void Prepare(const Operator& op) {
@@ -815,12 +870,15 @@ class Executor {
     if (op.kind == OpKind::HASH_JOIN || op.kind == OpKind::CROSS_PRODUCT) return true;
     return op.kind == OpKind::SELECT && Streamable(op.child()) && StreamHasJoin(op.child());
   }
-  MatBuffer RunAggregate(const Operator& op);
+  MatBuffer RunAggregate(const Operator& op, bool root = false);
   // any_order: the consumer (an ORDER BY) orders the rows itself, so the
   // groups may come out in any order with their first-appearance key as the
   // stream position (pos_is_index false) instead of being sorted by it
-  MatBuffer RunGroupBy(const Operator& op, bool any_order = false, const Operator* order_by = nullptr);
-  MatBuffer RunOrderBy(const Operator& op);
+  // root: the groups are the query's result (under an order_by: if they come
+  // out in its order)
+  MatBuffer RunGroupBy(const Operator& op, bool any_order = false, const Operator* order_by = nullptr,
+                       bool root = false);
+  MatBuffer RunOrderBy(const Operator& op, bool root = false);
   MatBuffer RunSkinner(const Operator& op, const SkinnerAgg* agg = nullptr);
   MatBuffer SkinnerRows(const Operator& child);
   MatBuffer SmallOrderBy(const Operator& op, MatBuffer& m);
@@ -832,7 +890,7 @@ class Executor {
   // high words hold the rows (read by EmitMatScan instead of an index array)
   const uint64_t* order_items_ = nullptr;
   MatBuffer RunGroupByDense(const Operator& op, const std::vector<AggPlan>& plans, const KeyLayout& kl,
-                            const Operator* order_by = nullptr);
+                            const Operator* order_by = nullptr, bool root = false);
   // the ORDER BY was done by its GROUP BY child (dense path)
   bool group_sorted_ = false;
   bool BuildRowGroups(const Operator& op, std::vector<int>* key_cols);
@@ -2027,11 +2085,13 @@ MatBuffer Executor::MaterializeCounted(const Operator& op, const std::function<v
 }
 
 MatBuffer Executor::Materialize(const Operator& op) {
+  if (op.kind == OpKind::OUTPUT) return Materialize(op.child());
+  const bool root = root_result_;
+  root_result_ = false;
   switch (op.kind) {
-    case OpKind::OUTPUT: return Materialize(op.child());
-    case OpKind::AGGREGATE: return RunAggregate(op);
-    case OpKind::GROUP_BY_AGGREGATE: return RunGroupBy(op);
-    case OpKind::ORDER_BY: return RunOrderBy(op);
+    case OpKind::AGGREGATE: return RunAggregate(op, root);
+    case OpKind::GROUP_BY_AGGREGATE: return RunGroupBy(op, false, nullptr, root);
+    case OpKind::ORDER_BY: return RunOrderBy(op, root);
     case OpKind::SKINNER_JOIN: return RunSkinner(op);
     default: return MaterializeStream(op);
   }
@@ -2099,11 +2159,10 @@ CVal GroupResult(ExprGen& eg, const AggPlan& p, const std::string& sv, const std
 // combines the partials in block order and evaluates the output schema.
 // ---------------------------------------------------------------------------
 
-MatBuffer Executor::RunAggregate(const Operator& op) {
+MatBuffer Executor::RunAggregate(const Operator& op, bool root) {
   int flags = 0;
   std::vector<AggPlan> plans;
   for (const auto& a : op.aggs) plans.push_back(PlanAgg(*a, flags));
-  const int nw = static_cast<int>(plans.size()) * 2 + 2;  // per agg: value, count; + rows, first
   const int block = 256;
   // An aggregate of exact, order-free states (COUNT, MIN/MAX of keys,
   // integer SUM) over non-NULL inputs directly above a Skinner join is
@@ -2121,41 +2180,59 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
   if (any_text) ctx_.Memset(text_state, 0, sizeof(uint64_t) * (plans.size() + 1));
   // Finalize.  Every output column gets a NULL array: an empty input emits a
   // single all-NULL row even for COUNT (aggregate_translator.cc:82-89).
-  MatBuffer out = AllocMat(op.output, 1);
+  MatBuffer out = root ? AllocResult(op.output, 1, true) : AllocMat(op.output, 1);
   for (auto& mc : out.cols)
     if (!mc.nulls) {
       mc.nullable = true;
       mc.nulls = arena_.AllocT<int8_t>(1);
     }
-  bool fused_finalize = false;
-  // (the finalize is emitted into the aggregate kernel's last CTA, or into
-  // a one-block kernel after a fused Skinner join)
+  // Words of a partial: each aggregate's value and its count of non-NULL
+  // inputs (-1: the input is never NULL, so the count is the rows), the rows,
+  // and the first position (only where COUNT asks for the first row's flag).
+  // A fused Skinner join keeps them all (SkinnerAgg).
+  std::vector<int> vw(plans.size(), -1), cw(plans.size(), -1);
+  int nw = 0, rows_w = -1, first_w = -1;
+  std::vector<char> counted(plans.size(), 1);
+  auto lay_out = [&](bool all) {
+    nw = 0;
+    for (size_t j = 0; j < plans.size(); j++) {
+      const StateKind k = plans[j].kind;
+      if (all || (k != StateKind::Count && k != StateKind::MinMaxText)) vw[j] = nw++;
+      if (all || counted[j]) cw[j] = nw++;
+    }
+    rows_w = nw++;
+    if (all || flags > 0) first_w = nw++;
+  };
+  // One block combines the partials.  (As the aggregate kernel's last CTA it
+  // saves a launch, but its serial tail runs after all others instead of
+  // starting under them: 1 us slower per query from 10k to 8M rows.)
   auto emit_finalize = [&](KernelSource& fk, ExprGen& fg, const std::string& fp, const std::string& G) {
   std::string ftp = fk.Ptr(text_state, "uint64_t", true);
   {
     std::vector<WordKind> kinds(nw, WordKind::AddI64);
     for (size_t j = 0; j < plans.size(); j++) {
       const AggPlan& p = plans[j];
-      if (p.kind == StateKind::SumF64 || p.kind == StateKind::AvgF64) kinds[j * 2] = WordKind::AddF64;
-      if (p.kind == StateKind::MinMaxKey) kinds[j * 2] = p.is_min ? WordKind::MinU64 : WordKind::MaxU64;
+      if (p.kind == StateKind::SumF64 || p.kind == StateKind::AvgF64) kinds[vw[j]] = WordKind::AddF64;
+      if (p.kind == StateKind::MinMaxKey) kinds[vw[j]] = p.is_min ? WordKind::MinU64 : WordKind::MaxU64;
     }
-    kinds[nw - 1] = WordKind::MinU64;
+    if (first_w >= 0) kinds[first_w] = WordKind::MinU64;
     EmitPartialReduce(fk, fp, G, nw, kinds);
   }
   fk.Open("if (threadIdx.x == 0)");
+  fk.L("const int64_t trows = (int64_t)tot[" + std::to_string(rows_w) + "];");
   for (size_t j = 0; j < plans.size(); j++) {
     const AggPlan& p = plans[j];
-    std::string J = std::to_string(j), W = std::to_string(j * 2), C = std::to_string(j * 2 + 1);
+    const std::string J = std::to_string(j), W = "tot[" + std::to_string(vw[j]) + "]";
     switch (p.kind) {
       case StateKind::SumF64:
-      case StateKind::AvgF64: fk.L("double s" + J + " = __longlong_as_double((long long)tot[" + W + "]);"); break;
-      case StateKind::MinMaxKey: fk.L("uint64_t s" + J + " = tot[" + W + "];"); break;
-      default: fk.L("int64_t s" + J + " = (int64_t)tot[" + W + "];"); break;
+      case StateKind::AvgF64: fk.L("double t" + J + " = __longlong_as_double((long long)" + W + ");"); break;
+      case StateKind::MinMaxKey: fk.L("uint64_t t" + J + " = " + W + ";"); break;
+      case StateKind::SumI64: fk.L("int64_t t" + J + " = (int64_t)" + W + ";"); break;
+      default: break;
     }
-    fk.L("int64_t c" + J + " = (int64_t)tot[" + C + "];");
+    fk.L("int64_t tc" + J + " = " + (cw[j] >= 0 ? "(int64_t)tot[" + std::to_string(cw[j]) + "]" : std::string("trows")) + ";");
   }
-  fk.L("int64_t rows = (int64_t)tot[" + std::to_string(nw - 2) + "];");
-  fk.L("uint64_t first = tot[" + std::to_string(nw - 1) + "];");
+  if (first_w >= 0) fk.L("uint64_t tfirst = tot[" + std::to_string(first_w) + "];");
   std::vector<CVal> virt;
   for (size_t j = 0; j < plans.size(); j++) {
     const AggPlan& p = plans[j];
@@ -2163,20 +2240,20 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
     const Type& rt = p.agg->type;
     const Type& ct = p.agg->kid(0).type;
     switch (p.kind) {
-      case StateKind::SumF64: virt.push_back(fg.Bind(rt, "s" + J, "c" + J + " == 0")); break;
-      case StateKind::SumI64: virt.push_back(fg.Bind(rt, "(" + CType(rt.id) + ")s" + J, "c" + J + " == 0")); break;
+      case StateKind::SumF64: virt.push_back(fg.Bind(rt, "t" + J, "tc" + J + " == 0")); break;
+      case StateKind::SumI64: virt.push_back(fg.Bind(rt, "(" + CType(rt.id) + ")t" + J, "tc" + J + " == 0")); break;
       case StateKind::AvgF64:
-        virt.push_back(fg.Bind(rt, "__ddiv_rn(s" + J + ", (double)c" + J + ")", "c" + J + " == 0"));
+        virt.push_back(fg.Bind(rt, "__ddiv_rn(t" + J + ", (double)tc" + J + ")", "tc" + J + " == 0"));
         break;
       case StateKind::Count: {
-        std::string v = "c" + J;
-        if (p.count_flag >= 0) v = "(c" + J + " + (int64_t)((first >> " + std::to_string(p.count_flag) + ") & 1ULL))";
+        std::string v = "tc" + J;
+        if (p.count_flag >= 0) v = "(tc" + J + " + (int64_t)((tfirst >> " + std::to_string(p.count_flag) + ") & 1ULL))";
         virt.push_back(fg.Bind(rt, v, "false"));
         break;
       }
-      case StateKind::MinMaxKey: virt.push_back(fg.Bind(rt, OKeyInv(ct, "s" + J), "c" + J + " == 0")); break;
+      case StateKind::MinMaxKey: virt.push_back(fg.Bind(rt, OKeyInv(ct, "t" + J), "tc" + J + " == 0")); break;
       case StateKind::MinMaxText:
-        virt.push_back(fg.Bind(rt, "kdb_str_from_handle(" + ftp + "[" + J + "])", "c" + J + " == 0"));
+        virt.push_back(fg.Bind(rt, "kdb_str_from_handle(" + ftp + "[" + J + "])", "tc" + J + " == 0"));
         break;
     }
   }
@@ -2190,13 +2267,15 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
     std::string val = mc.type.id == TypeId::BOOLEAN ? "(int8_t)(" + vals[c].v + " ? 1 : 0)" : vals[c].v;
     fk.L(dp + "[0] = " + val + ";");
     std::string np = fk.Ptr(mc.nulls, "int8_t");
-    fk.L(np + "[0] = (rows == 0 || (" + vals[c].n + ")) ? 1 : 0;");
+    fk.L(np + "[0] = (trows == 0 || (" + vals[c].n + ")) ? 1 : 0;");
   }
   std::string posp = fk.Ptr(out.pos, "uint64_t");
   fk.L(posp + "[0] = 0;");
+  EmitHostError(fk, out);
   fk.Close();
   };
   if (fuse) {
+    lay_out(true);
     part = arena_.AllocT<uint64_t>(nw);
     std::vector<uint64_t> init(nw, 0);
     for (size_t j = 0; j < plans.size(); j++)
@@ -2237,6 +2316,7 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
       CVal c = eg.Emit(p.agg->kid(0), s);
       std::string J = std::to_string(j);
       if (p.count_flag >= 0) fl += " | ((" + c.n + ") ? " + std::to_string(1 << p.count_flag) + "ULL : 0ULL)";
+      counted[j] = c.n != "false";
       ks.Open("if (!(" + c.n + "))");
       switch (p.kind) {
         case StateKind::SumF64: ks.L("s" + J + " = __dadd_rn(s" + J + ", " + c.v + ");"); break;
@@ -2253,11 +2333,12 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
           break;
         case StateKind::Count: break;
       }
-      ks.L("c" + J + "++;");
+      if (counted[j]) ks.L("c" + J + "++;");
       ks.Close();
     }
     ks.L("rows++;");
-    ks.L("{ uint64_t f = ((uint64_t)(" + pos + ") << 8) | (" + fl + "); first = f < first ? f : first; }");
+    if (flags > 0)
+      ks.L("{ uint64_t f = ((uint64_t)(" + pos + ") << 8) | (" + fl + "); first = f < first ? f : first; }");
   };
   if (Streamable(op.child())) EmitStream(ks, eg, op.child(), consume, src_rows);
   else EmitMatScan(ks, mats_.at(&op.child()), nullptr, consume, src_rows);
@@ -2265,82 +2346,64 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
   // Enough rows per thread that every thread runs a few prefetched
   // iterations (at 1M rows one row group per thread left most of the
   // kernel's time to ramp-up and the block reductions), at least one CTA
-  // per SM.
+  // per SM as long as every thread has a row group of its own.
   {
+    const int64_t rows = std::max<int64_t>(src_rows, 1);
     const int64_t rpt = ctx_.OptStr("KDB_AGG_ROWS_PER_THREAD") ? std::atoll(ctx_.OptStr("KDB_AGG_ROWS_PER_THREAD"))
                                                                : 16;
-    const int64_t want = (std::max<int64_t>(src_rows, 1) + block * rpt - 1) / (block * rpt);
-    grid = static_cast<int>(std::max<int64_t>(std::min<int64_t>(ctx_.GridFor(std::max<int64_t>(src_rows, 1), block),
-                                                                want),
-                                              std::min<int64_t>(ctx_.num_sms, ctx_.GridFor(std::max<int64_t>(src_rows, 1), block))));
+    const int64_t want = (rows + block * rpt - 1) / (block * rpt);
+    const int64_t groups = (rows + 4 * block - 1) / (4 * block);
+    grid = static_cast<int>(std::max<int64_t>(std::min<int64_t>(ctx_.GridFor(rows, block), want),
+                                              std::min<int64_t>(ctx_.num_sms, groups)));
   }
+  lay_out(false);
   part = arena_.AllocT<uint64_t>(static_cast<size_t>(grid) * nw);
   std::string pp = ks.Ptr(part, "uint64_t");
-  ks.L("__shared__ uint64_t red_u[32];");
-  ks.L("__shared__ double red_d[32];");
-  ks.L("__shared__ int64_t red_i[32];");
-  auto store = [&](int w, const std::string& val) {
-    ks.L("if (threadIdx.x == 0) " + pp + "[(int64_t)" + std::to_string(w) + " * gridDim.x + blockIdx.x] = " + val +
-         ";");
-  };
-  for (size_t j = 0; j < plans.size(); j++) {
-    const AggPlan& p = plans[j];
-    std::string J = std::to_string(j);
-    switch (p.kind) {
-      case StateKind::SumF64:
-      case StateKind::AvgF64:
-        ks.Open("");
-        ks.L("double t = kdb_block_reduce(s" + J + ", KdbAddF64(), red_d);");
-        store(static_cast<int>(j) * 2, "(uint64_t)__double_as_longlong(t)");
-        ks.Close();
-        break;
-      case StateKind::SumI64:
-        ks.Open("");
-        ks.L("int64_t t = kdb_block_reduce(s" + J + ", KdbAddI64(), red_i);");
-        store(static_cast<int>(j) * 2, "(uint64_t)t");
-        ks.Close();
-        break;
-      case StateKind::MinMaxKey:
-        ks.Open("");
-        ks.L("uint64_t t = kdb_block_reduce(s" + J + (p.is_min ? ", KdbMinU64(), red_u);" : ", KdbMaxU64(), red_u);"));
-        store(static_cast<int>(j) * 2, "t");
-        ks.Close();
-        break;
-      default:
-        store(static_cast<int>(j) * 2, "0ULL");
-        break;
+  // all words at once: a shuffle tree per warp, one barrier, then one thread
+  // per word folds the warps in order (with the words nobody reads left out,
+  // 64M rows of the Q6 shape take 188 instead of 206 us)
+  {
+    const std::string NWS = std::to_string(nw);
+    ks.L("__shared__ uint64_t kdb_red[" + NWS + "][" + std::to_string(block / 32) + "];");
+    ks.L("const int kdb_lane = threadIdx.x & 31, kdb_warp = threadIdx.x >> 5;");
+    std::vector<WordKind> kinds(nw, WordKind::AddI64);
+    auto word = [&](int w, const std::string& var, const std::string& ctype, WordKind k) {
+      const bool f = ctype == "double";
+      const std::string a = f ? "(uint64_t)__double_as_longlong(" + var + ")" : "(uint64_t)" + var;
+      ks.Open("");
+      ks.L("uint64_t x = " + a + ";");
+      ks.L("_Pragma(\"unroll\") for (int o = 16; o > 0; o >>= 1) { const uint64_t y = __shfl_xor_sync(0xffffffffu, x, o); x = " +
+           CombineBits(k, "x", "y") + "; }");
+      ks.L("if (kdb_lane == 0) kdb_red[" + std::to_string(w) + "][kdb_warp] = x;");
+      ks.Close();
+      kinds[w] = k;
+    };
+    for (size_t j = 0; j < plans.size(); j++) {
+      const AggPlan& p = plans[j];
+      const std::string J = std::to_string(j);
+      switch (p.kind) {
+        case StateKind::SumF64:
+        case StateKind::AvgF64: word(vw[j], "s" + J, "double", WordKind::AddF64); break;
+        case StateKind::SumI64: word(vw[j], "s" + J, "int64_t", WordKind::AddI64); break;
+        case StateKind::MinMaxKey:
+          word(vw[j], "s" + J, "uint64_t", p.is_min ? WordKind::MinU64 : WordKind::MaxU64);
+          break;
+        default: break;
+      }
+      if (cw[j] >= 0) word(cw[j], "c" + J, "int64_t", WordKind::AddI64);
     }
-    ks.Open("");
-    ks.L("int64_t t = kdb_block_reduce(c" + J + ", KdbAddI64(), red_i);");
-    store(static_cast<int>(j) * 2 + 1, "(uint64_t)t");
-    ks.Close();
-  }
-  ks.Open("");
-  ks.L("int64_t t = kdb_block_reduce(rows, KdbAddI64(), red_i);");
-  store(nw - 2, "(uint64_t)t");
-  ks.Close();
-  ks.Open("");
-  ks.L("uint64_t t = kdb_block_reduce(first, KdbMinU64(), red_u);");
-  store(nw - 1, "t");
-  ks.Close();
-  // The last CTA can combine the partials itself (KDB_AGG_FUSED_FINALIZE),
-  // but measured at 1M rows that kernel's serial tail costs more than the
-  // second one-block launch (13.1 us vs 10.6 + 6.6 us; step 50.2 vs 49.1 us)
-  fused_finalize = ctx_.OptStr("KDB_AGG_FUSED_FINALIZE") != nullptr;
-  if (fused_finalize) {
-    // the last CTA to finish combines the partials (same fixed-order
-    // reduction as the separate finalize) and writes the result row
-    uint32_t* done = arena_.AllocT<uint32_t>(1);
-    ctx_.Memset(done, 0, sizeof(uint32_t));
-    const std::string dn = ks.Ptr(done, "unsigned");
-    ks.L("__shared__ bool kdb_last_block;");
-    ks.L("__threadfence();");
+    word(rows_w, "rows", "int64_t", WordKind::AddI64);
+    if (first_w >= 0) word(first_w, "first", "uint64_t", WordKind::MinU64);
     ks.L("__syncthreads();");
-    ks.L("if (threadIdx.x == 0) kdb_last_block = atomicAdd(" + dn + ", 1u) == gridDim.x - 1;");
-    ks.L("__syncthreads();");
-    ks.Open("if (kdb_last_block)");
-    ks.L("__threadfence();");
-    emit_finalize(ks, eg, pp, "gridDim.x");
+    const std::string kt = "kdb_block_kinds" + std::to_string(ks.lits++);
+    ks.globals << "__device__ const unsigned char " << kt << "[" << nw << "] = {";
+    for (int w = 0; w < nw; w++) ks.globals << static_cast<int>(kinds[w]) << ",";
+    ks.globals << "};\n";
+    ks.Open("for (int k = threadIdx.x; k < " + NWS + "; k += blockDim.x)");
+    ks.L("uint64_t x = kdb_red[k][0];");
+    ks.L("for (int w = 1; w < " + std::to_string(block / 32) + "; w++) x = kdb_word_combine(" + kt +
+         "[k], x, kdb_red[k][w]);");
+    ks.L(pp + "[(int64_t)k * gridDim.x + blockIdx.x] = x;");
     ks.Close();
   }
   {
@@ -2353,7 +2416,7 @@ MatBuffer Executor::RunAggregate(const Operator& op) {
   }
   }  // not fused
 
-  if (!fused_finalize) {
+  {
     KernelSource fk;
     ExprGen fg(ctx_, fk);
     const std::string fp = fk.Ptr(part, "uint64_t", true);
@@ -2459,7 +2522,7 @@ std::string Executor::ChildSig(const Operator& child, const std::set<int>& index
 // (compile/proxy/aggregate_hash_table.cc:187-243) turns into on a GPU when the
 // group count is tiny.
 MatBuffer Executor::RunGroupByDense(const Operator& op, const std::vector<AggPlan>& plans,
-                                    const KeyLayout& kl, const Operator* order_by) {
+                                    const KeyLayout& kl, const Operator* order_by, bool root) {
   const int64_t D = static_cast<int64_t>(kl.domain);
   // words per group: per-agg value / count words (shared when identical),
   // then rows and first position
@@ -2722,7 +2785,6 @@ MatBuffer Executor::RunGroupByDense(const Operator& op, const std::vector<AggPla
 
   // finalize: one block combines the per-CTA partials (warp per word, fixed
   // order), orders present groups by first position, evaluates the output
-  MatBuffer out = AllocMat(op.output, D);
   uint64_t* ngroups = arena_.AllocT<uint64_t>(1);
   KernelSource fk;
   ExprGen fg(ctx_, fk);
@@ -2760,6 +2822,7 @@ MatBuffer Executor::RunGroupByDense(const Operator& op, const std::vector<AggPla
     }
   }
   const bool fuse_order_pre = !sort_key.empty();
+  MatBuffer out = root && (!order_by || fuse_order_pre) ? AllocResult(op.output, D, false) : AllocMat(op.output, D);
   // the sort keys' enum string ranks, staged in shared memory by all
   // threads (thread 0's comparisons below then wait on no global load)
   std::vector<std::string> rank_smem(op.group_by.size());
@@ -2825,6 +2888,7 @@ MatBuffer Executor::RunGroupByDense(const Operator& op, const std::vector<AggPla
     fk.Close();
   }
   fk.L("kdb_ng = ng;");
+  EmitHostError(fk, out);
   fk.Close();
   fk.L("__syncthreads();");
   std::vector<std::string> optr, onull;
@@ -2885,8 +2949,7 @@ MatBuffer Executor::RunGroupByDense(const Operator& op, const std::vector<AggPla
     CUfunction f = ctx_.Kernel(src, "kdb_group_by_finalize");
     ctx_.Launch(f, 1, 1024, fk.Args(), 0, "group by finalize");
   }
-  out.rows = ReadU64(ngroups);
-  ctx_.CheckDeviceError("group by");
+  out.rows = ReadU64Checked(ngroups, "group by");
   out.pos_is_index = true;
   group_sorted_ = fuse_order;
   return out;
@@ -3207,7 +3270,7 @@ MatBuffer Executor::RunGroupByBuildRows(const Operator& op, const std::vector<Ag
   return out;
 }
 
-MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operator* order_by) {
+MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operator* order_by, bool root) {
   PrepareInput(op.child());
   int flags = 0;
   std::vector<AggPlan> plans;
@@ -3230,7 +3293,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
     }
     int64_t words = static_cast<int64_t>(distinct.size()) + 2;
     if (dense && static_cast<int64_t>(kl.domain) * words <= 64 && !ctx_.OptStr("KDB_NO_DENSE_GROUPBY"))
-      return RunGroupByDense(op, plans, kl, order_by);
+      return RunGroupByDense(op, plans, kl, order_by, root);
   }
 
   {
@@ -3709,23 +3772,24 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
 // NULL sorts last ascending, LessThan in evaluate.cc:339-402).
 // ---------------------------------------------------------------------------
 
-MatBuffer Executor::RunOrderBy(const Operator& op) {
+MatBuffer Executor::RunOrderBy(const Operator& op, bool root) {
   // every ORDER BY path below orders rows that are not in stream order by
   // their stream position, so a GROUP BY child need not sort its groups
   group_sorted_ = false;
+  bool identity = op.output.size() == op.child().output.size();
+  for (size_t c = 0; identity && c < op.output.size(); c++) {
+    const Expr& e = *op.output[c].expr;
+    identity = e.kind == ExprKind::ColRef && e.child_idx == 0 && e.column_idx == static_cast<int>(c);
+  }
+  const Operator* fused = ctx_.OptStr("KDB_NO_GROUP_ORDER_FUSE") ? nullptr : &op;
   MatBuffer m = op.child().kind == OpKind::GROUP_BY_AGGREGATE && !ctx_.OptStr("KDB_GROUP_ORDER_SORT")
-                    ? RunGroupBy(op.child(), true, ctx_.OptStr("KDB_NO_GROUP_ORDER_FUSE") ? nullptr : &op)
+                    ? RunGroupBy(op.child(), true, fused, root && identity && fused)
                     : Materialize(op.child());
   if (group_sorted_) {
     // the dense GROUP BY wrote its groups in this ORDER BY's order; an
     // output schema that passes every column through in place needs no
     // further work
     group_sorted_ = false;
-    bool identity = op.output.size() == m.cols.size();
-    for (size_t c = 0; identity && c < op.output.size(); c++) {
-      const Expr& e = *op.output[c].expr;
-      identity = e.kind == ExprKind::ColRef && e.child_idx == 0 && e.column_idx == static_cast<int>(c);
-    }
     if (identity) return m;
     uint32_t* idx = arena_.AllocT<uint32_t>(std::max<int64_t>(m.rows, 1));
     if (m.rows > 0) {
@@ -5513,6 +5577,32 @@ HostResult Executor::Download(const MatBuffer& m, const Operator& root, bool che
   const auto& schema = SchemaOf(root);
   HostResult res;
   res.rows = m.rows;
+  if (m.host) {
+    // the query's last kernel wrote the rows (and the error word) here
+    KDB_CUDA(cudaStreamSynchronize(ctx_.stream));
+    int err = 0;
+    std::memcpy(&err, m.host.get(), sizeof(err));
+    if (check_error && err) {
+      KDB_CUDA(cudaMemsetAsync(ctx_.d_err, 0, sizeof(int) * 4, ctx_.stream));
+      throw Error(-4, "replayed query raised a device error");
+    }
+    res.block = std::shared_ptr<char>(new char[Context::kResultSlotBytes], std::default_delete<char[]>());
+    std::memcpy(res.block.get(), m.host.get(), Context::kResultSlotBytes);
+    for (size_t c = 0; c < m.cols.size(); c++) {
+      const MatCol& mc = m.cols[c];
+      HostColumn hc;
+      hc.name = schema[c].name;
+      hc.type = mc.type;
+      hc.packed = true;
+      hc.data = res.block.get() + (static_cast<const char*>(mc.data) - m.host_device);
+      hc.nulls = mc.nulls ? reinterpret_cast<const int8_t*>(res.block.get()) +
+                                (reinterpret_cast<const char*>(mc.nulls) - m.host_device)
+                          : nullptr;
+      hc.width = static_cast<int>(StoreWidth(mc.type.id));
+      res.cols.push_back(std::move(hc));
+    }
+    return res;
+  }
   // one batch of device->host copies into the context's pinned staging
   // buffer and a single synchronisation (not one per column); with
   // `check_error` the device error word travels in the same batch

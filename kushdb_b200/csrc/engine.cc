@@ -214,6 +214,44 @@ std::shared_ptr<char> Context::AcquireHostBlock(size_t bytes) {
   return host_blocks_->Acquire(bytes);
 }
 
+struct Context::ResultSlots {
+  std::mutex mu;
+  char* host = nullptr;
+  char* device = nullptr;
+  std::vector<char*> free;
+  ~ResultSlots() {
+    if (host) cudaFreeHost(host);
+  }
+};
+
+std::shared_ptr<char> Context::AcquireResultSlot() {
+  if (dry) return nullptr;
+  if (!result_slots_) {
+    auto slots = std::make_shared<ResultSlots>();
+    void *h = nullptr, *d = nullptr;
+    KDB_CUDA(cudaHostAlloc(&h, kResultSlotBytes * kResultSlots, cudaHostAllocMapped));
+    slots->host = static_cast<char*>(h);
+    KDB_CUDA(cudaHostGetDevicePointer(&d, h, 0));
+    slots->device = static_cast<char*>(d);
+    for (size_t i = kResultSlots; i-- > 0;) slots->free.push_back(slots->host + i * kResultSlotBytes);
+    result_slots_ = std::move(slots);
+  }
+  std::lock_guard<std::mutex> g(result_slots_->mu);
+  if (result_slots_->free.empty()) return nullptr;
+  char* p = result_slots_->free.back();
+  result_slots_->free.pop_back();
+  std::memset(p, 0, kResultSlotBytes);
+  // the slots live as long as anything that holds one
+  return std::shared_ptr<char>(p, [slots = result_slots_](char* q) {
+    std::lock_guard<std::mutex> g(slots->mu);
+    slots->free.push_back(q);
+  });
+}
+
+char* Context::ResultSlotDevice(const char* slot) const {
+  return result_slots_->device + (slot - result_slots_->host);
+}
+
 void Context::ReserveHostBlocks(int count, size_t bytes) {
   std::vector<std::shared_ptr<char>> held;
   for (int i = 0; i < count; i++) held.push_back(AcquireHostBlock(bytes));

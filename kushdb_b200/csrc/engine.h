@@ -87,6 +87,10 @@ struct MatBuffer {
   int64_t pos_bound = -1;     // positions are distinct numbers below this (-1: not known)
   int64_t rows = 0;
   int64_t cap = 0;
+  // a query's result in pinned host memory: its block, and where the device
+  // sees it (`cols` point into that)
+  std::shared_ptr<char> host;
+  char* host_device = nullptr;
 };
 
 // A compiled pipeline program (one CUDA module from NVRTC).
@@ -371,6 +375,12 @@ class Context {
   // result keeps it until it is freed, then it returns to the context's pool
   // (no host copy of the columns, no pinned allocation per query).
   std::shared_ptr<char> AcquireHostBlock(size_t bytes);
+  // Small pinned blocks that a query's last kernel writes its result into:
+  // slots of one mapped allocation (made on first use), back to it when the
+  // last owner lets go; null when all are taken.
+  static constexpr size_t kResultSlotBytes = 4096, kResultSlots = 256;
+  std::shared_ptr<char> AcquireResultSlot();
+  char* ResultSlotDevice(const char* slot) const;
   // Puts `count` blocks of `bytes` into the pool ahead of use (a pinned
   // allocation synchronises with the device).
   void ReserveHostBlocks(int count, size_t bytes);
@@ -427,6 +437,8 @@ class Context {
   std::shared_ptr<ProgramCache> cache_ = std::make_shared<ProgramCache>();
   cudaEvent_t query_ev_[2] = {nullptr, nullptr};
   bool owns_catalog_ = true;
+  struct ResultSlots;
+  std::shared_ptr<ResultSlots> result_slots_;
   uint64_t* scan_sums_ = nullptr;  // part sums of ScanParted (made on first use)
   void ThrowDeviceError(int err, const char* what);
   void ScanParted(uint64_t* a, int64_t n, const uint64_t* n_ptr);

@@ -69,6 +69,7 @@ class Server {
     for (int i = 0; i < slots; i++) {
       slots_.push_back(std::make_unique<Context>(parent));
       slots_.back()->ReserveHostBlocks(4, 16 << 20);  // pinned result blocks up front: no host-alloc syncs later
+      slots_.back()->AcquireResultSlot();             // (the blocks small results are written into, too)
       slots_.back()->build_cache = cache_;
     }
     for (int i = 0; i < slots; i++) workers_.emplace_back([this, i] { Loop(i); });
