@@ -5327,7 +5327,10 @@ class SkinnerEngine : public JoinEnv {
       ks.L("atomicAdd((unsigned long long*)a.w[" + std::to_string(w_count_) + "], kdb_sfa[" + R + "]);");
       ks.Close();
     }
-    std::string src = ks.Kernel("kdb_skinner_episode", 128);
+    // 8 CTAs per SM (the grid's): 64 registers instead of 110, and twice the
+    // warps; the walk waits on dependent loads (position-2 expansion of a
+    // star join 217 -> 160 us; 5 to 16 CTAs measured within 2% of this)
+    std::string src = ks.Kernel("kdb_skinner_episode", 128, 8);
     fn_ = ctx_.Kernel(src, "kdb_skinner_episode");
     args_ = ks.Args();
   }
