@@ -137,7 +137,7 @@ class KernelSource {
   }
 
   int Arg(uint64_t w) {
-    if (args.size() >= 384) throw Error(-5, "pipeline needs more than 384 kernel argument words");
+    if (args.size() >= 384 + lit_words) throw Error(-5, "pipeline needs more than 384 kernel argument words");
     args.push_back(w);
     return static_cast<int>(args.size()) - 1;
   }
@@ -152,19 +152,45 @@ class KernelSource {
   }
   std::string Lit(const std::string& s) {
     std::string name = "kdb_lit" + std::to_string(lits++);
-    globals << "__device__ const char " << name << "[" << (s.size() + 1) << "] = {";
+    // (padded: string predicates read whole aligned words)
+    globals << "__device__ const __align__(8) char " << name << "[" << ((s.size() + 1 + 7) & ~size_t(7)) << "] = {";
     for (unsigned char c : s) globals << static_cast<int>(c) << ",";
     globals << "0};\n";
     return "kdb_mkstr(" + name + ", " + std::to_string(s.size()) + ")";
   }
 
+  // A string as argument words (its length, then its bytes): the length and
+  // the 4-byte word accessor that the kdb_lit_* predicates take.  False when
+  // it does not fit the words that the argument block keeps for strings: they
+  // hold the patterns of a query, and a long list stays in the source.
+  struct ArgString {
+    std::string len, get;
+  };
+  size_t lit_words = 0;
+  bool ArgLit(const std::string& s, ArgString* out) {
+    const size_t words = std::max<size_t>((s.size() + 7) / 8, 1);
+    if (lit_words + words + 1 > kLiteralWords) return false;
+    lit_words += words + 1;
+    out->len = "(int32_t)" + Word(s.size());
+    const int first = static_cast<int>(args.size());
+    for (size_t i = 0; i < words; i++) {
+      uint64_t w = 0;
+      for (size_t b = 0; b < 8 && 8 * i + b < s.size(); b++)
+        w |= static_cast<uint64_t>(static_cast<unsigned char>(s[8 * i + b])) << (8 * b);
+      Arg(w);
+    }
+    const std::string f = std::to_string(first);
+    out->get = "[&](int i) -> uint32_t { return (uint32_t)(a.w[" + f + " + (i >> 1)] >> (32 * (i & 1))); }";
+    return true;
+  }
+
   std::string Kernel(const std::string& name, int block, int min_blocks = 1) const {
     int words = 16;
     while (words < static_cast<int>(args.size())) words *= 2;
-    if (words > 384) words = 384;
+    if (words > kArgWords) words = kArgWords;
     std::ostringstream o;
     o << globals.str() << "\nextern \"C\" __global__ void __launch_bounds__(" << block << ", " << min_blocks
-      << ") " << name << "(KArgsN<" << words << "> a) {\n"
+      << ") " << name << "(const __grid_constant__ KArgsN<" << words << "> a) {\n"
       << kGridDependencyWait << pre.str() << body.str() << "}\n";
     return o.str();
   }
@@ -322,6 +348,25 @@ class ExprGen {
       case ExprKind::Binary: break;
     }
     CVal l = Emit(e.kid(0), s);
+    if (const Expr& lit = e.kid(1); lit.kind == ExprKind::Literal && lit.type.id == TypeId::TEXT && !lit.lit_null &&
+                                    (l.type.id == TypeId::TEXT || l.type.id == TypeId::ENUM)) {
+      // a string tested against a literal: the literal is an argument
+      const bool eq = l.type.id == TypeId::TEXT && (e.bop == BinOp::EQ || e.bop == BinOp::NEQ);
+      KernelSource::ArgString a;
+      if ((eq || e.bop == BinOp::STARTS_WITH || e.bop == BinOp::ENDS_WITH || e.bop == BinOp::CONTAINS) &&
+          ks_.ArgLit(lit.sval, &a)) {
+        const std::string str = l.type.id == TypeId::ENUM ? EnumString(l.type, l.v) : l.v;
+        const std::string tail = a.len + ", " + a.get + ")";
+        switch (e.bop) {
+          case BinOp::EQ: return Bind(e.type, "kdb_lit_eq(" + str + ", " + tail, l.n);
+          case BinOp::NEQ: return Bind(e.type, "!kdb_lit_eq(" + str + ", " + tail, l.n);
+          case BinOp::STARTS_WITH: return Bind(e.type, "kdb_lit_starts(" + str + ", " + tail, l.n);
+          case BinOp::ENDS_WITH: return Bind(e.type, "kdb_lit_ends(" + str + ", " + tail, l.n);
+          default:
+            return Bind(e.type, "kdb_lit_contains(" + str + ", " + tail, l.n);
+        }
+      }
+    }
     CVal r = Emit(e.kid(1), s);
     if (e.bop == BinOp::AND) {
       // expression_translator.cc:74-91

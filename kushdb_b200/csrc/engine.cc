@@ -353,6 +353,10 @@ void Context::FreeColumn(DevColumn& c) {
   c = DevColumn();
 }
 
+// Bytes allocated for string storage: whole words, since string predicates
+// read the aligned words that a string's bytes lie in.
+static size_t TextBytes(size_t bytes) { return std::max<size_t>((bytes + 7) & ~size_t(7), 16); }
+
 static void CheckRows(DevTable& t, int64_t n, const std::string& name) {
   if (t.rows >= 0 && t.rows != n)
     throw Error(-1, "column " + name + " has " + std::to_string(n) + " rows, table has " +
@@ -489,7 +493,7 @@ void Context::AddTextColumn(const std::string& table, const std::string& column,
     c.max_text_len = std::max<int32_t>(c.max_text_len, static_cast<int32_t>(off[r + 1] - off[r]));
   c.toff = static_cast<int64_t*>(DevAlloc(sizeof(int64_t) * (n + 1)));
   H2D(c.toff, off.data(), sizeof(int64_t) * (n + 1));
-  c.tchars = static_cast<char*>(DevAlloc(std::max<int64_t>(nbytes, 16)));
+  c.tchars = static_cast<char*>(DevAlloc(TextBytes(nbytes)));
   H2D(c.tchars, chars + base, nbytes);
   c.bytes = sizeof(int64_t) * (n + 1) + nbytes;
   if (nulls) {
@@ -535,7 +539,7 @@ void Context::AddTextColumnFromKdb(const std::string& table, const std::string& 
   c.n = card;
   c.max_text_len = max_len;
   c.toff = static_cast<int64_t*>(DevAlloc(sizeof(int64_t) * (card + 1)));
-  c.tchars = static_cast<char*>(DevAlloc(std::max<uint64_t>(nbytes, 16)));
+  c.tchars = static_cast<char*>(DevAlloc(TextBytes(nbytes)));
   c.bytes = sizeof(int64_t) * (card + 1) + nbytes;
   if (!dry && card > 0) {
     void* d_raw = nullptr;
@@ -591,7 +595,7 @@ void Context::RegisterEnum(int32_t id, std::vector<std::string> values) {
   for (int32_t r = 0; r < n; r++) e.rank[order[r]] = r;
   e.d_off = static_cast<int64_t*>(DevAlloc(sizeof(int64_t) * (n + 1)));
   H2D(e.d_off, off.data(), sizeof(int64_t) * (n + 1));
-  e.d_chars = static_cast<char*>(DevAlloc(std::max<size_t>(chars.size(), 16)));
+  e.d_chars = static_cast<char*>(DevAlloc(TextBytes(chars.size())));
   H2D(e.d_chars, chars.data(), chars.size());
   e.d_rank = static_cast<int32_t*>(DevAlloc(sizeof(int32_t) * std::max(n, 1)));
   H2D(e.d_rank, e.rank.data(), sizeof(int32_t) * n);

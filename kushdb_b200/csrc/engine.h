@@ -116,9 +116,11 @@ constexpr const char* kGridDependencyWait =
     "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"
     "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
 
-// Host mirror of the device KArgs struct (passed by value).
+// A generated kernel's argument words (passed by value, as many as it uses):
+// some for strings that predicates compare with, beside 384 for all else.
+constexpr int kLiteralWords = 64, kArgWords = 384 + kLiteralWords;
 struct KArgs {
-  uint64_t w[384];
+  uint64_t w[kArgWords];
 };
 
 class Context;

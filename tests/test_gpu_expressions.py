@@ -187,3 +187,42 @@ def test_like_random_strings(setup, pattern):
     plan = OutputOperator(ScanSelectOperator(out, scan, rel, [Like(VirtColRef(scan, "s"), pattern)]))
     assert compare(e.execute(plan), o.execute(plan), ordered=False) == ""
     o.close()
+
+
+# substring search by words: every alignment of the string (its start in the
+# column moves with the rows before it), needles shorter and longer than a
+# word, at the start, the end and across word edges; literals are kernel
+# arguments, so one pipeline serves all needles of a form
+@pytest.mark.parametrize("needle", ["", "a", "ab", "abc", "abcd", "abcde", "bcdefghij", "\u00e9", "x" * 129, "y" * 505])
+@pytest.mark.parametrize("op", ["contains", "starts", "ends", "eq", "neq"])
+def test_string_literal_predicates_at_word_edges(needle, op):
+    import numpy as np
+    from kushdb_b200.data import HostColumn, HostTable, catalog_of
+    from kushdb_b200.engine import Engine
+    from kushdb_b200.plan import (ColRef, Contains, EndsWith, Eq, Literal, Neq, OperatorSchema, OutputOperator,
+                                  ScanOperator, SelectOperator, StartsWith, Type)
+    rng = np.random.default_rng(5)
+    strings = ["", needle, needle + "z", "z" + needle, "abcdefghijkl", "aab", "abab", "xabc", "xyabcd", "xyzabcde"]
+    for _ in range(600):
+        s = "".join("abcdefghijz\u00e9"[int(i)] for i in rng.integers(0, 12, int(rng.integers(0, 15))))
+        at = int(rng.integers(0, len(s) + 1))
+        strings.append(s[:at] + needle + s[at:] if rng.random() < 0.4 else s)
+    nulls = (rng.random(len(strings)) < 0.05).astype(np.int8)
+    t = HostTable("word_edges")
+    t.add(HostColumn.from_strings("s", strings, nulls))
+    t.add(HostColumn("id", Type.Int(), values=np.arange(len(strings), dtype=np.int32)))
+    rel = catalog_of([t])["word_edges"]
+    ss = OperatorSchema()
+    ss.AddGeneratedColumns(rel, ["s", "id"])
+    scan = ScanOperator(ss, rel)
+    f = {"contains": Contains, "starts": StartsWith, "ends": EndsWith, "eq": Eq, "neq": Neq}[op]
+    out = OperatorSchema()
+    out.AddPassthroughColumns(scan, ["id"])
+    plan = OutputOperator(SelectOperator(out, scan, f(ColRef(scan, "s"), Literal(needle))))
+    b = needle.encode()
+    want = {"contains": lambda x: b in x, "starts": lambda x: x.startswith(b), "ends": lambda x: x.endswith(b),
+            "eq": lambda x: x == b, "neq": lambda x: x != b}[op]
+    with Engine(0) as e:
+        e.register_table(t)
+        got = sorted(int(v) for v in e.execute(plan).columns[0].values)
+    assert got == [i for i, s in enumerate(strings) if not nulls[i] and want(s.encode())]
