@@ -45,20 +45,17 @@ namespace ops {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kPartBlock = 1024;                 // threads of a partitioned build / probe CTA
+constexpr int kBuildBlock = 512;                 // threads of a partitioned build CTA
+constexpr int kPartBlock = 1024;                 // threads of a partitioning CTA
 constexpr int kMaxPartBits = 13;                 // at most 8192 sub-tables
 constexpr size_t kSmemTableMax = 128 << 10;      // a sub-table built in shared memory
-constexpr size_t kTableBuf = 64 << 10;           // a probe-side sub-table buffer (two of them)
-constexpr int kProbeTile = 2048;                 // probe tuples per bulk-copied tile
+constexpr int kBuildTile = 2048;                 // staged tuples per bulk-copied tile
 constexpr uint32_t kWaitLimit = 1u << 24;        // bounded mbarrier waits
 constexpr int kErrWait = 1;                      // device error word: a wait gave up
 constexpr int kErrFull = 2;                      // a table ran out of empty slots
 constexpr int kDupKey = 4;                       // (not an error) two build rows share a key
 constexpr int kMatchTile = 4096;                 // probe rows per CTA when matches are compacted
-constexpr unsigned kOutStage = 4096;             // pairs a partitioned-probe CTA stages
-constexpr unsigned kFlatStage = 2048;            // pairs a flat-probe CTA stages
-constexpr int kTupCap = 3072;                    // probe tuples per partition buffer (warp-level probe)
-constexpr int kWarpStage = 64;                   // pairs a warp stages before one global append
+constexpr unsigned kOutStage = 2048;             // pairs a probe CTA stages
 
 // ---- keys --------------------------------------------------------------------
 struct KeyCol {
@@ -159,28 +156,6 @@ __device__ __forceinline__ void BulkLoad(void* dst, const void* src, uint32_t by
       "l"(src), "r"(bytes), "r"(SmemAddr(bar))
       : "memory");
 }
-// Several copies completing on one barrier phase: one thread announces their
-// total bytes (the phase's one arrival), then starts each copy.
-__device__ __forceinline__ void BarExpect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(SmemAddr(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void BulkCopy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          SmemAddr(dst)),
-      "l"(src), "r"(bytes), "r"(SmemAddr(bar))
-      : "memory");
-}
-// The same as several copies of at most `piece` bytes (a multiple of 16),
-// all in flight together.
-__device__ __forceinline__ void BulkCopyPieces(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
-                                               uint32_t piece) {
-  for (uint32_t o = 0; o < bytes; o += piece)
-    BulkCopy(static_cast<char*>(dst) + o, static_cast<const char*>(src) + o, bytes - o < piece ? bytes - o : piece,
-             bar);
-}
-
 // Waits for phase `parity` of `bar` to complete; false when the wait gave up.
 __device__ __forceinline__ bool BarWait(uint64_t* bar, uint32_t parity) {
   for (uint32_t it = 0; it < kWaitLimit; it++) {
@@ -242,9 +217,8 @@ __global__ void __launch_bounds__(kPartBlock) PartHistogram(KeyCol key, const in
 // One block: partition p's staged tuples start at stage_off[p] (each
 // partition padded to an even count, so every partition starts on a 16-byte
 // boundary), its sub-table at slot_off[p] with a power-of-two capacity of at
-// least count / load_factor and at least 16 slots (slot_off == nullptr: no
-// tables, probe side).  Totals go to stage_off[P] / slot_off[P]; the scatter
-// cursors are zeroed.
+// least count / load_factor and at least 16 slots.  Totals go to stage_off[P]
+// and slot_off[P]; the scatter cursors are zeroed.
 __global__ void PartOffsets(const unsigned* __restrict__ hist, int parts, double load_factor,
                             unsigned long long* __restrict__ stage_off, unsigned long long* __restrict__ slot_off,
                             unsigned* __restrict__ cursor) {
@@ -283,13 +257,13 @@ __global__ void PartOffsets(const unsigned* __restrict__ hist, int parts, double
     unsigned long long want = static_cast<unsigned long long>(ceil(static_cast<double>(c) / load_factor));
     unsigned long long cap = 16;
     while (cap < want + 1) cap <<= 1;
-    if (slot_off) slot_off[p] = sl;
+    slot_off[p] = sl;
     sl += cap;
     cursor[p] = 0;
   }
   if (threadIdx.x == 1023) {
     stage_off[parts] = s_stage[1023];
-    if (slot_off) slot_off[parts] = s_slot[1023];
+    slot_off[parts] = s_slot[1023];
   }
 }
 
@@ -345,38 +319,53 @@ __device__ __forceinline__ int Insert(typename Slot<WIDE>::T* tab, uint64_t cap,
   return kErrFull;
 }
 
+// What a warp's inserts reported, with one atomic at most per warp (one per
+// row on the same word: 338 against 101 us for 3.5M rows of which half share
+// a key).
+__device__ __forceinline__ void Report(int found, int* err) {
+  const int all = static_cast<int>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(found)));
+  if (all != 0 && (threadIdx.x & 31) == 0 && (*static_cast<volatile int*>(err) & all) != all) atomicOr(err, all);
+}
+
 // One table: every selected row with a non-NULL key.
 template <bool WIDE>
 __global__ void BuildFlat(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
                           typename Slot<WIDE>::T* __restrict__ tab, uint64_t cap, int* err) {
+  int found = 0;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t r = RowAt(sel, i);
     if (KeyNull(key, r)) continue;
     const int64_t k = LoadKey(key, r);
-    const int e = Insert<WIDE>(tab, cap, Hash32(static_cast<uint64_t>(k)), Slot<WIDE>::Make(k, r));
-    if (e) atomicOr(err, e);
+    found |= Insert<WIDE>(tab, cap, Hash32(static_cast<uint64_t>(k)), Slot<WIDE>::Make(k, r));
   }
+  Report(found, err);
 }
 
 // Persistent CTAs, partitions p = blockIdx.x + i * gridDim.x (empty ones are
-// only cleared).  A partition's staged tuples come
+// only cleared).  Shared memory is sized for the sub-tables that evenly spread
+// rows make, so that up to four CTAs of an SM overlap one another's waits (a
+// partition is clear, wait, insert and write out, one after the other): 6M
+// rows in 4096 sub-tables of 32 KB took 148 us with one CTA of 1024 threads
+// and 128 KB for the table per SM, and take 83 with three of 512 (87 with 256
+// threads, 144 with 1024).  A partition's staged tuples come
 // into shared memory in bulk-copied tiles through a two-buffer ring that
 // runs one tile ahead, across partition boundaries too; a sub-table that
 // fits shared memory is built there with shared-memory CAS and written out
 // with coalesced stores, a larger one is built in place in HBM.
 template <bool WIDE>
-__global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WIDE>::T* __restrict__ staged,
+__global__ void __launch_bounds__(kBuildBlock) BuildParts(const typename Slot<WIDE>::T* __restrict__ staged,
                                                      const unsigned long long* __restrict__ stage_off,
                                                      const unsigned* __restrict__ hist,
                                                      const unsigned long long* __restrict__ slot_off, int parts,
-                                                     typename Slot<WIDE>::T* __restrict__ slots, int* err) {
+                                                     typename Slot<WIDE>::T* __restrict__ slots, uint32_t tab_bytes,
+                                                     int* err) {
   using S = Slot<WIDE>;
   using T = typename S::T;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
-  T* tiles[2] = {reinterpret_cast<T*>(smem), reinterpret_cast<T*>(smem + kProbeTile * sizeof(T))};
-  T* stab = reinterpret_cast<T*>(smem + 2 * kProbeTile * sizeof(T));
+  T* tiles[2] = {reinterpret_cast<T*>(smem), reinterpret_cast<T*>(smem + kBuildTile * sizeof(T))};
+  T* stab = reinterpret_cast<T*>(smem + 2 * kBuildTile * sizeof(T));
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; b++) BarInit(&bar[b]);
     FenceProxyAsync();
@@ -389,8 +378,8 @@ __global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WID
     return q;
   };
   auto issue_tile = [&](int q, uint64_t t, int b) {
-    const uint64_t count = hist[q], t0 = t * kProbeTile;
-    const uint32_t n = static_cast<uint32_t>(umin64(kProbeTile, count - t0));
+    const uint64_t count = hist[q], t0 = t * kBuildTile;
+    const uint32_t n = static_cast<uint32_t>(umin64(kBuildTile, count - t0));
     FenceProxyAsync();
     BulkLoad(tiles[b], staged + stage_off[q] + t0, (n * sizeof(T) + 15) & ~15u, &bar[b]);
     issued[b]++;
@@ -401,7 +390,7 @@ __global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WID
   // the sub-tables that no shared-memory table is written over
   for (int q = blockIdx.x; q < parts; q += gridDim.x) {
     const uint64_t qcap = slot_off[q + 1] - slot_off[q];
-    if (hist[q] != 0 && qcap * sizeof(T) <= kSmemTableMax) continue;
+    if (hist[q] != 0 && qcap * sizeof(T) <= tab_bytes) continue;
     for (uint64_t i = threadIdx.x; i < qcap; i += blockDim.x) slots[slot_off[q] + i] = T{};
   }
   __syncthreads();
@@ -411,10 +400,10 @@ __global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WID
   while (p < parts && !failed) {
     const uint64_t cap = slot_off[p + 1] - slot_off[p];
     T* gtab = slots + slot_off[p];
-    const bool in_smem = cap * sizeof(T) <= kSmemTableMax;
+    const bool in_smem = cap * sizeof(T) <= tab_bytes;
     T* tab = in_smem ? stab : gtab;
     const uint64_t count = hist[p];
-    const uint64_t ntiles = (count + kProbeTile - 1) / kProbeTile;
+    const uint64_t ntiles = (count + kBuildTile - 1) / kBuildTile;
     const int np = next_part(p);
     if (in_smem) {
       // the previous partition's table was written out before the barrier
@@ -435,7 +424,7 @@ __global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WID
         break;
       }
       waited[b]++;
-      const uint32_t nt = static_cast<uint32_t>(umin64(kProbeTile, count - t * kProbeTile));
+      const uint32_t nt = static_cast<uint32_t>(umin64(kBuildTile, count - t * kBuildTile));
       for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
         const T v = tiles[b][i];
         const int64_t k = S::Key(v);
@@ -449,7 +438,7 @@ __global__ void __launch_bounds__(kPartBlock) BuildParts(const typename Slot<WID
     __syncthreads();
     p = np;
   }
-  if (found) atomicOr(err, found);
+  Report(found, err);
   if (failed && threadIdx.x == 0) {
     for (int b = 0; b < 2; b++)
       for (; waited[b] < issued[b]; waited[b]++) BarWait(&bar[b], waited[b] & 1);
@@ -514,11 +503,15 @@ __device__ __forceinline__ void FlushPairs(Stage& st, unsigned long long* out, u
 }
 
 template <bool WIDE, typename Stage>
-__device__ __forceinline__ void ProbeOne(const typename Slot<WIDE>::T* tab, uint64_t cap, int64_t k,
-                                         int64_t probe_row, Stage& st, unsigned long long* out,
+__device__ __forceinline__ void ProbeOne(const typename Slot<WIDE>::T* slots, const unsigned long long* slot_off,
+                                         int bits, int64_t k, int64_t probe_row, Stage& st, unsigned long long* out,
                                          unsigned long long out_cap, unsigned long long* counter) {
   using S = Slot<WIDE>;
-  uint64_t i = Hash32(static_cast<uint64_t>(k)) & (cap - 1);
+  const uint32_t h = Hash32(static_cast<uint64_t>(k)), p = PartOf(h, bits);
+  const unsigned long long first = slot_off[p];
+  const uint64_t cap = slot_off[p + 1] - first;
+  const typename S::T* tab = slots + first;
+  uint64_t i = h & (cap - 1);
   for (uint64_t step = 0; step < cap; step++) {
     const typename S::T s = tab[i];
     if (S::Empty(s)) return;
@@ -527,14 +520,21 @@ __device__ __forceinline__ void ProbeOne(const typename Slot<WIDE>::T* tab, uint
   }
 }
 
-// One table: every selected probe row looks its key up directly; the CTA
-// appends its staged pairs whenever the stage is half full.
+// Every selected probe row looks its key up in its sub-table; the CTA appends
+// its staged pairs whenever the stage is half full.  Bound by the random
+// reads of the table.  The probe side is not partitioned, however many
+// sub-tables there are: with 2048 threads an SM in flight, reading a slot
+// sector per row costs less than writing the rows out by partition and
+// copying every sub-table into shared memory.  4M x 3M rows: 46 us against
+// 47 + 76; 30M x 20M: 520 against 601 + 416; with every build key 8 times,
+// 48 against 22 + 419.
 template <bool WIDE>
-__global__ void __launch_bounds__(kBlock) ProbeFlat(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
-                                                    const typename Slot<WIDE>::T* __restrict__ tab, uint64_t cap,
+__global__ void __launch_bounds__(kBlock) ProbeRows(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
+                                                    const typename Slot<WIDE>::T* __restrict__ slots,
+                                                    const unsigned long long* __restrict__ slot_off, int bits,
                                                     unsigned long long* __restrict__ out,
                                                     unsigned long long out_cap, unsigned long long* counter) {
-  __shared__ OutStage<kFlatStage> st;
+  __shared__ OutStage<kOutStage> st;
   if (threadIdx.x == 0) st.count = 0;
   __syncthreads();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -542,10 +542,10 @@ __global__ void __launch_bounds__(kBlock) ProbeFlat(KeyCol key, const int32_t* _
     const int64_t i = b0 + threadIdx.x;
     if (i < n) {
       const int64_t r = RowAt(sel, i);
-      if (!KeyNull(key, r)) ProbeOne<WIDE>(tab, cap, LoadKey(key, r), r, st, out, out_cap, counter);
+      if (!KeyNull(key, r)) ProbeOne<WIDE>(slots, slot_off, bits, LoadKey(key, r), r, st, out, out_cap, counter);
     }
     // every thread's matches of this round are staged before thread 0 looks
-    if (__syncthreads_or(threadIdx.x == 0 && st.count >= kFlatStage / 2)) FlushPairs(st, out, out_cap, counter);
+    if (__syncthreads_or(threadIdx.x == 0 && st.count >= kOutStage / 2)) FlushPairs(st, out, out_cap, counter);
   }
   FlushPairs(st, out, out_cap, counter);
 }
@@ -555,15 +555,20 @@ __global__ void __launch_bounds__(kBlock) ProbeFlat(KeyCol key, const int32_t* _
 // its match is one word at the row's own place and the pairs in probe-row
 // order are those words compacted: no pair list and no sort of it (520 us of
 // radix passes for 2.4M pairs, against 29 us for the compaction).
-__global__ void __launch_bounds__(kBlock) MatchFlat(KeyCol key, int64_t n, const unsigned long long* __restrict__ tab,
-                                                    uint64_t cap, int32_t* __restrict__ match) {
+__global__ void __launch_bounds__(kBlock) MatchRows(KeyCol key, int64_t n, const unsigned long long* __restrict__ slots,
+                                                    const unsigned long long* __restrict__ slot_off, int bits,
+                                                    int32_t* __restrict__ match) {
   using S = Slot<false>;
   for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < n;
        r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     int32_t m = -1;
     if (!KeyNull(key, r)) {
       const int64_t k = LoadKey(key, r);
-      uint64_t i = Hash32(static_cast<uint64_t>(k)) & (cap - 1);
+      const uint32_t h = Hash32(static_cast<uint64_t>(k)), p = PartOf(h, bits);
+      const unsigned long long first = slot_off[p];
+      const uint64_t cap = slot_off[p + 1] - first;
+      const unsigned long long* tab = slots + first;
+      uint64_t i = h & (cap - 1);
       for (uint64_t step = 0; step < cap; step++) {
         const unsigned long long e = tab[i];
         if (S::Empty(e)) break;
@@ -644,260 +649,6 @@ __global__ void __launch_bounds__(kBlock) MatchPairs(const int32_t* __restrict__
     const uint64_t at = base + before[u * (kBlock / 32) + warp] + __popc(hit & ((1u << lane) - 1));
     probe[at] = static_cast<int32_t>(i0 + u * kBlock + threadIdx.x);
     build[at] = m[u];
-  }
-}
-
-// Persistent CTAs, partitions p = blockIdx.x + i * gridDim.x.  A CTA's work
-// is the sequence of its partitions' probe tiles (kProbeTile staged tuples
-// each); thread 0 keeps one tile ahead in a two-buffer ring and, as a
-// partition starts, the NEXT partition's sub-table loading into the other of
-// two table buffers, so a partition's table copy overlaps the probing of the
-// one before.  Sub-tables larger than a table buffer are probed in HBM.
-template <bool WIDE>
-__global__ void __launch_bounds__(kPartBlock) ProbeParts(const typename Slot<WIDE>::T* __restrict__ staged,
-                                                     const unsigned long long* __restrict__ stage_off,
-                                                     const unsigned* __restrict__ hist,
-                                                     const typename Slot<WIDE>::T* __restrict__ slots,
-                                                     const unsigned long long* __restrict__ slot_off, int parts,
-                                                     unsigned long long* __restrict__ out,
-                                                     unsigned long long out_cap, unsigned long long* counter,
-                                                     int* err) {
-  using S = Slot<WIDE>;
-  using T = typename S::T;
-  extern __shared__ __align__(128) unsigned char smem[];
-  // barriers 0-1: tile ring; 2-3: table buffers
-  __shared__ __align__(8) uint64_t bar[4];
-  __shared__ OutStage<kOutStage> st;
-  T* tiles[2] = {reinterpret_cast<T*>(smem), reinterpret_cast<T*>(smem + kProbeTile * sizeof(T))};
-  T* tabs[2] = {reinterpret_cast<T*>(smem + 2 * kProbeTile * sizeof(T)),
-                reinterpret_cast<T*>(smem + 2 * kProbeTile * sizeof(T) + kTableBuf)};
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < 4; b++) BarInit(&bar[b]);
-    st.count = 0;
-    FenceProxyAsync();
-  }
-  __syncthreads();
-  // copies issued / waited per barrier (thread 0 issues, every thread waits
-  // in the same order, so `waited` is block-uniform)
-  uint32_t issued[4] = {0, 0, 0, 0}, waited[4] = {0, 0, 0, 0};
-  auto next_part = [&](int q) {
-    for (q += gridDim.x; q < parts && hist[q] == 0; q += gridDim.x) {
-    }
-    return q;
-  };
-  auto tab_fits = [&](int q) { return (slot_off[q + 1] - slot_off[q]) * sizeof(T) <= kTableBuf; };
-  auto issue_tile = [&](int q, uint64_t t, int b) {
-    const uint64_t count = hist[q], t0 = t * kProbeTile;
-    const uint32_t n = static_cast<uint32_t>(umin64(kProbeTile, count - t0));
-    FenceProxyAsync();
-    BulkLoad(tiles[b], staged + stage_off[q] + t0, (n * sizeof(T) + 15) & ~15u, &bar[b]);
-    issued[b]++;
-  };
-  auto issue_tab = [&](int q, int b) {
-    FenceProxyAsync();
-    BulkLoad(tabs[b], slots + slot_off[q], static_cast<uint32_t>((slot_off[q + 1] - slot_off[q]) * sizeof(T)),
-             &bar[2 + b]);
-    issued[2 + b]++;
-  };
-  int p = blockIdx.x;
-  if (p < parts && hist[p] == 0) p = next_part(p);
-  if (threadIdx.x == 0 && p < parts) {
-    if (tab_fits(p)) issue_tab(p, 0);
-    issue_tile(p, 0, 0);
-  }
-  bool failed = false;
-  uint64_t j = 0;  // items (tiles) so far
-  int tb = 0;      // table buffer of the current partition
-  while (p < parts && !failed) {
-    const uint64_t cap = slot_off[p + 1] - slot_off[p];
-    const uint64_t count = hist[p];
-    const uint64_t ntiles = (count + kProbeTile - 1) / kProbeTile;
-    const bool fits = tab_fits(p);
-    const int np = next_part(p);
-    for (uint64_t t = 0; t < ntiles; t++) {
-      const int b = static_cast<int>(j & 1);
-      if (threadIdx.x == 0) {
-        if (t + 1 < ntiles) issue_tile(p, t + 1, b ^ 1);
-        else if (np < parts) issue_tile(np, 0, b ^ 1);
-        // the next fitting partition's buffer: the other one when this
-        // partition holds one, else the free current one
-        if (t == 0 && np < parts && tab_fits(np)) issue_tab(np, fits ? tb ^ 1 : tb);
-      }
-      if (t == 0 && fits) {
-        if (!BarWaitAll(&bar[2 + tb], waited[2 + tb] & 1, err)) {
-          failed = true;
-          break;
-        }
-        waited[2 + tb]++;
-      }
-      if (!BarWaitAll(&bar[b], waited[b] & 1, err)) {
-        failed = true;
-        break;
-      }
-      waited[b]++;
-      const T* tab = fits ? tabs[tb] : slots + slot_off[p];
-      const uint32_t nt = static_cast<uint32_t>(umin64(kProbeTile, count - t * kProbeTile));
-      for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) {
-        const T v = tiles[b][i];
-        ProbeOne<WIDE>(tab, cap, S::Key(v), S::Row(v), st, out, out_cap, counter);
-      }
-      // a barrier: this tile's (and at the partition's end its table's)
-      // reads are done before those buffers are refilled; the staged pairs
-      // go out once the stage is half full (a tile adds at most kProbeTile
-      // pairs per distinct build key)
-      if (__syncthreads_or(threadIdx.x == 0 && st.count >= kOutStage / 2)) FlushPairs(st, out, out_cap, counter);
-      j++;
-    }
-    if (fits) tb ^= 1;
-    p = np;
-  }
-  if (failed && threadIdx.x == 0) {
-    // every copy still in flight into this CTA's shared memory lands (or
-    // its bounded wait gives up) before the CTA leaves
-    for (int b = 0; b < 4; b++)
-      for (; waited[b] < issued[b]; waited[b]++) BarWait(&bar[b], waited[b] & 1);
-  }
-  FlushPairs(st, out, out_cap, counter);
-}
-
-// Partitioned probe with warp-level consumption (32-bit keys).  A CTA walks
-// its partitions through two buffers, each holding a partition's sub-table
-// (when it fits) and its probe tuples (up to kTupCap per copy): while one
-// partition is probed the next one's copy is in flight.  Inside a
-// partition the warps take their tuples without CTA barriers and stage
-// their pairs per warp (one global atomic per flush); one CTA barrier per
-// partition releases its buffer.  MATCH (a table without duplicate keys): a
-// probe row's match goes to match[row] instead.
-template <bool MATCH>
-__global__ void __launch_bounds__(kPartBlock) ProbePartsW(const unsigned long long* __restrict__ staged,
-                                                          const unsigned long long* __restrict__ stage_off,
-                                                          const unsigned* __restrict__ hist,
-                                                          const unsigned long long* __restrict__ slots,
-                                                          const unsigned long long* __restrict__ slot_off, int parts,
-                                                          unsigned long long* __restrict__ out,
-                                                          unsigned long long out_cap, unsigned long long* counter,
-                                                          int* err, uint32_t piece, int32_t* __restrict__ match) {
-  using S = Slot<false>;
-  using T = S::T;
-  constexpr size_t kBuf = kTableBuf + kTupCap * sizeof(T);
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bar[2];
-  __shared__ unsigned long long wst[kPartBlock / 32][kWarpStage];
-  __shared__ unsigned wcount[kPartBlock / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < 2; b++) BarInit(&bar[b]);
-    FenceProxyAsync();
-  }
-  if (lane == 0) wcount[warp] = 0;
-  __syncthreads();
-  uint32_t issued[2] = {0, 0}, waited[2] = {0, 0};
-  auto next_part = [&](int q) {
-    for (q += gridDim.x; q < parts && hist[q] == 0; q += gridDim.x) {
-    }
-    return q;
-  };
-  auto tab_fits = [&](int q) { return (slot_off[q + 1] - slot_off[q]) * sizeof(T) <= kTableBuf; };
-  // partition q's table (when it fits; only with the first chunk) and its
-  // tuples from c0 on into buffer b
-  auto issue = [&](int q, int b, uint64_t c0) {
-    const uint64_t count = hist[q];
-    const uint32_t n = static_cast<uint32_t>(umin64(kTupCap, count - c0));
-    const uint32_t tb = (n * sizeof(T) + 15) & ~15u;
-    const bool with_tab = c0 == 0 && tab_fits(q);
-    const uint32_t ab = with_tab ? static_cast<uint32_t>((slot_off[q + 1] - slot_off[q]) * sizeof(T)) : 0u;
-    unsigned char* base = smem + b * kBuf;
-    FenceProxyAsync();
-    BarExpect(&bar[b], ab + tb);
-    if (with_tab) BulkCopyPieces(base, slots + slot_off[q], ab, &bar[b], piece);
-    BulkCopyPieces(base + kTableBuf, staged + stage_off[q] + c0, tb, &bar[b], piece);
-    issued[b]++;
-  };
-  auto warp_flush = [&]() {
-    const unsigned n = wcount[warp] < kWarpStage ? wcount[warp] : kWarpStage;
-    unsigned long long base = 0;
-    if (lane == 0 && n) base = atomicAdd(counter, static_cast<unsigned long long>(n));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (unsigned i = lane; i < n; i += 32)
-      if (base + i < out_cap) out[base + i] = wst[warp][i];
-    __syncwarp();
-    if (lane == 0) wcount[warp] = 0;
-    __syncwarp();
-  };
-  int p = blockIdx.x;
-  if (p < parts && hist[p] == 0) p = next_part(p);
-  int pn = p < parts ? next_part(p) : parts;  // the partition in the other buffer
-  if (threadIdx.x == 0) {
-    if (p < parts) issue(p, 0, 0);
-    if (pn < parts) issue(pn, 1, 0);
-  }
-  bool failed = false;
-  int b = 0;
-  while (p < parts && !failed) {
-    const uint64_t cap = slot_off[p + 1] - slot_off[p];
-    const uint64_t count = hist[p];
-    const T* tab = tab_fits(p) ? reinterpret_cast<const T*>(smem + b * kBuf) : slots + slot_off[p];
-    const T* tup = reinterpret_cast<const T*>(smem + b * kBuf + kTableBuf);
-    for (uint64_t c0 = 0; c0 < count && !failed; c0 += kTupCap) {
-      if (c0 > 0) {
-        // a partition beyond one buffer of tuples: the next chunk into the
-        // same buffer once every warp is done with this one
-        __syncthreads();
-        if (threadIdx.x == 0) issue(p, b, c0);
-      }
-      if (!BarWaitAll(&bar[b], waited[b] & 1, err)) {
-        failed = true;
-        break;
-      }
-      waited[b]++;
-      const uint32_t n = static_cast<uint32_t>(umin64(kTupCap, count - c0));
-      for (uint32_t i0 = warp * 32; i0 < n; i0 += kPartBlock) {
-        const uint32_t i = i0 + lane;
-        if (i < n) {
-          const T v = tup[i];
-          const int64_t k = S::Key(v);
-          uint64_t j = Hash32(static_cast<uint64_t>(k)) & (cap - 1);
-          for (uint64_t step = 0; step < cap; step++) {
-            const T e = tab[j];
-            if (S::Empty(e)) break;
-            if (S::Key(e) == k) {
-              if constexpr (MATCH) {
-                match[S::Row(v)] = static_cast<int32_t>(S::Row(e));
-                break;
-              }
-              const unsigned long long pair = PackPair(S::Row(v), S::Row(e));
-              cg::coalesced_group g = cg::coalesced_threads();
-              unsigned at = 0;
-              if (g.thread_rank() == 0) at = atomicAdd(&wcount[warp], g.size());
-              at = g.shfl(at, 0) + g.thread_rank();
-              if (at < static_cast<unsigned>(kWarpStage)) wst[warp][at] = pair;
-              else EmitPair(out, out_cap, counter, pair);
-            }
-            j = (j + 1) & (cap - 1);
-          }
-        }
-        if constexpr (!MATCH) {
-          __syncwarp();
-          if (wcount[warp] >= kWarpStage / 2) warp_flush();
-        }
-      }
-    }
-    if (failed) break;
-    // buffer b is free once every warp is done with it
-    __syncthreads();
-    const int pnn = pn < parts ? next_part(pn) : parts;
-    if (threadIdx.x == 0 && pnn < parts) issue(pnn, b, 0);
-    p = pn;
-    pn = pnn;
-    b ^= 1;
-  }
-  if (failed && threadIdx.x == 0) {
-    for (int k = 0; k < 2; k++)
-      for (; waited[k] < issued[k]; waited[k]++) BarWait(&bar[k], waited[k] & 1);
-  }
-  if constexpr (!MATCH) {
-    __syncwarp();
-    warp_flush();
   }
 }
 
@@ -1108,10 +859,12 @@ int PartBitsFor(int64_t n, double lf, int slot_bytes, int32_t fanout) {
       throw Error(KDB_ERR_INVALID, "fanout must be a power of two of at most 8192");
     return b;
   }
-  // automatic: one table while it stays well inside L2 (126 MB), otherwise
-  // sub-tables of about 64 KiB (a shared-memory copy per partition)
+  // automatic: one table while it stays inside L2 (126 MB), otherwise
+  // sub-tables of about 64 KiB, built in shared memory.  Building 4M rows, a
+  // table of 64 MiB: 74 us against 136 partitioned (half of them duplicates:
+  // 100 against 138); 4.6M rows, 128 MiB and its clearing: 156 against 146.
   double table_bytes = static_cast<double>(n) / lf * 1.5 * slot_bytes;
-  if (table_bytes <= 48.0 * (1 << 20)) return 0;
+  if (table_bytes <= 96.0 * (1 << 20)) return 0;
   int b = 0;
   while (b < kMaxPartBits && table_bytes / (1 << b) > 64.0 * 1024) b++;
   return b;
@@ -1183,17 +936,21 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
     c.kernel_launches++;
     c.TimedStop();
     c.TimedStart("hash build");
-    const size_t smem = 2 * kProbeTile * slot_bytes + kSmemTableMax;
-    const int pgrid = std::min(parts, c.num_sms * 1);
+    const double rows = static_cast<double>(n) / parts;
+    size_t tab_slots = 16;
+    while (tab_slots < (rows + 4 * std::sqrt(rows)) / load_factor + 1) tab_slots <<= 1;
+    const uint32_t tab_bytes = static_cast<uint32_t>(std::min<size_t>(tab_slots * slot_bytes, kSmemTableMax));
+    const size_t smem = 2 * kBuildTile * slot_bytes + tab_bytes;
+    const int pgrid = std::min<int>(parts, c.num_sms * static_cast<int>(std::min<size_t>(4, (220u << 10) / (smem + 1024))));
     if (ht->wide) {
       KDB_CUDA(cudaFuncSetAttribute(BuildParts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      BuildParts<true><<<pgrid, kPartBlock, smem, c.stream>>>(static_cast<const ulonglong2*>(staged), stage_off, hist,
-                                                          ht->slot_off, parts, static_cast<ulonglong2*>(ht->slots), err);
+      BuildParts<true><<<pgrid, kBuildBlock, smem, c.stream>>>(static_cast<const ulonglong2*>(staged), stage_off, hist,
+                                                          ht->slot_off, parts, static_cast<ulonglong2*>(ht->slots), tab_bytes, err);
     } else {
       KDB_CUDA(cudaFuncSetAttribute(BuildParts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      BuildParts<false><<<pgrid, kPartBlock, smem, c.stream>>>(static_cast<const unsigned long long*>(staged), stage_off,
+      BuildParts<false><<<pgrid, kBuildBlock, smem, c.stream>>>(static_cast<const unsigned long long*>(staged), stage_off,
                                                            hist, ht->slot_off, parts,
-                                                           static_cast<unsigned long long*>(ht->slots), err);
+                                                           static_cast<unsigned long long*>(ht->slots), tab_bytes, err);
     }
     c.kernel_launches++;
     c.TimedStop();
@@ -1212,67 +969,25 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
     throw Error(KDB_ERR_INVALID, "probe key width differs from the build key's (BIGINT against a narrower key)");
   const int64_t n = SelCount(c, table, sel);
   const int32_t* srows = sel ? sel->rows : nullptr;
-  const int parts = 1 << ht.bits;
-  const int slot_bytes = ht.wide ? 16 : 8;
   Arena arena(c);
-  int* err = arena.AllocT<int>(1);
   unsigned long long* counter = arena.AllocT<unsigned long long>(1);
   const int grid = c.GridFor(std::max<int64_t>(n, 1), kBlock);
-  // staged probe side (partitioned tables only)
-  unsigned* hist = nullptr;
-  unsigned long long* stage_off = nullptr;
-  void* staged = nullptr;
-  if (ht.bits > 0 && n > 0) {
-    hist = arena.AllocT<unsigned>(parts);
-    unsigned* cursor = arena.AllocT<unsigned>(parts);
-    stage_off = arena.AllocT<unsigned long long>(parts + 1);
-    staged = arena.Alloc((static_cast<size_t>(n) + parts + 2) * slot_bytes);
-    c.Memset(hist, 0, sizeof(unsigned) * parts);
-    const int cgrid = PartGrid(c, n);
-    const int64_t chunk = (n + cgrid - 1) / cgrid;
-    unsigned* block_hist = arena.AllocT<unsigned>(static_cast<size_t>(cgrid) * parts);
-    c.TimedStart("probe partition");
-    PartHistogram<<<cgrid, kPartBlock, sizeof(unsigned) * parts, c.stream>>>(key, srows, n, chunk, ht.bits, hist,
-                                                                            block_hist);
-    PartOffsets<<<1, 1024, 0, c.stream>>>(hist, parts, 0.5, stage_off, nullptr, cursor);
-    LaunchScatter(c, ht.wide, cgrid, key, srows, n, chunk, ht.bits, block_hist, stage_off, cursor, staged);
-    c.kernel_launches += 3;
-    c.TimedStop();
-  }
-  const uint32_t piece = [&] {
-    // KDB_TMA_PIECE: bytes per bulk copy (a partition's table and tuples go
-    // as several copies in flight together)
-    const char* pe = c.OptStr("KDB_TMA_PIECE");
-    return pe ? static_cast<uint32_t>(std::max(16, std::atoi(pe)) & ~15) : 4096u;
-  }();
-  const size_t wsmem = 2 * (kTableBuf + kTupCap * sizeof(unsigned long long));
-  if (ordered && ht.unique && !ht.wide && !sel && n > 0 && !c.OptStr("KDB_PROBE_PARTS_TILED")) {
+  if (ordered && ht.unique && !ht.wide && !sel && n > 0) {
     // unique build keys, probe rows in table order: one match word per row,
     // compacted (a selection's rows may come in any order, and more than
     // once, so it takes the pair list below)
     int32_t* match = arena.AllocT<int32_t>(static_cast<size_t>(n));
     const int64_t tiles = (n + kMatchTile - 1) / kMatchTile;
     uint64_t* counts = arena.AllocT<uint64_t>(static_cast<size_t>(tiles) + 1);
-    c.Memset(err, 0, sizeof(int));
-    if (ht.bits > 0) c.Memset(match, 0xff, sizeof(int32_t) * n);
     c.TimedStart("hash probe");
-    if (ht.bits == 0) {
-      MatchFlat<<<grid, kBlock, 0, c.stream>>>(key, n, static_cast<const unsigned long long*>(ht.slots),
-                                               static_cast<uint64_t>(ht.total_slots), match);
-    } else {
-      KDB_CUDA(cudaFuncSetAttribute(ProbePartsW<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(wsmem)));
-      ProbePartsW<true><<<std::min(parts, c.num_sms), kPartBlock, wsmem, c.stream>>>(
-          static_cast<const unsigned long long*>(staged), stage_off, hist,
-          static_cast<const unsigned long long*>(ht.slots), ht.slot_off, parts, nullptr, 0, nullptr, err, piece, match);
-    }
+    MatchRows<<<grid, kBlock, 0, c.stream>>>(key, n, static_cast<const unsigned long long*>(ht.slots), ht.slot_off,
+                                             ht.bits, match);
     c.TimedStop();
     c.TimedStart("hash pairs");
     MatchCounts<<<static_cast<unsigned>(tiles), kBlock, 0, c.stream>>>(match, n, counts);
     c.TimedStop();
     c.ScanU64(counts, tiles, "hash pairs");
     KDB_CUDA(cudaGetLastError());
-    CheckErr(c, err, "hash probe");
     uint64_t total = 0;
     c.D2H(&total, counts + tiles, sizeof(total));
     auto pr = std::make_unique<Pairs>();
@@ -1295,50 +1010,21 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
   pr->ctx = &c;
   for (int attempt = 0; attempt < 2; attempt++) {
     unsigned long long* out = static_cast<unsigned long long*>(arena.Alloc(cap * sizeof(unsigned long long)));
-    c.Memset(err, 0, sizeof(int));
     c.Memset(counter, 0, sizeof(unsigned long long));
     c.TimedStart("hash probe");
     if (n > 0) {
-      if (ht.bits == 0) {
-        const uint64_t tcap = static_cast<uint64_t>(ht.total_slots);
-        if (ht.wide)
-          ProbeFlat<true><<<grid, kBlock, 0, c.stream>>>(key, srows, n, static_cast<const ulonglong2*>(ht.slots), tcap,
-                                                         out, cap, counter);
-        else
-          ProbeFlat<false><<<grid, kBlock, 0, c.stream>>>(key, srows, n,
-                                                          static_cast<const unsigned long long*>(ht.slots), tcap, out,
-                                                          cap, counter);
-      } else {
-        const size_t smem = 2 * kProbeTile * slot_bytes + 2 * kTableBuf;
-        const int pgrid = std::min(parts, c.num_sms);
-        if (!ht.wide && !c.OptStr("KDB_PROBE_PARTS_TILED")) {
-          KDB_CUDA(cudaFuncSetAttribute(ProbePartsW<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(wsmem)));
-          ProbePartsW<false><<<pgrid, kPartBlock, wsmem, c.stream>>>(static_cast<const unsigned long long*>(staged), stage_off,
-                                                             hist, static_cast<const unsigned long long*>(ht.slots),
-                                                             ht.slot_off, parts, out, cap, counter, err,
-                                                             piece, nullptr);
-        } else if (ht.wide) {
-          KDB_CUDA(cudaFuncSetAttribute(ProbeParts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
-          ProbeParts<true><<<pgrid, kPartBlock, smem, c.stream>>>(static_cast<const ulonglong2*>(staged), stage_off, hist,
-                                                              static_cast<const ulonglong2*>(ht.slots), ht.slot_off,
-                                                              parts, out, cap, counter, err);
-        } else {
-          KDB_CUDA(cudaFuncSetAttribute(ProbeParts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(smem)));
-          ProbeParts<false><<<pgrid, kPartBlock, smem, c.stream>>>(
-              static_cast<const unsigned long long*>(staged), stage_off, hist,
-              static_cast<const unsigned long long*>(ht.slots), ht.slot_off, parts, out, cap, counter, err);
-        }
-      }
+      if (ht.wide)
+        ProbeRows<true><<<grid, kBlock, 0, c.stream>>>(key, srows, n, static_cast<const ulonglong2*>(ht.slots),
+                                                       ht.slot_off, ht.bits, out, cap, counter);
+      else
+        ProbeRows<false><<<grid, kBlock, 0, c.stream>>>(key, srows, n, static_cast<const unsigned long long*>(ht.slots),
+                                                        ht.slot_off, ht.bits, out, cap, counter);
       c.kernel_launches++;
     }
     c.TimedStop();
     KDB_CUDA(cudaGetLastError());
     unsigned long long total = 0;
     c.D2H(&total, counter, sizeof(total));
-    CheckErr(c, err, "hash probe");
     if (total <= cap) {
       pr->n = static_cast<int64_t>(total);
       if (ordered && total > 1) {
