@@ -76,3 +76,36 @@ def test_order_matches_reference_merge_sort(setup, keys, asc, sort):
         for name, _ in opts:
             e.set_option(name, None)
     assert compare(got, o.execute(plan), ordered=True) == ""
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 33, 128, 129, 2048, 2049, 4096, 4097])
+@pytest.mark.parametrize("keys,asc", [(["r"], [True]), (["i"], [False]), (["s"], [True]),
+                                      (["i", "s", "r"], [False, True, False])])
+def test_small_order_matches_reference_merge_sort(n, keys, asc):
+    """Around the sizes where comparing all pairs of rows hands over to the
+    range buckets (one numeric key) and to the radix passes (other keys):
+    ties, NULLs, strings."""
+    from kushdb_b200.engine import Engine
+    from oracle import Oracle
+    rng = np.random.default_rng(n)
+    t = HostTable("ob_small")
+    t.add(HostColumn("id", Type.Int(), values=np.arange(n, dtype=np.int32)))
+    t.add(HostColumn("r", Type.Real(), values=rng.integers(0, 900, n).astype(np.float64) / 4.0,
+                     nulls=(rng.random(n) < 0.1).astype(np.int8)))
+    t.add(HostColumn("i", Type.Int(), values=rng.integers(-5, 5, n).astype(np.int32)))
+    t.add(HostColumn.from_strings("s", ["k" * int(a) + str(int(b)) for a, b in
+                                        zip(rng.integers(0, 4, n), rng.integers(0, 30, n))]))
+    rel = catalog_of([t])[t.name]
+    s = OperatorSchema()
+    s.AddGeneratedColumns(rel, ["id", "r", "i", "s"])
+    base = ScanOperator(s, rel)
+    out = OperatorSchema()
+    out.AddPassthroughColumns(base)
+    plan = OutputOperator(OrderByOperator(out, base, [ColRef(base, k) for k in keys], asc)).to_json()
+    o = Oracle()
+    o.register_table(t)
+    with Engine(0) as e:
+        e.register_table(t)
+        want = o.execute(plan)
+        for _ in range(3):  # fresh, recorded and replayed
+            assert compare(e.execute(plan), want, ordered=True) == ""
