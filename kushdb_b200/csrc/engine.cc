@@ -747,9 +747,14 @@ void Context::Launch(CUfunction f, int grid, int block, const KArgs& args, size_
   }
 }
 
+cudaEvent_t Context::MarkEvent() {
+  if (!query_ev_[2]) KDB_CUDA(cudaEventCreateWithFlags(&query_ev_[2], cudaEventDisableTiming));
+  return query_ev_[2];
+}
+
 void Context::QueryEvents(cudaEvent_t* start, cudaEvent_t* end) {
-  for (cudaEvent_t& e : query_ev_)
-    if (!e) KDB_CUDA(cudaEventCreate(&e));
+  for (int i = 0; i < 2; i++)
+    if (!query_ev_[i]) KDB_CUDA(cudaEventCreate(&query_ev_[i]));
   *start = query_ev_[0];
   *end = query_ev_[1];
 }
@@ -813,6 +818,24 @@ uint64_t Context::ReadWordChecked(const uint64_t* d, const char* what) {
   std::memcpy(&err, h + 1, sizeof(err));
   ThrowDeviceError(err, what);
   return word;
+}
+
+void Context::ReadWordsChecked(uint64_t* h, const uint64_t* d, size_t words, const char* what) {
+  const size_t off = (words * sizeof(uint64_t) + 15) & ~size_t(15);
+  if (dry) {
+    std::memset(h, 0, words * sizeof(uint64_t));
+    return;
+  }
+  char* stage = static_cast<char*>(HostStage(off + 16));
+  PackSegs segs;
+  segs.seg[segs.n++] = PackSeg{reinterpret_cast<const char*>(d), words * sizeof(uint64_t), 0};
+  segs.seg[segs.n++] = PackSeg{reinterpret_cast<const char*>(d_err), 16, off};
+  PackToHost(segs, off + 16, stage);
+  KDB_CUDA(cudaStreamSynchronize(stream));
+  std::memcpy(h, stage, words * sizeof(uint64_t));
+  int err;
+  std::memcpy(&err, stage + off, sizeof(err));
+  ThrowDeviceError(err, what);
 }
 
 void Context::ThrowDeviceError(int err, const char* what) {

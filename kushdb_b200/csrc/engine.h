@@ -361,6 +361,8 @@ class Context {
   void DelayStream(double us);
   // the two events that time each query (made on first use)
   void QueryEvents(cudaEvent_t* start, cudaEvent_t* end);
+  // An event for waiting on a point of the stream while later work runs.
+  cudaEvent_t MarkEvent();
   void TimedStart(const char* tag);
   void TimedStop();
   int GridFor(int64_t n, int block) const;
@@ -432,17 +434,20 @@ class Context {
   void CheckDeviceError(const char* what);
   // the word at `d` and the device error word, in one round trip
   uint64_t ReadWordChecked(const uint64_t* d, const char* what);
+  // Throws for a device error word that is not 0 (and clears the device's).
+  void ThrowDeviceError(int err, const char* what);
+  // `words` device words and the device error word in one round trip.
+  void ReadWordsChecked(uint64_t* h, const uint64_t* d, size_t words, const char* what);
 
   EnumDicts HostEnums() const;
 
  private:
   std::shared_ptr<ProgramCache> cache_ = std::make_shared<ProgramCache>();
-  cudaEvent_t query_ev_[2] = {nullptr, nullptr};
+  cudaEvent_t query_ev_[3] = {nullptr, nullptr, nullptr};  // two of the timer, one of MarkEvent
   bool owns_catalog_ = true;
   struct ResultSlots;
   std::shared_ptr<ResultSlots> result_slots_;
   uint64_t* scan_sums_ = nullptr;  // part sums of ScanParted (made on first use)
-  void ThrowDeviceError(int err, const char* what);
   void ScanParted(uint64_t* a, int64_t n, const uint64_t* n_ptr);
   void* stage_ = nullptr;
   size_t stage_bytes_ = 0;

@@ -173,3 +173,52 @@ def test_grouped_index_edges_match_oracle(engine, rows, keys):
     finally:
         engine.set_skinner()
     assert compare(g, o.execute(plan)) == ""
+
+
+# filtered children are counted while the others' indexes build: none, some or
+# all of them filtered, a filter that keeps one row, all rows or none
+@pytest.mark.parametrize("filtered", [(), (1,), (0, 2), (0, 1, 2)])
+@pytest.mark.parametrize("keep", ["none", "one", "some", "all"])
+def test_filtered_children_match_oracle(engine, filtered, keep):
+    import numpy as np
+    from kushdb_b200.data import HostColumn, HostTable, catalog_of
+    from kushdb_b200.plan import (AggregateOperator, ColRef, Count, Eq, Literal, Lt, OperatorSchema, OutputOperator,
+                                  ScanOperator, ScanSelectOperator, SkinnerJoinOperator, Sum, Type, VirtColRef)
+    from oracle import Oracle
+    rng = np.random.default_rng(17)
+    tables = []
+    for i, n in enumerate((3000, 400, 1500)):
+        t = HostTable(f"fc_{i}_{len(filtered)}_{keep}")
+        t.add(HostColumn("k", Type.Int(), values=rng.integers(0, 90, n).astype(np.int32)))
+        t.add(HostColumn("g", Type.Int(), values=rng.integers(0, 120, n).astype(np.int32),
+                         nulls=(rng.random(n) < 0.1).astype(np.int8)))
+        t.add(HostColumn("id", Type.Int(), values=np.arange(n, dtype=np.int32)))
+        tables.append(t)
+    below = {"none": 0, "one": 1, "some": 350, "all": 3000}[keep]
+    db = catalog_of(tables)
+    kids = []
+    for i, t in enumerate(tables):
+        s = OperatorSchema()
+        s.AddGeneratedColumns(db[t.name], ["k", "g", "id"])
+        if i in filtered:
+            out = OperatorSchema()
+            out.AddVirtualPassthroughColumns(s, ["k", "g", "id"])
+            kids.append(ScanSelectOperator(out, s, db[t.name], [Lt(VirtColRef(s, "id"), Literal(below))]))
+        else:
+            kids.append(ScanOperator(s, db[t.name]))
+    js = OperatorSchema()
+    js.AddPassthroughColumns(kids[0], ["id"], 0)
+    join = SkinnerJoinOperator(js, kids, [Eq(ColRef(kids[0], "k", 0), ColRef(kids[1], "k", 1)),
+                                          Eq(ColRef(kids[1], "g", 1), ColRef(kids[2], "g", 2))])
+    aggs = [Count(), Sum(ColRef(join, "id"))]
+    out = OperatorSchema()
+    for i, name in enumerate(("n", "total")):
+        out.AddDerivedColumn(name, VirtColRef(aggs[i], i))
+    plan = OutputOperator(AggregateOperator(out, join, aggs))
+    o = Oracle()
+    for t in tables:
+        engine.register_table(t)
+        o.register_table(t)
+    want = o.execute(plan)
+    for _ in range(2):
+        assert compare(engine.execute(plan), want) == ""
