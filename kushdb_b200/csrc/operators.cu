@@ -54,6 +54,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;        // bounded mbarrier waits
 constexpr int kErrWait = 1;                      // device error word: a wait gave up
 constexpr int kErrFull = 2;                      // a table ran out of empty slots
 constexpr int kDupKey = 4;                       // (not an error) two build rows share a key
+constexpr int64_t kMatchRowsMin = 1 << 21;       // unordered probes from here on by match words
 constexpr int kMatchTile = 4096;                 // probe rows per CTA when matches are compacted
 constexpr unsigned kOutStage = 2048;             // pairs a probe CTA stages
 
@@ -526,8 +527,9 @@ __device__ __forceinline__ void ProbeOne(const typename Slot<WIDE>::T* slots, co
 // sub-tables there are: with 2048 threads an SM in flight, reading a slot
 // sector per row costs less than writing the rows out by partition and
 // copying every sub-table into shared memory.  4M x 3M rows: 46 us against
-// 47 + 76; 30M x 20M: 520 against 601 + 416; with every build key 8 times,
-// 48 against 22 + 419.
+// 47 + 76; with every build key 8 times, 48 against 22 + 419.  (More rows in
+// flight per thread were slower, 80 against 62 us for 2M x 2M: the pairs'
+// staging is the other half of the time.)
 template <bool WIDE>
 __global__ void __launch_bounds__(kBlock) ProbeRows(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
                                                     const typename Slot<WIDE>::T* __restrict__ slots,
@@ -972,10 +974,13 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
   Arena arena(c);
   unsigned long long* counter = arena.AllocT<unsigned long long>(1);
   const int grid = c.GridFor(std::max<int64_t>(n, 1), kBlock);
-  if (ordered && ht.unique && !ht.wide && !sel && n > 0) {
+  if (ht.unique && !ht.wide && !sel && n > 0 && (ordered || n >= kMatchRowsMin)) {
     // unique build keys, probe rows in table order: one match word per row,
     // compacted (a selection's rows may come in any order, and more than
-    // once, so it takes the pair list below)
+    // once, so it takes the pair list below).  From kMatchRowsMin rows on
+    // unordered pairs are made so, too: as a pair list 3M probes of 6M rows
+    // took 95 us against 80, 20M of 30M 1121 against 589, but 100k 13
+    // against 33 for the more launches.
     int32_t* match = arena.AllocT<int32_t>(static_cast<size_t>(n));
     const int64_t tiles = (n + kMatchTile - 1) / kMatchTile;
     uint64_t* counts = arena.AllocT<uint64_t>(static_cast<size_t>(tiles) + 1);

@@ -433,3 +433,26 @@ def test_sort_rows_matches_order_by_semantics(engine, keys, asc, with_sel):
     got = sort_rows(engine, t.name, keys, asc, sel=sel).rows()
     assert list(got) == _sorted_rows(cols, keys, asc, rows)
     engine.drop_table(t.name)
+
+
+def test_unordered_unique_probe_on_both_sides_of_the_match_rows_size(engine):
+    """Unordered pairs of a unique build: as a pair list below 2^21 probe rows,
+    by match words from there on; the same set of pairs either way."""
+    from kushdb_b200.operators import HashTable
+    nb = 5_000
+    rng = np.random.default_rng(8)
+    b = _key_table("ops_un_b", rng.permutation(nb).astype(np.int32))
+    engine.register_table(b)
+    inv = np.empty(nb, np.int64)
+    inv[b.columns["k"].values] = np.arange(nb)
+    ht = HashTable(engine, b.name, "k")
+    for np_ in ((1 << 21) - 1, 1 << 21):
+        pk = rng.integers(-50, nb + 50, np_).astype(np.int32)
+        p = _key_table(f"ops_un_p{np_}", pk)
+        engine.register_table(p)
+        got_p, got_b = ht.probe(p.name, "k", ordered=False)
+        order = np.argsort(got_p, kind="stable")
+        hit = np.nonzero((pk >= 0) & (pk < nb))[0]
+        np.testing.assert_array_equal(np.asarray(got_p)[order], hit)
+        np.testing.assert_array_equal(np.asarray(got_b)[order], inv[pk[hit]])
+    ht.close()
