@@ -1826,7 +1826,7 @@ JoinTable Executor::BuildIndex(const MatBuffer& m, const std::vector<int>& key_c
 //
 // Built by counting instead of sorting, every index of the call in the same
 // three launches: each row finds its hash's slot and takes a place in that
-// hash's group (a returning count, one atomic per distinct slot in a warp),
+// hash's group (CountIndexRows, one returning atomic per distinct slot in a warp),
 // the slots' groups are laid out (PlaceIndexGroups), and each row goes to its
 // place (FillIndexRows).  A radix sort per index took four passes over the
 // hashes and about ten launches each: 2.7 ms for the ten indexes of a star
@@ -1858,76 +1858,35 @@ std::vector<JoinTable> Executor::BuildGroupedIndexes(const std::vector<std::pair
     uint32_t* len_at = reinterpret_cast<uint32_t*>(region + slots * 8);
     unsigned long long* used = reinterpret_cast<unsigned long long*>(region + slots * 12);
     IndexBatch batch;
-    KernelSource ks;
-    ExprGen eg(ctx_, ks);
     int64_t blocks = 0;
-    ks.L("const int lane = threadIdx.x & 31;");
-    ks.L("int64_t r0 = 0, n = 0; uint64_t* slots = nullptr; uint32_t* lens = nullptr; uint32_t mask = 0; uint2* place = nullptr;");
-    ks.L("uint32_t hash[4]; bool ok[4];");
     for (size_t j = 0; j < nb; j++) {
       const MatBuffer& m = *cols[b0 + j].first;
+      const MatCol& mc = m.cols.at(cols[b0 + j].second);
       JoinTable& jt = out[b0 + j];
       const int64_t n = m.rows, cap = static_cast<int64_t>(jt.mask) + 1;
       jt.slots = slot_at;
       jt.lens = len_at;
       jt.srow = srow;
-      batch.index[j] = IndexBuild{jt.slots, jt.lens, place, jt.srow, used + j, cap, n};
-      const int64_t nblocks = (n + kIndexRows - 1) / kIndexRows;
-      if (n > 0) {
-        // this index's rows: kIndexRows per CTA, four per thread
-        ks.Open("if (blockIdx.x >= " + ks.Word(static_cast<uint64_t>(blocks)) + " && blockIdx.x < " +
-                ks.Word(static_cast<uint64_t>(blocks + nblocks)) + ")");
-        ks.L("r0 = (blockIdx.x - (int64_t)" + ks.Word(static_cast<uint64_t>(blocks)) + ") * " + std::to_string(kIndexRows) +
-             "; n = (int64_t)" + ks.Word(static_cast<uint64_t>(n)) + ";");
-        ks.L("slots = " + ks.Ptr(jt.slots, "uint64_t") + "; lens = " + ks.Ptr(jt.lens, "uint32_t") + "; place = " +
-             ks.Ptr(place, "uint2") + "; mask = (uint32_t)" + ks.Word(jt.mask) + ";");
-        ks.L("_Pragma(\"unroll\")");
-        ks.Open("for (int u = 0; u < 4; u++)");
-        ks.L("const int64_t r = r0 + u * 256 + threadIdx.x;");
-        ks.L("ok[u] = false; hash[u] = 0;");
-        ks.Open("if (r < n)");
-        const MatCol& mc = m.cols.at(cols[b0 + j].second);
-        std::string v = ks.Ptr(mc.data, StoreType(mc.type.id), true) + "[r]";
-        if (mc.type.id == TypeId::BOOLEAN) v = "(" + v + " != 0)";
-        const CVal key = eg.Bind(mc.type, v, mc.nullable ? "(" + ks.Ptr(mc.nulls, "int8_t", true) + "[r] != 0)" : "false");
-        ks.L("ok[u] = !(" + key.n + "); hash[u] = " + JoinHash(eg, {key}) + ";");
-        ks.Close();
-        ks.Close();
-        ks.Close();
+      int kind = kIndexI32;
+      switch (mc.type.id) {
+        case TypeId::BOOLEAN: kind = kIndexBool; break;
+        case TypeId::SMALLINT: kind = kIndexI16; break;
+        case TypeId::BIGINT: kind = kIndexI64; break;
+        case TypeId::REAL: kind = kIndexReal; break;
+        case TypeId::TEXT: kind = kIndexText; break;
+        default: break;
       }
+      batch.index[j] = IndexBuild{jt.slots, jt.lens, place, jt.srow, used + j, cap, n, mc.data,
+                                  mc.nullable ? mc.nulls : nullptr, kind};
       slot_at += cap;
       len_at += cap;
       srow += n;
       place += n;
-      blocks += nblocks;
+      blocks += (n + kIndexRows - 1) / kIndexRows;
     }
     batch.n = static_cast<int>(nb);
     if (blocks == 0) continue;
     if (blocks > std::numeric_limits<int>::max()) throw Error(-5, "join indexes over too many rows");
-    ks.L("_Pragma(\"unroll\")");
-    ks.Open("for (int u = 0; u < 4; u++)");
-    ks.L("const int64_t r = r0 + u * 256 + threadIdx.x;");
-    ks.L("uint32_t s = ~0u;");
-    ks.Open("if (ok[u])");
-    ks.L("const uint64_t e = ((uint64_t)hash[u] << 32) | 1ULL;  // nonzero; the group's index replaces the 1");
-    ks.L("s = hash[u] & mask;");
-    ks.Open("for (uint32_t k = 0; k <= mask; k++, s = (s + 1) & mask)");
-    ks.L("unsigned long long x = __ldcg((const unsigned long long*)&slots[s]);");
-    ks.L("if (x == 0) x = atomicCAS((unsigned long long*)&slots[s], 0ULL, (unsigned long long)e);");
-    ks.L("if (x == 0 || x == e) break;");
-    ks.Close();
-    ks.Close();
-    ks.L("__syncwarp();");
-    ks.L("const unsigned peers = __match_any_sync(0xffffffffu, s);");
-    ks.L("const int leader = __ffs(peers) - 1;");
-    ks.L("uint32_t at = 0;");
-    ks.L("if (lane == leader && ok[u]) at = atomicAdd(&lens[s], (uint32_t)__popc(peers));");
-    ks.L("at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & ((1u << lane) - 1));");
-    ks.L("if (r < n) place[r] = make_uint2(s, at);");
-    ks.Close();
-    const std::string name = KernelName("index count");
-    CUfunction f = ctx_.Kernel(ks.Kernel(name, 256), name);
-    ctx_.Launch(f, static_cast<int>(blocks), 256, ks.Args(), 0, "index count");
     ctx_.GroupIndexRows(batch);
   }
   return out;

@@ -169,7 +169,11 @@ struct IndexBuild {
   unsigned long long* used;  // rows of the groups laid out so far
   int64_t cap;               // slots
   int64_t n;                 // rows
+  const void* key;           // the key column as stored, and its NULL flags
+  const int8_t* nulls;
+  int kind;                  // an IndexKey
 };
+enum IndexKey { kIndexBool, kIndexI16, kIndexI32, kIndexI64, kIndexReal, kIndexText };
 struct IndexBatch {
   IndexBuild index[kMaxIndexBatch];
   int n = 0;

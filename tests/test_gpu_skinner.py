@@ -222,3 +222,48 @@ def test_filtered_children_match_oracle(engine, filtered, keep):
     want = o.execute(plan)
     for _ in range(2):
         assert compare(engine.execute(plan), want) == ""
+
+
+# the index hashes by the key column's stored type; lookups hash the same way
+@pytest.mark.parametrize("kind", ["BOOLEAN", "SMALLINT", "INT", "DATE", "BIGINT", "REAL", "TEXT"])
+def test_index_key_types_match_oracle(engine, kind):
+    import numpy as np
+    from kushdb_b200.data import HostColumn, HostTable, catalog_of
+    from kushdb_b200.plan import (AggregateOperator, ColRef, Count, Eq, OperatorSchema, OutputOperator, ScanOperator,
+                                  SkinnerJoinOperator, Sum, Type, VirtColRef)
+    from oracle import Oracle
+    rng = np.random.default_rng(29)
+    tables = []
+    for i, n in enumerate((900, 300, 60)):
+        t = HostTable(f"kt_{kind}_{i}")
+        v = rng.integers(-20, 20, n)
+        nulls = (rng.random(n) < 0.1).astype(np.int8)
+        if kind == "TEXT":
+            t.add(HostColumn.from_strings("k", ["s" * (int(x) % 5 + 5) + str(int(x)) for x in v], nulls))
+        else:
+            values = {"BOOLEAN": (v > 15).astype(np.int8), "SMALLINT": v.astype(np.int16), "INT": v.astype(np.int32),
+                      "DATE": (v + 2440588).astype(np.int32), "BIGINT": v * (1 << 33),
+                      "REAL": np.where(v == 0, -0.0 if i else 0.0, v * 0.37)}[kind]
+            t.add(HostColumn("k", Type(kind), values=values, nulls=nulls))
+        t.add(HostColumn("g", Type.Int(), values=rng.integers(0, 40, n).astype(np.int32)))
+        tables.append(t)
+    db = catalog_of(tables)
+    scans = []
+    for t in tables:
+        s = OperatorSchema()
+        s.AddGeneratedColumns(db[t.name], ["k", "g"])
+        scans.append(ScanOperator(s, db[t.name]))
+    js = OperatorSchema()
+    js.AddPassthroughColumns(scans[0], ["g"], 0)
+    join = SkinnerJoinOperator(js, scans, [Eq(ColRef(scans[0], "k", 0), ColRef(scans[1], "k", 1)),
+                                           Eq(ColRef(scans[1], "g", 1), ColRef(scans[2], "g", 2))])
+    aggs = [Count(), Sum(ColRef(join, "g"))]
+    out = OperatorSchema()
+    for i, name in enumerate(("n", "total")):
+        out.AddDerivedColumn(name, VirtColRef(aggs[i], i))
+    plan = OutputOperator(AggregateOperator(out, join, aggs))
+    o = Oracle()
+    for t in tables:
+        engine.register_table(t)
+        o.register_table(t)
+    assert compare(engine.execute(plan), o.execute(plan)) == ""
