@@ -3399,10 +3399,12 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       // and adds them to the table once at its end: a skewed key's rows would
       // otherwise queue on its record (3M rows of 200k Zipf keys: 1200 us
       // without the cache, 125 us with it; uniform keys 121 us; 1M rows of
-      // 100 keys 145 and 32 us).  A thread whose first 64 rows hit less than
-      // one time in eight (many keys, no skew) leaves the cache alone from
-      // then on.  Two blocks of 512 threads per SM: four of 256 flush twice
-      // the entries (137 us), three per SM spill registers (141 us).
+      // 100 keys 145 and 32 us).  Every row looks its key up: threads that left
+      // a cache with few hits alone gained nothing on 20M rows of 200k uniform
+      // keys (750 us either way), and a key that a tenth of the rows shared
+      // queued on its record (2500 against 680 us).  Two blocks of 512
+      // threads per SM: four of 256 flush twice the entries (137 us), three
+      // per SM spill registers (141 us).
       int entry = 16;  // bytes per cached key: key, first position, states
       for (const auto& p : plans) entry += (p.kind == StateKind::Count ? 0 : 8) + 4;
       const int C = entry <= 44 ? 1024 : (entry <= 88 ? 512 : 256);
@@ -3522,7 +3524,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             ks.L("bool ghit = false;");
             // cache places come from other hash bits than the table's
             ks.L("uint32_t gc = (uint32_t)(ghash >> 40) & " + std::to_string(C - 2) + "u;  // the first of a pair");
-            ks.Open(std::string("if (kdb_cache_on") + (wide ? " && gkey != 0" : "") + ")");
+            ks.Open(wide ? "if (gkey != 0)" : "");
             // two places per key: with one, a key that came first keeps a hot
             // one out of the whole block (240 against 121 us)
             ks.L("const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&kdb_ck[gc]);");
@@ -3535,10 +3537,13 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             ks.L("if (k == 0 || k == gkey) { ghit = true; gc += w; }");
             ks.Close();
             ks.Close();
-            ks.L("kdb_seen++; kdb_hits += ghit ? 1u : 0u;");
-            ks.L("if (kdb_seen == 64u && kdb_hits < 8u) kdb_cache_on = false;");
             ks.Close();
-            ks.Open("if (ghit)");
+            // (opaque: a compiler that knows which lanes hit at once sends them
+            // ahead, and the others no longer fold with them: 3M rows of 1000
+            // keys 127 us against 78)
+            ks.L("int gfold = ghit ? 1 : 0;");
+            ks.L("asm volatile(\"\" : \"+r\"(gfold));");
+            ks.Open("if (gfold)");
             fold_lanes("gc");
             ks.Open("if (gl)");
             for (size_t j = 0; j < plans.size(); j++) {
@@ -3610,7 +3615,6 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         }
         ks.Close();
       };
-      if (cache) ks.L("bool kdb_cache_on = true; unsigned kdb_seen = 0, kdb_hits = 0;");
       if (Streamable(op.child())) EmitStream(ks, eg, op.child(), consume, src_rows);
       else EmitMatScan(ks, mats_.at(&op.child()), nullptr, consume, src_rows);
       ks.globals << "#define KDB_R " << R << "\n";

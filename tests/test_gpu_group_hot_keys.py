@@ -1,0 +1,70 @@
+"""GROUP BY where one key holds many of the rows: the values, and that such a
+key costs no more than its rows would as other keys (its updates otherwise
+queue on one record, one row after the other)."""
+
+import numpy as np
+import pytest
+
+from kushdb_b200.data import HostColumn, HostTable, catalog_of
+from kushdb_b200.plan import (ColRef, ColRefE, Count, GroupByAggregateOperator, Min, OperatorSchema, OutputOperator,
+                              ScanOperator, Sum, Type, VirtColRef)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from kushdb_b200.engine import Engine
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def _plan(t):
+    s = OperatorSchema()
+    s.AddGeneratedColumns(catalog_of([t])[t.name], ["k", "v"])
+    src = ScanOperator(s, catalog_of([t])[t.name])
+    key = ColRefE(src, "k")
+    aggs = [Sum(ColRef(src, "v")), Min(ColRef(src, "v")), Count()]
+    o = OperatorSchema()
+    o.AddDerivedColumn("k", VirtColRef(key, 0))
+    for i, a in enumerate(aggs):
+        o.AddDerivedColumn(f"a{i}", VirtColRef(a, i + 1))
+    return OutputOperator(GroupByAggregateOperator(o, src, [key], aggs))
+
+
+def _run(engine, name, typ, keys):
+    """Checks the groups of `keys`; returns the GROUP BY kernel's time in us."""
+    v = (np.arange(len(keys)) * 37 % 1009 - 500).astype(np.int32)
+    t = HostTable(name)
+    t.add(HostColumn("k", typ, values=keys))
+    t.add(HostColumn("v", Type.Int(), values=v))
+    engine.register_table(t)
+    plan = _plan(t)
+    got = [np.asarray(c.values) for c in engine.execute(plan).columns]
+    uniq, first, member = np.unique(keys, return_index=True, return_inverse=True)
+    order = np.argsort(first)
+    low = np.full(len(uniq), 1 << 30, np.int64)
+    np.minimum.at(low, member, v)
+    want = [uniq, np.bincount(member, weights=v).astype(np.int64), low, np.bincount(member)]
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w[order])
+    engine.set_profiling(True)
+    us = []
+    for _ in range(5):
+        engine.execute(plan, fetch=False)
+        us.append(sum(k["ms"] for k in engine.last_kernels() if k["tag"] == "group by") * 1e3)
+    engine.set_profiling(False)
+    engine.drop_table(name)
+    return sorted(us)[2]
+
+
+# a row of a hot key costs at most what a row of any other key costs, and a
+# factor of two for the spread of the timings
+def test_hot_key_among_many_rows_per_thread(engine):
+    rows = 20_000_000  # over 64 rows for each thread of the GPU
+    rng = np.random.default_rng(1)
+    k = rng.integers(10, 50_000, rows).astype(np.int32)
+    spread = _run(engine, "hk_spread", Type.Int(), k)
+    k[rng.random(rows) < 0.1] = 7
+    assert _run(engine, "hk_hot", Type.Int(), k) < 2 * spread
