@@ -3394,7 +3394,6 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
           KL[k] = ks.Ptr(klen[k], "int32_t");
           KN[k] = ks.Ptr(kn[k], "int8_t");
         }
-      const std::string find_tail = std::string(", KDB_R, ") + M + ", ";
       // A block keeps the states of the keys it met first in shared memory
       // and adds them to the table once at its end: a skewed key's rows would
       // otherwise queue on its record (3M rows of 200k Zipf keys: 1200 us
@@ -3402,9 +3401,11 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       // 100 keys 145 and 32 us).  Every row looks its key up: threads that left
       // a cache with few hits alone gained nothing on 20M rows of 200k uniform
       // keys (750 us either way), and a key that a tenth of the rows shared
-      // queued on its record (2500 against 680 us).  Two blocks of 512
-      // threads per SM: four of 256 flush twice the entries (137 us), three
-      // per SM spill registers (141 us).
+      // queued on its record (2500 against 680 us).  BIGINT key 0, which marks
+      // an empty place, has an entry of its own behind the others (as half of
+      // 3M rows 4900 us without it, 190 with it).  Two blocks of 512 threads
+      // per SM: four of 256 flush twice the entries (137 us), three per SM
+      // spill registers (141 us).
       int entry = 16;  // bytes per cached key: key, first position, states
       for (const auto& p : plans) entry += (p.kind == StateKind::Count ? 0 : 8) + 4;
       const int C = entry <= 44 ? 1024 : (entry <= 88 ? 512 : 256);
@@ -3436,6 +3437,12 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         }
         const std::string f = "rec[" + g + " + " + std::to_string(fw) + "]";
         ks.L("atomicMax((unsigned long long*)&" + f + ", gf);");
+      };
+      // g, the record of `gkey` (-1: the table is full)
+      auto find_record = [&](const std::string& hash, bool zero) {
+        const std::string find = "kdb_group_find_rec(rec, KDB_R, " + M + ", gkey, " + hash + ", " + ERR + ")";
+        ks.L("const int64_t g = " + (zero ? "gkey == 0 ? (int64_t)(" + M + " + 1) * KDB_R : " : std::string()) + find + ";");
+        if (zero) ks.L("if (gkey == 0) rec[g] = 1ULL;  // occupied (a BIGINT key 0)");
       };
       // strings are compared in place: one update per row
       auto text_to_record = [&](const std::vector<CVal>& vals, const std::string& g) {
@@ -3521,10 +3528,11 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
           ks.L("const uint64_t gkey = " + pk + ";");
           ks.L("const uint64_t ghash = kdb_mix64(gkey);");
           if (cache) {
-            ks.L("bool ghit = false;");
+            ks.L(std::string("bool ghit = ") + (wide ? "gkey == 0;" : "false;"));
             // cache places come from other hash bits than the table's
             ks.L("uint32_t gc = (uint32_t)(ghash >> 40) & " + std::to_string(C - 2) + "u;  // the first of a pair");
-            ks.Open(wide ? "if (gkey != 0)" : "");
+            if (wide) ks.L("if (ghit) gc = " + CN + "u;");
+            ks.Open(wide ? "if (!ghit)" : "");
             // two places per key: with one, a key that came first keeps a hot
             // one out of the whole block (240 against 121 us)
             ks.L("const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&kdb_ck[gc]);");
@@ -3559,9 +3567,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             ks.Close();
             ks.Open("else");
           }
-          ks.L(std::string("const int64_t g = ") + (wide ? "gkey == 0 ? (int64_t)(" + M + " + 1) * KDB_R : " : "") +
-               "kdb_group_find_rec(rec" + find_tail + "gkey, ghash, " + ERR + ");");
-          if (wide) ks.L("if (gkey == 0) rec[g] = 1ULL;  // occupied (a BIGINT key 0)");
+          find_record("ghash", wide && !cache);
           ks.Open("if (g >= 0)");
           text_to_record(vals, "g");
           to_record("g");
@@ -3623,23 +3629,24 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       ks.args[w_rec] = reinterpret_cast<uint64_t>(rec);
       if (cache) {
         std::ostringstream& pre = ks.pre;
-        pre << "  __shared__ __align__(16) unsigned long long kdb_ck[" << C << "], kdb_cf[" << C << "];\n";
+        const int entries = wide ? C + 1 : C;
+        pre << "  __shared__ __align__(16) unsigned long long kdb_ck[" << entries << "], kdb_cf[" << entries << "];\n";
         std::string zero = "kdb_ck[i] = 0; kdb_cf[i] = 0;";
         for (size_t j = 0; j < plans.size(); j++) {
           if (plans[j].kind != StateKind::Count) {
-            pre << "  __shared__ " << (is_float(j) ? "double" : "unsigned long long") << " kdb_cv" << j << "[" << C << "];\n";
+            pre << "  __shared__ " << (is_float(j) ? "double" : "unsigned long long") << " kdb_cv" << j << "[" << entries << "];\n";
             zero += " kdb_cv" + std::to_string(j) + "[i] = 0;";
           }
-          pre << "  __shared__ unsigned kdb_cn" << j << "[" << C << "];\n";
+          pre << "  __shared__ unsigned kdb_cn" << j << "[" << entries << "];\n";
           zero += " kdb_cn" + std::to_string(j) + "[i] = 0;";
         }
-        pre << "  for (int i = threadIdx.x; i < " << C << "; i += blockDim.x) { " << zero << " }\n  __syncthreads();\n";
+        pre << "  for (int i = threadIdx.x; i < " << entries << "; i += blockDim.x) { " << zero << " }\n  __syncthreads();\n";
         // the cached keys' states into the table
         ks.L("__syncthreads();");
-        ks.Open("for (int i = threadIdx.x; i < " + CN + "; i += blockDim.x)");
+        ks.Open("for (int i = threadIdx.x; i < " + std::to_string(entries) + "; i += blockDim.x)");
+        ks.L("if (kdb_cf[i] == 0) continue;");
         ks.L("const uint64_t gkey = kdb_ck[i];");
-        ks.L("if (gkey == 0) continue;");
-        ks.L("const int64_t g = kdb_group_find_rec(rec" + find_tail + "gkey, kdb_mix64(gkey), " + ERR + ");");
+        find_record("kdb_mix64(gkey)", wide);
         ks.L("if (g < 0) continue;");
         for (size_t j = 0; j < plans.size(); j++) {
           ks.L("const unsigned " + N(j) + " = kdb_cn" + std::to_string(j) + "[i];");

@@ -68,3 +68,14 @@ def test_hot_key_among_many_rows_per_thread(engine):
     spread = _run(engine, "hk_spread", Type.Int(), k)
     k[rng.random(rows) < 0.1] = 7
     assert _run(engine, "hk_hot", Type.Int(), k) < 2 * spread
+
+
+def test_bigint_zero_is_as_cheap_as_another_hot_key(engine):
+    rows = 3_000_017
+    rng = np.random.default_rng(2)
+    k = rng.integers(10, 200_000, rows)
+    hot = rng.random(rows) < 0.5
+    k[hot] = 7
+    other = _run(engine, "hk_seven", Type.BigInt(), k)
+    k[hot] = 0
+    assert _run(engine, "hk_zero", Type.BigInt(), k) < 2 * other
