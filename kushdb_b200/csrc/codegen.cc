@@ -3386,6 +3386,7 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       ks.pre << "  uint64_t* __restrict__ rec = (uint64_t*)a.w[" << w_rec << "];\n";
       std::string S = keyed ? "" : ks.Ptr(slots, "uint64_t");
       std::string M = "(uint64_t)" + ks.Word(mask);
+      if (keyed) ks.pre << "  const bool in_l2 = " << M << " * (8 * KDB_R) < (96ULL << 20);\n";
       std::string ERR = ks.Ptr(ctx_.d_err, "int");
       std::vector<std::string> KW(nk), KL(nk), KN(nk);
       if (!keyed)
@@ -3418,10 +3419,17 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
       auto V = [](size_t j) { return "gv" + std::to_string(j); };
       auto N = [](size_t j) { return "gn" + std::to_string(j); };
       // adds values gv*, counts gn*, position gf to the record at `g`; every
-      // update is one reduction without a result (reading a minimum first,
-      // to skip those that do not improve it, waits for each read: 185
-      // against 118 us over 3M rows of 200k uniform keys)
-      auto to_record = [&](const std::string& g) {
+      // update is one reduction without a result.  Values that the record's
+      // first position and extremes have had (gs*) come with the key, and most
+      // rows improve none of them (20M rows of 200k uniform keys 573 us, 750
+      // with every reduction; reading them after the key was found waits for
+      // each: 185 against 118 us at 3M rows).  The extremes are left out where
+      // the records outgrow L2 (96 of its 126 MB): their reads then go to
+      // HBM, and a group has fewer rows (20M rows of 2M keys 1490 against
+      // 1150 us).
+      auto seen_word = [&](size_t j) { return plans[j].kind == StateKind::MinMaxKey; };
+      enum Seen { kSeenNothing, kSeenFirst, kSeenAll };
+      auto to_record = [&](const std::string& g, Seen seen = kSeenNothing) {
         for (size_t j = 0; j < plans.size(); j++) {
           const std::string w = "rec[" + g + " + " + std::to_string(vw[j]) + "]";
           if (is_float(j)) {
@@ -3429,18 +3437,27 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
           } else if (plans[j].kind == StateKind::SumI64) {
             ks.L("if (" + N(j) + ") atomicAdd((unsigned long long*)&" + w + ", " + V(j) + ");");
           } else if (plans[j].kind == StateKind::MinMaxKey) {
-            ks.L("if (" + N(j) + ") atomicMax((unsigned long long*)&" + w + ", " + V(j) + ");");
+            ks.L("if (" + N(j) + (seen == kSeenAll && seen_word(j) ? " && " + V(j) + " > gs" + std::to_string(j) : "") +
+                 ") atomicMax((unsigned long long*)&" + w + ", " + V(j) + ");");
           }
           if (cw[j] >= 0)
             ks.L("if (" + N(j) + ") atomicAdd((unsigned long long*)&rec[" + g + " + " + std::to_string(cw[j]) +
                  "], (unsigned long long)" + N(j) + ");");
         }
         const std::string f = "rec[" + g + " + " + std::to_string(fw) + "]";
-        ks.L("atomicMax((unsigned long long*)&" + f + ", gf);");
+        ks.L(std::string(seen != kSeenNothing ? "if (gf > gsf) " : "") + "atomicMax((unsigned long long*)&" + f + ", gf);");
       };
-      // g, the record of `gkey` (-1: the table is full)
-      auto find_record = [&](const std::string& hash, bool zero) {
-        const std::string find = "kdb_group_find_rec(rec, KDB_R, " + M + ", gkey, " + hash + ", " + ERR + ")";
+      // g, the record of `gkey` (-1: the table is full), and gs*
+      auto find_record = [&](const std::string& hash, bool zero, Seen seen) {
+        std::string read = "gsf = __ldcg(p + " + std::to_string(fw) + ");";
+        ks.L("unsigned long long gsf = 0;");
+        for (size_t j = 0; j < plans.size(); j++)
+          if (seen == kSeenAll && seen_word(j)) {
+            ks.L("unsigned long long gs" + std::to_string(j) + " = 0;");
+            read += " gs" + std::to_string(j) + " = __ldcg(p + " + std::to_string(vw[j]) + ");";
+          }
+        const std::string find = "kdb_group_find_rec(rec, KDB_R, " + M + ", gkey, " + hash +
+                                 ", [&](const unsigned long long* p) { " + read + " }, " + ERR + ")";
         ks.L("const int64_t g = " + (zero ? "gkey == 0 ? (int64_t)(" + M + " + 1) * KDB_R : " : std::string()) + find + ";");
         if (zero) ks.L("if (gkey == 0) rec[g] = 1ULL;  // occupied (a BIGINT key 0)");
       };
@@ -3567,11 +3584,18 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             ks.Close();
             ks.Open("else");
           }
-          find_record("ghash", wide && !cache);
-          ks.Open("if (g >= 0)");
-          text_to_record(vals, "g");
-          to_record("g");
-          ks.Close();
+          bool extremes = false;
+          for (size_t j = 0; j < plans.size(); j++) extremes |= seen_word(j);
+          for (const Seen seen : {kSeenAll, kSeenFirst}) {
+            if (seen == kSeenAll && !extremes) continue;
+            ks.Open(!extremes ? "" : seen == kSeenAll ? "if (in_l2)" : "else");
+            find_record("ghash", wide && !cache, seen);
+            ks.Open("if (g >= 0)");
+            text_to_record(vals, "g");
+            to_record("g", seen);
+            ks.Close();
+            ks.Close();
+          }
           if (cache) ks.Close();
         } else {
           std::string h = "0x2545f4914f6cdd1dULL";
@@ -3646,14 +3670,14 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         ks.Open("for (int i = threadIdx.x; i < " + std::to_string(entries) + "; i += blockDim.x)");
         ks.L("if (kdb_cf[i] == 0) continue;");
         ks.L("const uint64_t gkey = kdb_ck[i];");
-        find_record("kdb_mix64(gkey)", wide);
+        find_record("kdb_mix64(gkey)", wide, kSeenFirst);
         ks.L("if (g < 0) continue;");
         for (size_t j = 0; j < plans.size(); j++) {
           ks.L("const unsigned " + N(j) + " = kdb_cn" + std::to_string(j) + "[i];");
           if (plans[j].kind != StateKind::Count) ks.L("const auto " + V(j) + " = kdb_cv" + std::to_string(j) + "[i];");
         }
         ks.L("const unsigned long long gf = kdb_cf[i];");
-        to_record("g");
+        to_record("g", kSeenFirst);
         ks.Close();
         // few, large blocks: every block flushes its cache at the end
         const int block = 512;

@@ -503,12 +503,16 @@ KDB_DEV void kdb_join_insert(uint64_t* slots, uint64_t mask, uint32_t h, uint32_
 
 // The table is an array of records of `stride` words whose first word is the
 // key (0: empty; the record's other words start as zeros); returns the word
-// offset of the key's record.
-KDB_DEV int64_t kdb_group_find_rec(uint64_t* rec, int stride, uint64_t mask, uint64_t key, uint64_t hash, int* err) {
+// offset of the key's record.  read(p) loads what the caller wants to know of
+// a record while its key is on the way; the last call is for the key's own.
+template <typename READ>
+KDB_DEV int64_t kdb_group_find_rec(uint64_t* rec, int stride, uint64_t mask, uint64_t key, uint64_t hash, READ read,
+                                   int* err) {
   uint64_t i = hash & mask;
   for (uint64_t k = 0; k <= mask && k < KDB_MAX_PROBE; k++) {
     unsigned long long* p = (unsigned long long*)(rec + i * stride);
     unsigned long long s = __ldcg(p);
+    read(p);
     if (s == 0) s = atomicCAS(p, 0ULL, (unsigned long long)key);
     if (s == 0 || s == key) return (int64_t)(i * stride);
     i = (i + 1) & mask;
