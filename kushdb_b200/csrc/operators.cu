@@ -45,7 +45,8 @@ namespace ops {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kBuildBlock = 512;                 // threads of a partitioned build CTA
+constexpr int kBuildBlock = 512;                 // threads of a partitioned build CTA, with others on its SM
+constexpr int kBuildAlone = 1024;                // and where its shared memory leaves room for no other
 constexpr int kPartBlock = 1024;                 // threads of a partitioning CTA
 constexpr int kMaxPartBits = 13;                 // at most 8192 sub-tables
 constexpr size_t kSmemTableMax = 128 << 10;      // a sub-table built in shared memory
@@ -192,6 +193,14 @@ __device__ __forceinline__ bool BarWaitAll(uint64_t* bar, uint32_t parity, int* 
 // partition's places for the whole chunk with one atomic and then takes them
 // through shared-memory cursors.  (One returning global atomic per row: 262
 // against 71 us for 6M rows in 4096 partitions.)
+//
+// Every CTA then has a sector of its own open in every partition for as long
+// as the kernel runs.  Once the staged tuples outgrow L2 those sectors are
+// written back half full and read again, so the second pass takes its places
+// row by row from global cursors instead (PartScatterRows): the CTAs fill a
+// partition's sectors together, one after the other.  By chunks and by rows,
+// INT keys: 11M rows 179 and 313 us, 15M 328 and 314, 30M 918 and 626, 60M
+// 2170 and 1400; BIGINT: 5M 114 and 149, 7M 187 and 154, 30M 1170 and 731.
 __global__ void __launch_bounds__(kPartBlock) PartHistogram(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
                                                             int64_t chunk, int bits, unsigned* __restrict__ hist,
                                                             unsigned* __restrict__ block_hist) {
@@ -207,10 +216,10 @@ __global__ void __launch_bounds__(kPartBlock) PartHistogram(KeyCol key, const in
     atomicAdd(&sh_hist[PartOf(Hash32(static_cast<uint64_t>(LoadKey(key, r))), bits)], 1u);
   }
   __syncthreads();
-  unsigned* mine = block_hist + static_cast<int64_t>(blockIdx.x) * parts;
+  unsigned* mine = block_hist ? block_hist + static_cast<int64_t>(blockIdx.x) * parts : nullptr;
   for (int i = threadIdx.x; i < parts; i += blockDim.x) {
     const unsigned c = sh_hist[i];
-    mine[i] = c;
+    if (mine) mine[i] = c;
     if (c) atomicAdd(&hist[i], c);
   }
 }
@@ -296,6 +305,23 @@ __global__ void __launch_bounds__(kPartBlock) PartScatter(KeyCol key, const int3
   }
 }
 
+// The same with a global cursor per partition (starting at 0).
+template <bool WIDE>
+__global__ void __launch_bounds__(kBlock) PartScatterRows(KeyCol key, const int32_t* __restrict__ sel, int64_t n,
+                                                          int bits, const unsigned long long* __restrict__ stage_off,
+                                                          unsigned* __restrict__ cursor,
+                                                          typename Slot<WIDE>::T* __restrict__ staged) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = RowAt(sel, i);
+    if (KeyNull(key, r)) continue;
+    const int64_t k = LoadKey(key, r);
+    const uint32_t p = PartOf(Hash32(static_cast<uint64_t>(k)), bits);
+    const unsigned at = atomicAdd(&cursor[p], 1u);
+    staged[stage_off[p] + at] = Slot<WIDE>::Make(k, r);
+  }
+}
+
 // ---- build -------------------------------------------------------------------
 // Inserts into table `tab` of capacity `cap` (a power of two) at the hash's
 // low bits, linear probing; returns 0, kDupKey when the walk passed a slot
@@ -349,13 +375,14 @@ __global__ void BuildFlat(KeyCol key, const int32_t* __restrict__ sel, int64_t n
 // partition is clear, wait, insert and write out, one after the other): 6M
 // rows in 4096 sub-tables of 32 KB took 148 us with one CTA of 1024 threads
 // and 128 KB for the table per SM, and take 83 with three of 512 (87 with 256
-// threads, 144 with 1024).  A partition's staged tuples come
+// threads, 144 with 1024); where a sub-table leaves room for one CTA only,
+// that one has 1024 (30M BIGINT keys 697 us, 758 with 512).  A partition's staged tuples come
 // into shared memory in bulk-copied tiles through a two-buffer ring that
 // runs one tile ahead, across partition boundaries too; a sub-table that
 // fits shared memory is built there with shared-memory CAS and written out
 // with coalesced stores, a larger one is built in place in HBM.
 template <bool WIDE>
-__global__ void __launch_bounds__(kBuildBlock) BuildParts(const typename Slot<WIDE>::T* __restrict__ staged,
+__global__ void __launch_bounds__(kBuildAlone) BuildParts(const typename Slot<WIDE>::T* __restrict__ staged,
                                                      const unsigned long long* __restrict__ stage_off,
                                                      const unsigned* __restrict__ hist,
                                                      const unsigned long long* __restrict__ slot_off, int parts,
@@ -700,9 +727,23 @@ void* PoolAlloc(Context& c, size_t bytes) {
   return p;
 }
 
+// Staged tuples of this many bytes are scattered by chunks: most of L2.
+constexpr int64_t kChunkedBytes = int64_t(96) << 20;
+
+// block_hist: of PartHistogram with the same grid and chunk, or null (by rows)
 void LaunchScatter(Context& c, bool wide, int grid, const KeyCol& key, const int32_t* sel, int64_t n, int64_t chunk,
                    int bits, const unsigned* block_hist, const unsigned long long* stage_off, unsigned* cursor,
                    void* staged) {
+  if (!block_hist) {
+    const int rgrid = c.GridFor(n, kBlock);
+    if (wide)
+      PartScatterRows<true><<<rgrid, kBlock, 0, c.stream>>>(key, sel, n, bits, stage_off, cursor,
+                                                            static_cast<ulonglong2*>(staged));
+    else
+      PartScatterRows<false><<<rgrid, kBlock, 0, c.stream>>>(key, sel, n, bits, stage_off, cursor,
+                                                             static_cast<unsigned long long*>(staged));
+    return;
+  }
   const int smem = static_cast<int>(sizeof(unsigned)) << bits;  // 32 KB at most
   if (wide) {
     PartScatter<true><<<grid, kPartBlock, smem, c.stream>>>(key, sel, n, chunk, bits, block_hist, stage_off, cursor,
@@ -919,7 +960,8 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
     c.Memset(hist, 0, sizeof(unsigned) * parts);
     const int cgrid = PartGrid(c, n);
     const int64_t chunk = (n + cgrid - 1) / cgrid;
-    unsigned* block_hist = arena.AllocT<unsigned>(static_cast<size_t>(cgrid) * parts);
+    const bool chunked = n * slot_bytes <= kChunkedBytes;
+    unsigned* block_hist = chunked ? arena.AllocT<unsigned>(static_cast<size_t>(cgrid) * parts) : nullptr;
     c.TimedStart("hash partition");
     PartHistogram<<<cgrid, kPartBlock, sizeof(unsigned) * parts, c.stream>>>(key, srows, n, chunk, ht->bits, hist,
                                                                             block_hist);
@@ -943,14 +985,16 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
     while (tab_slots < (rows + 4 * std::sqrt(rows)) / load_factor + 1) tab_slots <<= 1;
     const uint32_t tab_bytes = static_cast<uint32_t>(std::min<size_t>(tab_slots * slot_bytes, kSmemTableMax));
     const size_t smem = 2 * kBuildTile * slot_bytes + tab_bytes;
-    const int pgrid = std::min<int>(parts, c.num_sms * static_cast<int>(std::min<size_t>(4, (220u << 10) / (smem + 1024))));
+    const int per_sm = static_cast<int>(std::min<size_t>(4, (220u << 10) / (smem + 1024)));
+    const int pgrid = std::min<int>(parts, c.num_sms * per_sm);
+    const int bblock = per_sm == 1 ? kBuildAlone : kBuildBlock;
     if (ht->wide) {
       KDB_CUDA(cudaFuncSetAttribute(BuildParts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      BuildParts<true><<<pgrid, kBuildBlock, smem, c.stream>>>(static_cast<const ulonglong2*>(staged), stage_off, hist,
+      BuildParts<true><<<pgrid, bblock, smem, c.stream>>>(static_cast<const ulonglong2*>(staged), stage_off, hist,
                                                           ht->slot_off, parts, static_cast<ulonglong2*>(ht->slots), tab_bytes, err);
     } else {
       KDB_CUDA(cudaFuncSetAttribute(BuildParts<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      BuildParts<false><<<pgrid, kBuildBlock, smem, c.stream>>>(static_cast<const unsigned long long*>(staged), stage_off,
+      BuildParts<false><<<pgrid, bblock, smem, c.stream>>>(static_cast<const unsigned long long*>(staged), stage_off,
                                                            hist, ht->slot_off, parts,
                                                            static_cast<unsigned long long*>(ht->slots), tab_bytes, err);
     }

@@ -456,3 +456,31 @@ def test_unordered_unique_probe_on_both_sides_of_the_match_rows_size(engine):
         np.testing.assert_array_equal(np.asarray(got_p)[order], hit)
         np.testing.assert_array_equal(np.asarray(got_b)[order], inv[pk[hit]])
     ht.close()
+
+
+# staged tuples on both sides of 96 MiB (by chunks, by rows), and sub-tables
+# that leave room for one CTA per SM (BIGINT, 8M rows)
+@pytest.mark.parametrize("tname,nb", [("INT", 12_582_912), ("INT", 12_582_913), ("BIGINT", 6_291_456),
+                                      ("BIGINT", 6_291_457), ("BIGINT", 8_000_001)])
+def test_hash_build_scatters_around_l2(engine, tname, nb):
+    rng = np.random.default_rng(nb)
+    keys = rng.permutation(nb)
+    nulls = np.zeros(nb, np.int8)
+    nulls[rng.integers(0, nb, 1000)] = 1
+    dtype = np.int32 if tname == "INT" else np.int64
+    t = _key_table(f"hbs_{tname}_{nb}", keys.astype(dtype), nulls, dtype, tname)
+    pk = rng.integers(-50, nb + 50, 200_003)
+    p = _key_table(f"hbsp_{tname}_{nb}", pk.astype(dtype), None, dtype, tname)
+    for x in (t, p):
+        engine.register_table(x)
+    from kushdb_b200.operators import HashTable
+    h = HashTable(engine, t.name, "k")
+    probe, build = h.probe(p.name, "k")
+    h.close()
+    row_of = np.full(nb + 100, -1, np.int64)
+    row_of[keys + 50] = np.where(nulls != 0, -1, np.arange(nb))
+    want = row_of[pk + 50]
+    hit = want >= 0
+    assert np.array_equal(probe, np.nonzero(hit)[0]) and np.array_equal(build, want[hit])
+    for x in (t, p):
+        engine.drop_table(x.name)
