@@ -3898,14 +3898,12 @@ MatBuffer Executor::SmallOrderBy(const Operator& op, MatBuffer& m) {
     };
     {
       KernelSource ks;
-      const std::string P = ks.Ptr(m.pos, "uint64_t", true), T = ks.Ptr(ties, "uint32_t"),
-                        I = ks.Ptr(idx, "uint32_t");
+      const std::string P = ks.Ptr(m.pos, "uint64_t", true), T = ks.Ptr(ties, "uint32_t");
       row_per_warp(ks);
       ks.L("const uint64_t p = " + P + "[i];");
       ks.L("for (int64_t j = lane; j < nrows; j += 32) r += " + P + "[j] < p;");
       ks.L("r = __reduce_add_sync(0xffffffffu, r);");
-      // (every place holds a row even if NaN keys leave some unranked)
-      ks.L("if (lane == 0) { " + T + "[i] = (uint32_t)(kdb_tie_path(r, nrows) >> 32); " + I + "[i] = (uint32_t)i; }");
+      ks.L("if (lane == 0) " + T + "[i] = (uint32_t)(kdb_tie_path(r, nrows) >> 32);");
       const std::string name = KernelName("order by small rows");
       ctx_.Launch(ctx_.Kernel(ks.Kernel(name, 256), name), grid, 256, ks.Args(), 0, "order by small rows");
     }
@@ -3933,6 +3931,12 @@ MatBuffer Executor::SmallOrderBy(const Operator& op, MatBuffer& m) {
         case TypeId::ENUM:
           ab = "(" + eg.EnumRank(mc.type, D + "[ra]") + " < " + eg.EnumRank(mc.type, D + "[rb]") + ")";
           ba = "(" + eg.EnumRank(mc.type, D + "[rb]") + " < " + eg.EnumRank(mc.type, D + "[ra]") + ")";
+          break;
+        case TypeId::REAL:
+          // (as in the sorts of more rows, NaN has a place: by `<` it would
+          // have none, and two rows could rank alike)
+          ab = "kdb_real_less(" + D + "[ra], " + D + "[rb])";
+          ba = "kdb_real_less(" + D + "[rb], " + D + "[ra])";
           break;
         default:
           ab = "(" + D + "[ra] < " + D + "[rb])";
@@ -4068,7 +4072,7 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
              ";");
         std::string v = D + "[row]", norm;
         switch (t) {
-          case TypeId::REAL: norm = "kdb_dord(" + v + ")"; break;
+          case TypeId::REAL: norm = "kdb_real_key(" + v + ")"; break;
           case TypeId::ENUM: norm = "(uint64_t)(uint32_t)" + eg.EnumRank(mc.type, v); break;
           default: norm = "((uint64_t)(int64_t)" + v + " ^ 0x8000000000000000ULL)"; break;
         }
@@ -4210,7 +4214,7 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
             std::string v = load(ks, eg, I).first;
             std::string norm;
             switch (mc.type.id) {
-              case TypeId::REAL: norm = "kdb_dord(" + v + ")"; break;
+              case TypeId::REAL: norm = "kdb_real_key(" + v + ")"; break;
               case TypeId::ENUM: norm = "(uint64_t)(uint32_t)" + eg.EnumRank(mc.type, v); break;
               default: norm = "((uint64_t)(int64_t)" + v + " ^ 0x8000000000000000ULL)"; break;
             }
@@ -4265,10 +4269,10 @@ MatBuffer Executor::LargeOrderBy(const Operator& op, MatBuffer& m) {
           std::string D = ks.Ptr(mc.data, "double", true);
           if (mc.nullable) {
             std::string NP = ks.Ptr(mc.nulls, "int8_t", true);
-            ks.L("{ const bool na = " + NP + "[ra] != 0, nb = " + NP + "[rb] != 0; eq = eq && na == nb && (na || kdb_dord(" +
-                 D + "[ra]) == kdb_dord(" + D + "[rb])); }");
+            ks.L("{ const bool na = " + NP + "[ra] != 0, nb = " + NP + "[rb] != 0; eq = eq && na == nb && (na || kdb_real_key(" +
+                 D + "[ra]) == kdb_real_key(" + D + "[rb])); }");
           } else {
-            ks.L("eq = eq && kdb_dord(" + D + "[ra]) == kdb_dord(" + D + "[rb]);");
+            ks.L("eq = eq && kdb_real_key(" + D + "[ra]) == kdb_real_key(" + D + "[rb]);");
           }
         }
         ks.L("if (eq) atomicAdd(" + T + ", 1ULL);");

@@ -371,13 +371,26 @@ KDB_DEV uint64_t kdb_dbits(double d) {
 }
 
 // Order-preserving double <-> uint64 (for atomicMin/Max and radix keys).
+// (One xor with a mask: given `b | sign` of a double's bits the compiler may
+// negate the double, which does not keep the sign of a NaN.)
 KDB_DEV uint64_t kdb_dord(double d) {
-  uint64_t b = (uint64_t)__double_as_longlong(d);
-  return (b & 0x8000000000000000ULL) ? ~b : (b | 0x8000000000000000ULL);
+  const int64_t b = __double_as_longlong(d);
+  return (uint64_t)(b ^ ((b >> 63) | (int64_t)0x8000000000000000ULL));
 }
 KDB_DEV double kdb_dord_inv(uint64_t k) {
   uint64_t b = (k & 0x8000000000000000ULL) ? (k & 0x7fffffffffffffffULL) : ~k;
   return __longlong_as_double((long long)b);
+}
+
+// A REAL sort key: ordered like the numbers, -0.0 equal to 0.0, and NaN before
+// or after all of them by its sign.
+KDB_DEV uint64_t kdb_real_key(double d) {
+  const uint64_t b = (uint64_t)__double_as_longlong(d);
+  return b + b == 0 ? 0x8000000000000000ULL : kdb_dord(d);
+}
+// The same order (a NaN's bits are looked at only where there is one).
+KDB_DEV bool kdb_real_less(double a, double b) {
+  return a < b || ((a != a || b != b) && kdb_real_key(a) < kdb_real_key(b));
 }
 
 // ---- warp-aggregated slot allocation --------------------------------------
