@@ -23,6 +23,7 @@
 #include <limits>
 #include <list>
 #include <map>
+#include <numeric>
 #include <random>
 #include <set>
 #include <sstream>
@@ -4674,14 +4675,15 @@ class SkinnerEngine : public JoinEnv {
     } else {
       out_ = alloc_out_(1 << 12);
     }
-    // result count, a spare word, the two task queues' counts, then per episode of
-    // a batch its results and its work (all read back together)
-    stats_ = arena_.AllocT<uint64_t>(4 + 2 * kMaxBatch);
-    ctx_.Memset(stats_, 0, (4 + 2 * kMaxBatch) * sizeof(uint64_t));
+    // result count, a spare word, the two task queues' counts (short and long
+    // tasks of each), then per episode of a batch its results and its work
+    // (all read back together)
+    stats_ = arena_.AllocT<uint64_t>(6 + 2 * kMaxBatch);
+    ctx_.Memset(stats_, 0, (6 + 2 * kMaxBatch) * sizeof(uint64_t));
     count_ = stats_;
     tcount_ = stats_ + 2;
-    eres_ = stats_ + 4;
-    ework_ = stats_ + 4 + kMaxBatch;
+    eres_ = stats_ + 6;
+    ework_ = stats_ + 6 + kMaxBatch;
     ep_ = arena_.AllocT<uint64_t>(static_cast<size_t>(kMaxBatch) * EpWords());
     // episodes per batch: the next join orders are chosen before the
     // current ones' rewards are known (their placeholders corrected after),
@@ -4700,8 +4702,12 @@ class SkinnerEngine : public JoinEnv {
         beg2_ = arena_.AllocT<uint64_t>(kMaxItems2);
         offs2_ = arena_.AllocT<uint64_t>(kMaxItems2 + 1);
       }
-      split_ = T_ > 2 && !ctx_.OptStr("KDB_SKINNER_NO_SPLIT");
       if (const char* r = ctx_.OptStr("KDB_SKINNER_SPLIT")) split_run_ = std::max<int64_t>(1, std::atoll(r));
+      const int64_t most = *std::max_element(cards_.begin(), cards_.end());
+      split_ = T_ > 3 && most > split_run_ && !ctx_.OptStr("KDB_SKINNER_NO_SPLIT");
+      const int64_t all_rows = std::accumulate(cards_.begin(), cards_.end(), int64_t(0));
+      task_cap_ = kMinTasks;
+      while (task_cap_ < kMaxTasks && task_cap_ < all_rows) task_cap_ <<= 1;
       if (const char* c = ctx_.OptStr("KDB_SKINNER_TASKS")) task_cap_ = std::max<int64_t>(1, std::atoll(c));
       if (split_)
         for (int q = 0; q < 2; q++) tasks_[q] = arena_.AllocT<uint64_t>(task_cap_ * (4 + T_));
@@ -4878,7 +4884,7 @@ class SkinnerEngine : public JoinEnv {
     a.w[w_nep_] = static_cast<uint64_t>(nb);
     a.w[w_total_] = static_cast<uint64_t>(S);
     const int K = kMaxBatch;
-    std::vector<uint64_t> st(4 + 2 * K, 0);
+    std::vector<uint64_t> st(6 + 2 * K, 0);
     for (int attempt = 0; attempt < 8; attempt++) {
       a.w[w_cap_] = static_cast<uint64_t>(out_.cap);
       PatchOut(a);
@@ -4901,20 +4907,18 @@ class SkinnerEngine : public JoinEnv {
         }
       }
       ctx_.ReadWordsChecked(st.data(), stats_, st.size(), "skinner episode");
-      if (split_ && st[2] > 0 && !ctx_.dry) {
+      if (split_ && st[2] + st[3] > 0 && !ctx_.dry) {
         // queued hot runs: each round's tasks sit one position deeper than
         // the previous round's, so at most T rounds
         int qi = 0;
-        uint64_t pending = st[2];
-        for (int round = 0; pending > 0; round++) {
+        for (int round = 0; st[2 + 2 * qi] + st[3 + 2 * qi] > 0; round++) {
           if (round > T_) throw Error(-5, "skinner task rounds did not converge");
           a.w[w_phase_] = 4;
           a.w[w_qin_] = static_cast<uint64_t>(qi);
           ctx_.Launch(fn_, ctx_.num_sms * 8, 128, a, 0, "skinner tasks");
-          ctx_.Memset(tcount_ + qi, 0, sizeof(uint64_t));
+          ctx_.Memset(tcount_ + 2 * qi, 0, 2 * sizeof(uint64_t));
           qi = 1 - qi;
           ctx_.ReadWordsChecked(st.data(), stats_, st.size(), "skinner episode");
-          pending = st[2 + qi];
         }
       }
       int64_t total = static_cast<int64_t>(st[0]);
@@ -4935,8 +4939,8 @@ class SkinnerEngine : public JoinEnv {
     for (int e = 0; e < nb; e++) {
       const Pending& pe = pending_[e];
       const int64_t len = pe.s1 - pe.s0;
-      const int64_t results = static_cast<int64_t>(st[4 + e]);
-      const int64_t work = static_cast<int64_t>(st[4 + K + e]);
+      const int64_t results = static_cast<int64_t>(st[6 + e]);
+      const int64_t work = static_cast<int64_t>(st[6 + K + e]);
       lwork[pe.L] += work;
       llen[pe.L] += len;
       const double progress = static_cast<double>(len) / static_cast<double>(pe.remaining);
@@ -5185,7 +5189,7 @@ class SkinnerEngine : public JoinEnv {
     // positions bound) as tasks of split_run_ candidates on queue q; false
     // when the queue is full (the caller walks the run itself; the slots it
     // reserved past the capacity that are in range hold empty tasks)
-    std::string TQ0, TQ1, TC, RUN, TCAP;
+    std::string TQ0, TQ1, TC, RUN, TCAP, LONG, SHORTS;
     const std::string TW = std::to_string(4 + T);  // position, begin, end, rows, episode
     if (split_) {
       TQ0 = ks.Ptr(tasks_[0], "uint64_t");
@@ -5193,22 +5197,33 @@ class SkinnerEngine : public JoinEnv {
       TC = ks.Ptr(tcount_, "unsigned long long");
       RUN = "(int64_t)" + ks.Word(static_cast<uint64_t>(split_run_));
       TCAP = "(uint64_t)" + ks.Word(static_cast<uint64_t>(task_cap_));
+      SHORTS = "(uint64_t)" + ks.Word(static_cast<uint64_t>(task_cap_ / 2));
+      LONG = "(int64_t)" + ks.Word(static_cast<uint64_t>(std::max(kLongRun, split_run_)));
       ks.Open("auto push = [&](int p, int q) -> bool");
       ks.L("const int64_t len = ite[p] - iti[p];");
-      ks.L("const uint64_t n = (uint64_t)((len + " + RUN + " - 1) / " + RUN + ");");
-      ks.L("const uint64_t base = atomicAdd(&" + TC + "[q], (unsigned long long)n);");
+      // short tasks while their part of the queue lasts, then long ones
+      ks.Open("for (int part = 0; part < 2; part++)");
+      ks.L("const int64_t run = part ? " + LONG + " : " + RUN + ";");
+      ks.L("if (len <= run) return false;");
+      ks.L("const uint64_t first = part ? " + SHORTS + " : 0, cap = part ? " + TCAP + " : " + SHORTS + ";");
+      ks.L("unsigned long long* count = &" + TC + "[2 * q + part];");
+      ks.L("if (first + *(volatile unsigned long long*)count >= cap) continue;");
+      ks.L("const uint64_t n = (uint64_t)((len + run - 1) / run);");
+      ks.L("const uint64_t base = first + atomicAdd(count, (unsigned long long)n);");
       ks.L("uint64_t* tq = q ? " + TQ1 + " : " + TQ0 + ";");
-      ks.L("const bool ok = base + n <= " + TCAP + ";");
-      ks.L("const uint64_t lim = ok ? base + n : (base < " + TCAP + " ? " + TCAP + " : base);");
+      ks.L("const bool ok = base + n <= cap;");
+      ks.L("const uint64_t lim = ok ? base + n : cap;");
       ks.Open("for (uint64_t i = base; i < lim; i++)");
       ks.L("uint64_t* t = tq + i * " + TW + ";");
-      ks.L("const int64_t b = ok ? iti[p] + (int64_t)(i - base) * " + RUN + " : 0;");
-      ks.L("const int64_t e = ok ? (b + " + RUN + " < ite[p] ? b + " + RUN + " : ite[p]) : 0;");
+      ks.L("const int64_t b = ok ? iti[p] + (int64_t)(i - base) * run : 0;");
+      ks.L("const int64_t e = ok ? (b + run < ite[p] ? b + run : ite[p]) : 0;");
       ks.L("t[0] = (uint64_t)p; t[1] = (uint64_t)b; t[2] = (uint64_t)e;");
       ks.L("for (int k = 0; k < " + TS + "; k++) t[3 + k] = (uint64_t)rows[k];");
       ks.L("t[3 + " + TS + "] = (uint64_t)cur_e;");
       ks.Close();
-      ks.L("return ok;");
+      ks.L("if (ok) return true;");
+      ks.Close();
+      ks.L("return false;");
       ks.indent--;
       ks.L("};");
     }
@@ -5367,13 +5382,14 @@ class SkinnerEngine : public JoinEnv {
         // position; their hot runs go to the other queue
         ks.Open("else if (phase == 4)");
         ks.L("const int qi = (int)a.w[" + std::to_string(w_qin_) + "];");
-        ks.L("const uint64_t nq = " + TC + "[qi];");
-        ks.L("const uint64_t nt = nq < " + TCAP + " ? nq : " + TCAP + ";");
+        ks.L("const uint64_t n0 = " + TC + "[2 * qi], n1 = " + TC + "[2 * qi + 1], longs = " + TCAP + " - " + SHORTS + ";");
+        ks.L("const uint64_t ns = n0 < " + SHORTS + " ? n0 : " + SHORTS + ", nt = ns + (n1 < longs ? n1 : longs);");
         ks.L("const uint64_t* tq = qi ? " + TQ1 + " : " + TQ0 + ";");
         const std::string LANES = std::to_string(kTaskLanes);
         ks.Open("for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nt * " + LANES +
                 "; w += (uint64_t)gridDim.x * blockDim.x)");
-        ks.L("const uint64_t* t = tq + w / " + LANES + " * " + TW + ";");
+        ks.L("const uint64_t task = w / " + LANES + ";");
+        ks.L("const uint64_t* t = tq + (task < ns ? task : task - ns + " + SHORTS + ") * " + TW + ";");
         ks.L("use_ep((int)t[3 + " + TS + "]);");
         ks.L("const int tp = (int)t[0];");
         ks.L("const int64_t share = ((int64_t)(t[2] - t[1]) + " + LANES + " - 1) / " + LANES + ";");
@@ -5509,8 +5525,12 @@ class SkinnerEngine : public JoinEnv {
   // split_run_ at position 3 or deeper pushes it, in chunks of split_run_,
   // as tasks {position, begin, end, bound rows} to a queue instead of
   // walking it alone; the host then runs the queued tasks grid-wide (their
-  // own hot runs go to the other queue) until both are empty.  A full queue
-  // leaves the run to the thread that met it.  A candidate costs its thread
+  // own hot runs go to the other queue) until both are empty.  The second half
+  // of a queue takes runs beyond kLongRun in chunks of that when the first is
+  // full; a full queue leaves the run to the thread that met it (a chain of 10
+  // tables, 3.5M rows: 320 ms against 1.5).  Queues hold as many tasks as the
+  // joined tables have rows, within limits (16384 were enough on 3.5M rows; 12.6 MB
+  // for 8 tables at most).  A candidate costs its thread
   // about a microsecond of dependent loads and a round of tasks about 25 us,
   // so runs split early and kTaskLanes threads share a task: on a Zipf 1.5
   // chain of 8 tables (200k rows) 1.2 ms with chunks of 32, 1.6 with 128, 2.2
@@ -5518,8 +5538,9 @@ class SkinnerEngine : public JoinEnv {
   // round of tasks.
   bool split_ = false;
   static constexpr int kTaskLanes = 16;
+  static constexpr int64_t kLongRun = 2048, kMinTasks = 1 << 12, kMaxTasks = 1 << 16;
   int64_t split_run_ = 32;
-  int64_t task_cap_ = 1 << 18;
+  int64_t task_cap_ = kMinTasks;
   uint64_t* tasks_[2] = {nullptr, nullptr};
   uint64_t* tcount_ = nullptr;
   int w_qin_ = 0;

@@ -267,3 +267,27 @@ def test_index_key_types_match_oracle(engine, kind):
         engine.register_table(t)
         o.register_table(t)
     assert compare(engine.execute(plan), o.execute(plan)) == ""
+
+
+# a join of 8 tables of at most 1000 rows, in a process of its own: the fixed
+# scratch (34 MB of slices and items, the pool's granularity, the kernels) and
+# queues as large as such tables need; with room for 2^18 tasks they alone took 50 MB
+def test_small_join_takes_little_device_memory():
+    import os
+    import subprocess
+    import sys
+    code = (
+        "import torch\n"
+        "from kushdb_b200 import workloads as wl\n"
+        "from kushdb_b200.engine import Engine\n"
+        "e = Engine(0)\n"
+        "tables, tokens = wl.skinner_tables('chain', 8, 300, 1000, 0.0, prefix='sm')\n"
+        "for t in tables: e.register_table(t)\n"
+        "plan = wl.skinner_plan(tables, tokens, 'chain').to_json().encode()\n"
+        "free = torch.cuda.mem_get_info()[0]\n"
+        "e.execute(plan)\n"
+        "print((free - torch.cuda.mem_get_info()[0]) >> 20)\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert int(out.stdout) <= 96
