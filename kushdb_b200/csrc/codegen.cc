@@ -6236,10 +6236,7 @@ std::unique_ptr<ops::SelVec> ScanSelectRows(Context& ctx, const std::string& tab
   ctx.D2H(&total, counts + ntiles, sizeof(total));
   ctx.CheckDeviceError("scan select");
   sv->n = static_cast<int64_t>(total);
-  sv->rows = static_cast<int32_t*>(nullptr);
-  void* out = nullptr;
-  KDB_CUDA(cudaMallocAsync(&out, sizeof(int32_t) * std::max<uint64_t>(total, 1), ctx.stream));
-  sv->rows = static_cast<int32_t*>(out);
+  sv->rows = static_cast<int32_t*>(sv->memory.Alloc(ctx, sizeof(int32_t) * total));
   sv->ctx = &ctx;
   ops::GatherTiles(ctx, scratch, counts, ntiles, sv->rows);
   KDB_CUDA(cudaStreamSynchronize(ctx.stream));

@@ -277,6 +277,16 @@ std::map<std::string, std::string> OptionsFromEnvironment() {
 }
 }  // namespace
 
+namespace {
+std::shared_ptr<CUstream_st> OwnedStream(cudaStream_t* out) {
+  cudaStream_t s = nullptr;
+  KDB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  *out = s;
+  return std::shared_ptr<CUstream_st>(s, [](cudaStream_t p) { cudaStreamDestroy(p); });
+}
+}  // namespace
+
+
 Context::Context(int dev) : device(dev) {
   options = OptionsFromEnvironment();
   if (dev < 0) {
@@ -287,7 +297,7 @@ Context::Context(int dev) : device(dev) {
   KDB_CUDA(cudaSetDevice(dev));
   KDB_CUDA(cudaFree(nullptr));
   KDB_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
-  KDB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  stream_owner = OwnedStream(&stream);
   // keep freed stream-ordered memory in the pool between queries
   cudaMemPool_t pool;
   KDB_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
@@ -308,7 +318,7 @@ Context::Context(Context& parent)
     return;
   }
   KDB_CUDA(cudaSetDevice(device));
-  KDB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  stream_owner = OwnedStream(&stream);
   KDB_CUDA(cudaMalloc(&d_err, sizeof(int) * 4));
   KDB_CUDA(cudaMemset(d_err, 0, sizeof(int) * 4));
 }
@@ -342,7 +352,6 @@ Context::~Context() {
     for (auto& [k, p] : cache_->programs)
       if (p->module) g_drv.ModuleUnload(p->module);
   cudaFree(d_err);
-  cudaStreamDestroy(stream);
 }
 
 void Context::FreeColumn(DevColumn& c) {

@@ -235,6 +235,9 @@ class Context {
   bool dry = false;
   int num_sms = 148;
   cudaStream_t stream = nullptr;
+  // Keeps `stream` for objects whose memory is freed on it, which may outlive
+  // the context.
+  std::shared_ptr<CUstream_st> stream_owner;
   std::map<std::string, DevTable> tables;
   std::map<int32_t, DevEnum> enums;
   std::string last_error;

@@ -718,15 +718,6 @@ int CheckErr(Context& c, int* d_err, const char* what) {
   return h;
 }
 
-// Stream-ordered device memory of an operator's own object (freed on the
-// context's stream): a table or pair list of a hundred MB costs cudaMalloc
-// and cudaFree hundreds of microseconds and a device synchronisation each.
-void* PoolAlloc(Context& c, size_t bytes) {
-  void* p = nullptr;
-  KDB_CUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 16), c.stream));
-  return p;
-}
-
 // Staged tuples of this many bytes are scattered by chunks: most of L2.
 constexpr int64_t kChunkedBytes = int64_t(96) << 20;
 
@@ -765,18 +756,21 @@ int PartGrid(const Context& c, int64_t n) {
 // Host side
 // ---------------------------------------------------------------------------
 
-SelVec::~SelVec() {
-  if (ctx && rows) {
-    cudaSetDevice(ctx->device);
-    cudaFreeAsync(rows, ctx->stream);
-  }
+// A table or pair list of a hundred MB costs cudaMalloc and cudaFree hundreds
+// of microseconds and a device synchronisation each.
+void* StreamMemory::Alloc(Context& c, size_t bytes) {
+  stream_ = c.stream_owner;
+  device_ = c.device;
+  void* p = nullptr;
+  KDB_CUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 16), c.stream));
+  held_.push_back(p);
+  return p;
 }
 
-HashTable::~HashTable() {
-  if (!ctx) return;
-  cudaSetDevice(ctx->device);
-  if (slots) cudaFreeAsync(slots, ctx->stream);
-  if (slot_off) cudaFreeAsync(slot_off, ctx->stream);
+StreamMemory::~StreamMemory() {
+  if (held_.empty()) return;
+  cudaSetDevice(device_);
+  for (void* p : held_) cudaFreeAsync(p, stream_.get());
 }
 
 static int64_t SelCount(const Context& c, const std::string& table, const SelVec* sel) {
@@ -867,7 +861,7 @@ std::unique_ptr<SelVec> SortRows(Context& c, const std::string& table, const std
   out->ctx = &c;
   out->table = table;
   out->n = n;
-  KDB_CUDA(cudaMallocAsync(&out->rows, sizeof(int32_t) * std::max<int64_t>(n, 1), c.stream));
+  out->rows = static_cast<int32_t*>(out->memory.Alloc(c, sizeof(int32_t) * n));
   if (n == 0) return out;
   Arena arena(c);
   uint64_t* kbuf = arena.AllocT<uint64_t>(n);
@@ -936,9 +930,9 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
   if (ht->bits == 0) {
     uint64_t cap = 16;
     while (static_cast<double>(cap) * load_factor < static_cast<double>(n) + 1) cap <<= 1;
-    ht->slots = PoolAlloc(c, cap * slot_bytes);
+    ht->slots = ht->memory.Alloc(c, cap * slot_bytes);
     std::vector<unsigned long long> off = {0, cap};
-    ht->slot_off = static_cast<unsigned long long*>(PoolAlloc(c, sizeof(off[0]) * 2));
+    ht->slot_off = static_cast<unsigned long long*>(ht->memory.Alloc(c, sizeof(off[0]) * 2));
     KDB_CUDA(cudaMemcpyAsync(ht->slot_off, off.data(), sizeof(off[0]) * 2, cudaMemcpyHostToDevice, c.stream));
     c.Memset(ht->slots, 0, cap * slot_bytes);
     ht->total_slots = cap;
@@ -956,7 +950,7 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
     unsigned* hist = arena.AllocT<unsigned>(parts);
     unsigned* cursor = arena.AllocT<unsigned>(parts);
     unsigned long long* stage_off = arena.AllocT<unsigned long long>(parts + 1);
-    ht->slot_off = static_cast<unsigned long long*>(PoolAlloc(c, sizeof(unsigned long long) * (parts + 1)));
+    ht->slot_off = static_cast<unsigned long long*>(ht->memory.Alloc(c, sizeof(unsigned long long) * (parts + 1)));
     c.Memset(hist, 0, sizeof(unsigned) * parts);
     const int cgrid = PartGrid(c, n);
     const int64_t chunk = (n + cgrid - 1) / cgrid;
@@ -973,7 +967,7 @@ std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const
     KDB_CUDA(cudaMemcpyAsync(&totals[1], ht->slot_off + parts, 8, cudaMemcpyDeviceToHost, c.stream));
     KDB_CUDA(cudaStreamSynchronize(c.stream));
     ht->total_slots = static_cast<int64_t>(totals[1]);
-    ht->slots = PoolAlloc(c, totals[1] * slot_bytes);
+    ht->slots = ht->memory.Alloc(c, totals[1] * slot_bytes);
     void* staged = arena.Alloc(std::max<unsigned long long>(totals[0], 2) * slot_bytes);
     c.TimedStart("hash scatter");
     LaunchScatter(c, ht->wide, cgrid, key, srows, n, chunk, ht->bits, block_hist, stage_off, cursor, staged);
@@ -1042,8 +1036,8 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
     auto pr = std::make_unique<Pairs>();
     pr->ctx = &c;
     pr->n = static_cast<int64_t>(total);
-    pr->probe = static_cast<int32_t*>(PoolAlloc(c, sizeof(int32_t) * pr->n));
-    pr->build = static_cast<int32_t*>(PoolAlloc(c, sizeof(int32_t) * pr->n));
+    pr->probe = static_cast<int32_t*>(pr->memory.Alloc(c, sizeof(int32_t) * pr->n));
+    pr->build = static_cast<int32_t*>(pr->memory.Alloc(c, sizeof(int32_t) * pr->n));
     c.TimedStart("hash pairs");
     MatchPairs<<<static_cast<unsigned>(tiles), kBlock, 0, c.stream>>>(match, n, counts, pr->probe, pr->build);
     c.TimedStop();
@@ -1082,8 +1076,8 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
         uint32_t* dummy = arena.AllocT<uint32_t>(total);
         c.RadixSortPairs(reinterpret_cast<uint64_t*>(out), dummy, static_cast<int64_t>(total), arena, 64);
       }
-      pr->probe = static_cast<int32_t*>(PoolAlloc(c, sizeof(int32_t) * total));
-      pr->build = static_cast<int32_t*>(PoolAlloc(c, sizeof(int32_t) * total));
+      pr->probe = static_cast<int32_t*>(pr->memory.Alloc(c, sizeof(int32_t) * total));
+      pr->build = static_cast<int32_t*>(pr->memory.Alloc(c, sizeof(int32_t) * total));
       if (total > 0) {
         SplitPairs<<<c.GridFor(static_cast<int64_t>(total), kBlock), kBlock, 0, c.stream>>>(
             out, static_cast<int64_t>(total), pr->probe, pr->build);
@@ -1095,13 +1089,6 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
     cap = total;
   }
   throw Error(KDB_ERR_CAPACITY, "probe output did not converge");
-}
-
-Pairs::~Pairs() {
-  if (!ctx) return;
-  cudaSetDevice(ctx->device);
-  if (probe) cudaFreeAsync(probe, ctx->stream);
-  if (build) cudaFreeAsync(build, ctx->stream);
 }
 
 

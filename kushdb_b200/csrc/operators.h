@@ -1,6 +1,7 @@
 // Host-side objects of the per-operator entry points (operators.cu): device
 // selection vectors, hash tables, probe results, aggregate tables and column
-// indexes.  Each belongs to one Context and must be freed before it.
+// indexes.  Each belongs to one Context and must be freed before it (stream
+// memory is given back safely even if it is not).
 #pragma once
 
 #include <cstdint>
@@ -13,13 +14,28 @@
 namespace kdb {
 namespace ops {
 
+// Device memory from the stream-ordered pool that belongs to an object.
+class StreamMemory {
+ public:
+  StreamMemory() = default;
+  StreamMemory(const StreamMemory&) = delete;
+  StreamMemory& operator=(const StreamMemory&) = delete;
+  ~StreamMemory();
+  void* Alloc(Context& c, size_t bytes);
+
+ private:
+  std::shared_ptr<CUstream_st> stream_;
+  int device_ = 0;
+  std::vector<void*> held_;
+};
+
 // Ascending row ids of one table's rows that passed a scan-select.
 struct SelVec {
   Context* ctx = nullptr;
+  StreamMemory memory;
   std::string table;
   int32_t* rows = nullptr;  // device, n entries
   int64_t n = 0;
-  ~SelVec();
 };
 
 // A device join table over one integer key column (runtime::HashTable).
@@ -36,7 +52,7 @@ struct HashTable {
   unsigned long long* slot_off = nullptr;  // device, 2^bits + 1 sub-table offsets (slots)
   int64_t total_slots = 0;
   size_t bytes = 0;
-  ~HashTable();
+  StreamMemory memory;
 };
 
 // (probe row, build row) pairs of a probe, as two device arrays.
@@ -45,7 +61,7 @@ struct Pairs {
   int32_t* probe = nullptr;
   int32_t* build = nullptr;
   int64_t n = 0;
-  ~Pairs();
+  StreamMemory memory;
 };
 
 std::unique_ptr<HashTable> HashBuild(Context& c, const std::string& table, const std::string& key_column,

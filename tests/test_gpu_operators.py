@@ -484,3 +484,23 @@ def test_hash_build_scatters_around_l2(engine, tname, nb):
     assert np.array_equal(probe, np.nonzero(hit)[0]) and np.array_equal(build, want[hit])
     for x in (t, p):
         engine.drop_table(x.name)
+
+
+# `with Engine(0) as e:` closes the engine at the end of the block, the objects
+# made in it go when their names do
+def test_objects_closed_after_their_engine():
+    from kushdb_b200.engine import Engine
+    from kushdb_b200.operators import HashTable, scan_select, sort_rows
+    t = _key_table("late", np.arange(5000), None)
+    for fanout in (1, 64):
+        with Engine(0) as e:
+            e.register_table(t)
+            h = HashTable(e, "late", "k", fanout=fanout)
+            s = scan_select(e, "late", ["k"], Lt(V(Type.Int(), 0), LiteralExpression(Type.Int(), 100)))
+            o = sort_rows(e, "late", ["k"], [False], s)
+            assert len(h.probe("late", "k")[0]) == 5000 and list(o.rows()) == list(range(99, -1, -1))
+        for x in (h, s, o):
+            x.close()
+    with Engine(0) as e:
+        e.register_table(t)
+        assert len(HashTable(e, "late", "k").probe("late", "k")[0]) == 5000
