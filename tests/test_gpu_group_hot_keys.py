@@ -79,3 +79,10 @@ def test_bigint_zero_is_as_cheap_as_another_hot_key(engine):
     other = _run(engine, "hk_seven", Type.BigInt(), k)
     k[hot] = 0
     assert _run(engine, "hk_zero", Type.BigInt(), k) < 2 * other
+
+
+def test_records_beyond_l2(engine):
+    # 2M groups: the table regrows past L2, where only first positions are read ahead
+    k = np.random.default_rng(3).permutation(np.concatenate([np.arange(2_000_000), np.arange(2_000_000)]))
+    _run(engine, "hk_many", Type.Int(), k.astype(np.int32))
+    _run(engine, "hk_many_big", Type.BigInt(), k * 5)
