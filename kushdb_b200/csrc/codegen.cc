@@ -964,6 +964,8 @@ class Executor {
   void EmitJoinInsert(KernelSource& ks, ExprGen& eg, const JoinTable& jt, const std::vector<CVal>& vals,
                       const std::vector<int>& key_cols, const std::string& row);
   std::vector<JoinTable> BuildGroupedIndexes(const std::vector<std::pair<const MatBuffer*, int>>& cols);
+  // set while emitting a probe whose matches' handling folds a warp's lanes
+  bool gather_matches_ = false;
   std::string probe_br_;  // inside an on_match callback: the matched build row's index
   // set while emitting a probe whose kernel staged the join filter in
   // shared memory: the array's name
@@ -1708,18 +1710,33 @@ void Executor::EmitProbe(KernelSource& ks, ExprGen& eg, const JoinTable& jt,
   }
   std::string i = ks.Fresh("i"), k = ks.Fresh("k"), e = ks.Fresh("e");
   ks.L("uint32_t " + i + " = " + h + " & " + mask + ";");
-  ks.Open("for (uint32_t " + k + " = 0; " + k + " <= " + mask + "; " + k + "++, " + i + " = (" + i +
-          " + 1) & " + mask + ")");
-  if (ahead && ahead_slot_on_)
-    ks.L("uint64_t " + e + " = " + k + " == 0 ? " + ahead_slot_ + " : " + slots + "[" + i + "];");
-  else ks.L("uint64_t " + e + " = " + slots + "[" + i + "];");
-  ks.L("if (" + e + " == 0) break;");
+  const bool by_key = jt.key_in_slot && bkeys.size() == 1 && bkeys[0] == jt.key_col && pk[0].type.id != TypeId::REAL &&
+                      pk[0].type.id != TypeId::TEXT && pk[0].type.id != TypeId::BOOLEAN;
+  // a slot's key (sign-extended, against the probe value in 64 bits) or hash
+  const std::string same = by_key ? "(int64_t)(int32_t)(uint32_t)(" + e + " >> 32) == (int64_t)(" + pk[0].v + ")"
+                                  : "(uint32_t)(" + e + " >> 32) == " + h;
+  const std::string load = e + " = " + (ahead && ahead_slot_on_ ? k + " == 0 ? " + ahead_slot_ + " : " : "") + slots + "[" + i + "];";
+  const std::string step = k + "++, " + i + " = (" + i + " + 1) & " + mask;
+  if (gather_matches_) {
+    // each lane goes on to its next match first, and all that have one then
+    // handle theirs together (opaque, or the compiler sends each to its match
+    // as it finds it: the GROUP BY of 2M rows matched in a table of 200k, 300
+    // groups, 238 us against 82)
+    ks.L("uint64_t " + e + " = 0;");
+    ks.Open("for (uint32_t " + k + " = 0;; " + step + ")");
+    ks.L("for (; " + k + " <= " + mask + "; " + step + ") { " + load + " if (" + e + " == 0 || " + same + ") break; }");
+    ks.L("int " + k + "go = " + k + " <= " + mask + " && " + e + " != 0;");
+    ks.L("asm volatile(\"\" : \"+r\"(" + k + "go));");
+    ks.L("if (!" + k + "go) break;");
+  } else {
+    ks.Open("for (uint32_t " + k + " = 0; " + k + " <= " + mask + "; " + step + ")");
+    ks.L("uint64_t " + load);
+    ks.L("if (" + e + " == 0) break;");
+  }
   std::string br = ks.Fresh("br");
   std::vector<CVal> left;
-  if (jt.key_in_slot && bkeys.size() == 1 && bkeys[0] == jt.key_col && pk[0].type.id != TypeId::REAL &&
-      pk[0].type.id != TypeId::TEXT && pk[0].type.id != TypeId::BOOLEAN) {
-    // the stored key, sign-extended, against the probe value in 64 bits
-    ks.Open("if ((int64_t)(int32_t)(uint32_t)(" + e + " >> 32) == (int64_t)(" + pk[0].v + "))");
+  if (by_key) {
+    ks.Open("if (" + same + ")");
     ks.L("int64_t " + br + " = (int64_t)(uint32_t)" + e + " - 1;");
     left = LoadMatRow(ks, eg, jt.build, br, nullptr);
     const MatCol& kc = jt.build.cols.at(jt.key_col);
@@ -1727,7 +1744,7 @@ void Executor::EmitProbe(KernelSource& ks, ExprGen& eg, const JoinTable& jt,
     ks.Open("");
   } else {
     if (jt.key_in_slot) throw Error(-5, "join probe does not match its key-in-slot table");
-    ks.Open("if ((uint32_t)(" + e + " >> 32) == " + h + ")");
+    ks.Open("if (" + same + ")");
     ks.L("int64_t " + br + " = (int64_t)(uint32_t)" + e + " - 1;");
     left = LoadMatRow(ks, eg, jt.build, br, nullptr);
     std::string eq = "true";
@@ -3646,8 +3663,10 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         }
         ks.Close();
       };
+      gather_matches_ = cache;
       if (Streamable(op.child())) EmitStream(ks, eg, op.child(), consume, src_rows);
       else EmitMatScan(ks, mats_.at(&op.child()), nullptr, consume, src_rows);
+      gather_matches_ = false;
       ks.globals << "#define KDB_R " << R << "\n";
       rec = arena_.AllocT<uint64_t>(nrec * R);
       ctx_.Memset(rec, 0, nrec * R * sizeof(uint64_t));

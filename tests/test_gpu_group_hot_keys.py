@@ -6,8 +6,8 @@ import numpy as np
 import pytest
 
 from kushdb_b200.data import HostColumn, HostTable, catalog_of
-from kushdb_b200.plan import (ColRef, ColRefE, Count, GroupByAggregateOperator, Min, OperatorSchema, OutputOperator,
-                              ScanOperator, Sum, Type, VirtColRef)
+from kushdb_b200.plan import (AggregateOperator, ColRef, ColRefE, Count, GroupByAggregateOperator, HashJoinOperator, Max,
+                              Min, OperatorSchema, OutputOperator, ScanOperator, Sum, Type, VirtColRef)
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +86,82 @@ def test_records_beyond_l2(engine):
     k = np.random.default_rng(3).permutation(np.concatenate([np.arange(2_000_000), np.arange(2_000_000)]))
     _run(engine, "hk_many", Type.Int(), k.astype(np.int32))
     _run(engine, "hk_many_big", Type.BigInt(), k * 5)
+
+
+def _join_tables(prefix, nb, np_, dup, text):
+    rng = np.random.default_rng(nb + dup)
+    b, p = HostTable(prefix + "b"), HostTable(prefix + "p")
+    bk, pk = rng.permutation(nb) // dup, rng.integers(-nb // (8 * dup), nb // dup, np_)
+    for t, name, k in ((b, "bk", bk), (p, "pk", pk)):
+        if text:
+            t.add(HostColumn.from_strings(name, ["k%d" % x for x in k]))
+        else:
+            t.add(HostColumn(name, Type.Int(), values=k.astype(np.int32), nulls=(rng.random(len(k)) < 0.05).astype(np.int8)))
+    b.add(HostColumn("bg", Type.Int(), values=rng.integers(0, 900, nb).astype(np.int32)))
+    p.add(HostColumn("g", Type.Int(), values=rng.integers(0, 300, np_).astype(np.int32)))
+    p.add(HostColumn("big", Type.BigInt(), values=rng.integers(0, 3, np_)))
+    p.add(HostColumn("v", Type.Int(), values=rng.integers(-1000, 1000, np_).astype(np.int32)))
+    return b, p
+
+
+def _over_join(b, p, key):
+    db = catalog_of([b, p])
+    scans = []
+    for t in (b, p):
+        s = OperatorSchema()
+        s.AddGeneratedColumns(db[t.name], list(t.columns))
+        scans.append(ScanOperator(s, db[t.name]))
+    js = OperatorSchema()
+    js.AddPassthroughColumns(scans[0], ["bg"], 0)
+    js.AddPassthroughColumns(scans[1], ["g", "big", "v"], 1)
+    j = HashJoinOperator(js, scans[0], scans[1], [ColRef(scans[0], "bk", 0)], [ColRef(scans[1], "pk", 1)])
+    return _groups(j, key)
+
+
+def _groups(src, key):
+    aggs = [Sum(ColRef(src, "v")), Min(ColRef(src, "v")), Max(ColRef(src, "v")), Count()]
+    o = OperatorSchema()
+    k = ColRefE(src, key) if key else None
+    if key:
+        o.AddDerivedColumn("k", VirtColRef(k, 0))
+    for i, a in enumerate(aggs):
+        o.AddDerivedColumn(f"a{i}", VirtColRef(a, i + (1 if key else 0)))
+    return OutputOperator(GroupByAggregateOperator(o, src, [k], aggs) if key else AggregateOperator(o, src, aggs))
+
+
+# several build rows per key, slots that share a hash (TEXT keys are compared after it), rows without a match
+@pytest.mark.parametrize("dup", [1, 3])
+@pytest.mark.parametrize("text", [False, True])
+@pytest.mark.parametrize("key", ["bg", "g", "big"])
+def test_groups_over_a_join_match_oracle(engine, dup, text, key):
+    from oracle import Oracle
+    from parity import compare
+    b, p = _join_tables(f"gj{dup}{text}{key}", 6000, 50_011, dup, text)
+    o = Oracle()
+    for t in (b, p):
+        engine.register_table(t)
+        o.register_table(t)
+    plan = _over_join(b, p, key)
+    assert compare(engine.execute(plan), o.execute(plan)) == ""
+
+
+# the groups of a join's matches cost about the join and the groups of as many
+# rows of a table (half as much again for the spread of the timings)
+def test_groups_over_a_join_cost_the_join_and_the_groups(engine):
+    b, p = _join_tables("gt", 200_000, 2_000_000, 1, False)
+    for t in (b, p):
+        engine.register_table(t)
+    s = OperatorSchema()
+    s.AddGeneratedColumns(catalog_of([p])[p.name], ["g", "v"])
+    plans = [_over_join(b, p, "g"), _over_join(b, p, None), _groups(ScanOperator(s, catalog_of([p])[p.name]), "g")]
+    us = []
+    for plan in plans:
+        engine.execute(plan)
+        engine.set_profiling(True)
+        t = []
+        for _ in range(5):
+            engine.execute(plan, fetch=False)
+            t.append(sum(k["ms"] for k in engine.last_kernels() if k["tag"] in ("group by", "aggregate")) * 1e3)
+        engine.set_profiling(False)
+        us.append(sorted(t)[2])
+    assert us[0] < 1.5 * (us[1] + us[2])
