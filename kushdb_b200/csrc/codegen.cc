@@ -3479,11 +3479,16 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         ks.L("const int64_t g = " + (zero ? "gkey == 0 ? (int64_t)(" + M + " + 1) * KDB_R : " : std::string()) + find + ";");
         if (zero) ks.L("if (gkey == 0) rec[g] = 1ULL;  // occupied (a BIGINT key 0)");
       };
-      // strings are compared in place: one update per row
+      // strings are compared in place: one update per row, for those not NULL (gt*)
+      auto text_flags = [&] {
+        for (size_t j = 0; j < plans.size(); j++)
+          if (plans[j].kind == StateKind::MinMaxText)
+            ks.L("const unsigned gt" + std::to_string(j) + " = " + N(j) + ";");
+      };
       auto text_to_record = [&](const std::vector<CVal>& vals, const std::string& g) {
         for (size_t j = 0; j < plans.size(); j++)
           if (plans[j].kind == StateKind::MinMaxText)
-            ks.L("if (" + N(j) + ") kdb_atomic_str_minmax(&rec[" + g + " + " + std::to_string(vw[j]) + "], " + vals[j].v +
+            ks.L("if (gt" + std::to_string(j) + ") kdb_atomic_str_minmax(&rec[" + g + " + " + std::to_string(vw[j]) + "], " + vals[j].v +
                  ", " + (plans[j].is_min ? "true" : "false") + ");");
       };
       // folds the values of the lanes that share `id` into the first of
@@ -3609,8 +3614,18 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
             ks.Open(!extremes ? "" : seen == kSeenAll ? "if (in_l2)" : "else");
             find_record("ghash", wide && !cache, seen);
             ks.Open("if (g >= 0)");
-            text_to_record(vals, "g");
-            to_record("g", seen);
+            if (cache) {
+              to_record("g", seen);
+            } else {
+              // (MIN of a string over 1M rows of which half share a key: 363
+              // us, 1305 without folding)
+              text_flags();
+              fold_lanes("(unsigned long long)g");
+              ks.Open("if (gl)");
+              to_record("g", seen);
+              ks.Close();
+              text_to_record(vals, "g");
+            }
             ks.Close();
             ks.Close();
           }
@@ -3650,15 +3665,12 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
                ") | 0x8000000000000000ULL, [&](uint64_t i) { return " + eq + "; }, [&](uint64_t i) { " + init +
                "}, " + ERR + ");");
           ks.Open("if (g >= 0)");
-          if (any_text) {
-            text_to_record(vals, "g * KDB_R");
-            to_record("g * KDB_R");
-          } else {
-            fold_lanes("(unsigned)g");
-            ks.Open("if (gl)");
-            to_record("g * KDB_R");
-            ks.Close();
-          }
+          text_flags();
+          fold_lanes("(unsigned long long)g");
+          ks.Open("if (gl)");
+          to_record("g * KDB_R");
+          ks.Close();
+          text_to_record(vals, "g * KDB_R");
           ks.Close();
         }
         ks.Close();
@@ -3699,11 +3711,14 @@ MatBuffer Executor::RunGroupBy(const Operator& op, bool any_order, const Operato
         ks.L("const unsigned long long gf = kdb_cf[i];");
         to_record("g", kSeenFirst);
         ks.Close();
-        // few, large blocks: every block flushes its cache at the end
-        const int block = 512;
-        const int grid = std::min(ctx_.GridFor(std::max<int64_t>(src_rows, 1), block), 2 * ctx_.num_sms);
+        // few, large blocks: every block flushes its cache at the end.  Three per
+        // SM behind a join, whose probes wait on one read after the other (400k
+        // rows probing by a string 38 us, 50 with two; 2M rows by an INT 82 to
+        // 107 us either way).
+        const int block = 512, per_sm = StreamHasJoin(op.child()) ? 3 : 2;
+        const int grid = std::min(ctx_.GridFor(std::max<int64_t>(src_rows, 1), block), per_sm * ctx_.num_sms);
         const std::string name = KernelName("group by");
-        ctx_.Launch(ctx_.Kernel(ks.Kernel(name, block, 2), name), grid, block, ks.Args(), 0, "group by");
+        ctx_.Launch(ctx_.Kernel(ks.Kernel(name, block, per_sm), name), grid, block, ks.Args(), 0, "group by");
       } else {
         LaunchPipeline(ks, src_rows, "group by");
       }

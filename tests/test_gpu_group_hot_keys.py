@@ -165,3 +165,43 @@ def test_groups_over_a_join_cost_the_join_and_the_groups(engine):
         engine.set_profiling(False)
         us.append(sorted(t)[2])
     assert us[0] < 1.5 * (us[1] + us[2])
+
+
+# MIN / MAX of a string keeps the block cache out: a hot key's other states are
+# folded all the same.  (Its strings still meet in one word: a row costs up to
+# ten times what a row of any other key does; unfolded it was 45 times.)
+def test_hot_key_with_string_extremes(engine):
+    from oracle import Oracle
+    from parity import compare
+    rows = 1_000_003
+    rng = np.random.default_rng(4)
+    strings = ["m%04d" % x for x in rng.integers(0, 9999, rows)]
+    us = []
+    for name, share in (("st", 0.0), ("sh", 0.95)):
+        k = rng.integers(10, 50_000, rows).astype(np.int32)
+        k[rng.random(rows) < share] = 7
+        t = HostTable(name)
+        t.add(HostColumn("k", Type.Int(), values=k))
+        t.add(HostColumn.from_strings("s", strings, (rng.random(rows) < 0.1).astype(np.int8)))
+        s = OperatorSchema()
+        s.AddGeneratedColumns(catalog_of([t])[name], ["k", "s"])
+        src = ScanOperator(s, catalog_of([t])[name])
+        key = ColRefE(src, "k")
+        aggs = [Min(ColRef(src, "s")), Max(ColRef(src, "s")), Count(), Count(ColRef(src, "s"))]
+        o = OperatorSchema()
+        o.AddDerivedColumn("k", VirtColRef(key, 0))
+        for i, a in enumerate(aggs):
+            o.AddDerivedColumn(f"a{i}", VirtColRef(a, i + 1))
+        plan = OutputOperator(GroupByAggregateOperator(o, src, [key], aggs))
+        engine.register_table(t)
+        ora = Oracle()
+        ora.register_table(t)
+        assert compare(engine.execute(plan), ora.execute(plan)) == ""
+        engine.set_profiling(True)
+        ts = []
+        for _ in range(5):
+            engine.execute(plan, fetch=False)
+            ts.append(sum(x["ms"] for x in engine.last_kernels() if x["tag"] == "group by") * 1e3)
+        engine.set_profiling(False)
+        us.append(sorted(ts)[2])
+    assert us[1] < 10 * us[0]
