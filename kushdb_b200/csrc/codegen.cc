@@ -780,6 +780,15 @@ class Executor {
       }
     }
   }
+  // How far a stream's positions move up to make room for the position of a
+  // joined row, below `bound` (-1: not known).  32 bits for each would leave 24 for
+  // the first rows of a join's groups, which also carry 8 flags, and none
+  // for the first table of three.
+  static std::string PosBits(KernelSource& ks, int64_t bound) {
+    int bits = bound < 0 ? 32 : 0;
+    while (bits < 32 && (int64_t(1) << bits) < bound) bits++;
+    return "(int)" + ks.Word(static_cast<uint64_t>(bits));
+  }
   static bool Streamable(const Operator& op) {
     return op.kind == OpKind::SCAN || op.kind == OpKind::SCAN_SELECT || op.kind == OpKind::SELECT ||
            op.kind == OpKind::HASH_JOIN || op.kind == OpKind::CROSS_PRODUCT;
@@ -1608,6 +1617,7 @@ void Executor::EmitStream(KernelSource& ks, ExprGen& eg, const Operator& op, con
       const JoinTable& jt = joins_.at(&op);
       std::vector<int> bkeys;
       for (const auto& k : op.left_keys) bkeys.push_back(k->column_idx);
+      const std::string bits = PosBits(ks, jt.build.pos_is_index ? jt.build.rows : jt.build.pos_bound);
       auto body = [&](const std::vector<CVal>& right, const std::string& pos) {
         Scope s;
         s.child.resize(2);
@@ -1620,7 +1630,7 @@ void Executor::EmitStream(KernelSource& ks, ExprGen& eg, const Operator& op, con
           s2.child.push_back(right);
           std::vector<CVal> out;
           for (const auto& c : op.output) out.push_back(eg.Emit(*c.expr, s2));
-          consume(out, "((" + pos + ") << 32) | ((" + bpos + ") & 0xffffffffULL)");
+          consume(out, "((" + pos + ") << " + bits + ") | ((" + bpos + ") & 0xffffffffULL)");
         });
       };
       probe_side_scan_ = !ctx_.OptStr("KDB_VECTOR_PROBE_SCAN");
@@ -1640,6 +1650,7 @@ void Executor::EmitStream(KernelSource& ks, ExprGen& eg, const Operator& op, con
       const uint32_t* lorder = cross_order_.count(&op) ? cross_order_.at(&op) : nullptr;
       const std::string NL = "(int64_t)" + ks.Word(static_cast<uint64_t>(lm.rows));
       const std::string LO = lorder ? ks.Ptr(lorder, "uint32_t", true) : "";
+      const std::string bits = PosBits(ks, lm.rows);
       auto body = [&](const std::vector<CVal>& right, const std::string& pos) {
         const std::string li = ks.Fresh("li"), lr = ks.Fresh("lr");
         ks.Open("for (int64_t " + li + " = 0; " + li + " < " + NL + "; " + li + "++)");
@@ -1650,7 +1661,7 @@ void Executor::EmitStream(KernelSource& ks, ExprGen& eg, const Operator& op, con
         s2.child.push_back(right);
         std::vector<CVal> out;
         for (const auto& c : op.output) out.push_back(eg.Emit(*c.expr, s2));
-        consume(out, "((" + pos + ") << 32) | (uint64_t)" + li);
+        consume(out, "((" + pos + ") << " + bits + ") | (uint64_t)" + li);
         ks.Close();
       };
       if (Streamable(op.child(1))) EmitStream(ks, eg, op.child(1), body, src_rows);

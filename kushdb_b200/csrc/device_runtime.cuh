@@ -585,9 +585,6 @@ struct KdbAddI64 {
 struct KdbMinU64 {
   KDB_DEV uint64_t operator()(uint64_t a, uint64_t b) const { return a < b ? a : b; }
 };
-struct KdbMaxU64 {
-  KDB_DEV uint64_t operator()(uint64_t a, uint64_t b) const { return a > b ? a : b; }
-};
 struct KdbMinI64 {
   KDB_DEV int64_t operator()(int64_t a, int64_t b) const { return a < b ? a : b; }
 };

@@ -101,3 +101,27 @@ def test_batch_group_order_at_bitmap_edges(facts):
         _check_against_plain(e, b, qs)
         _check_against_plain(e, b, qs)  # a second run of the same graph
         b.close()
+
+
+# more order chunks (of 32768 fact rows) than a block counts in shared memory (1024)
+def test_batch_group_order_beyond_the_shared_counters():
+    from kushdb_b200.data import HostColumn, HostTable
+    from kushdb_b200.engine import Batch, Engine
+    nf, nd = 1025 * 32_768 + 77, 1003
+    rng = np.random.default_rng(8)
+    d, f = HostTable("bl_dim"), HostTable("bl_fact")
+    d.add(HostColumn("d_key", wl.Type.Int(), values=(np.arange(nd) * 7).astype(np.int32)))
+    d.add(HostColumn("d_date", wl.Type.Date(), values=rng.integers(2440588, 2450000, nd).astype(np.int32)))
+    d.add(HostColumn("d_seg", wl.Type.Int(), values=np.zeros(nd, np.int32)))
+    fk = rng.integers(0, nd - 3, nf)
+    fk[[5, nf - 2, nf - 1]] = nd - 1, nd - 2, nd - 3  # groups whose first rows lie in the first and the last chunk
+    f.add(HostColumn("f_fk", wl.Type.Int(), values=(fk * 7).astype(np.int32)))
+    f.add(HostColumn("f_price", wl.Type.Real(), values=rng.random(nf)))
+    f.add(HostColumn("f_disc", wl.Type.Real(), values=rng.integers(0, 10, nf) / 100.0))
+    with Engine(0) as e:
+        e.register_table(d)
+        e.register_table(f)
+        q = (d, f, 2449000, 0)
+        b = Batch(e, [wl.batch_query_desc(*q)])
+        _check_against_plain(e, b, [q])
+        b.close()
