@@ -272,10 +272,10 @@ int kdb_sort(kdb_ctx* ctx, const char* table, const char* const* key_columns, co
  * NULL key are not inserted (and never match), duplicates are all kept.
  * sel NULL = every row.  load_factor in (0.05, 0.95].  fanout: 1 = one
  * open-addressing table; a power of two up to 8192 = that many sub-tables
- * chosen by the key hash's top bits (radix partitioned: both sides are
- * scattered by partition and each partition joins in shared memory, its
- * sub-table and probe tiles brought in by TMA bulk copies); 0 = one table
- * while it fits well inside L2, partitioned above. */
+ * chosen by the key hash's top bits (radix partitioned: the rows are
+ * scattered by partition and each sub-table is built in shared memory from
+ * bulk-copied tiles; a probe reads its row's sub-table in place); 0 = one
+ * table while it stays inside L2, partitioned above. */
 typedef struct kdb_hash kdb_hash;
 typedef struct kdb_pairs kdb_pairs;
 int kdb_hash_build(kdb_ctx* ctx, const char* table, const char* key_column, const kdb_selvec* sel,

@@ -17,15 +17,13 @@
 //                                      (memory_column_index.cc:17-121,
 //                                      column_index.cc:67-144)
 //
-// Hash join (kernel b).  A build side whose table fits comfortably in L2 is
-// one open-addressing table probed straight from the probe column.  A larger
-// build side is radix partitioned by the top bits of the key hash into P
-// sub-tables of at most ~128 KiB each: both sides are scattered into
-// partition order, then one CTA per partition copies its sub-table into
-// shared memory with a TMA bulk copy (cp.async.bulk, completion on an
-// mbarrier) and streams its probe tuples through shared memory in
-// double-buffered bulk-copied tiles, so every probe is a shared-memory
-// access instead of a random HBM sector.
+// Hash join (kernel b).  A build side whose table stays inside L2 is one
+// open-addressing table.  A larger one is radix partitioned by the top bits of
+// the key hash into P sub-tables of about 64 KiB: its rows are scattered into
+// partition order, then a CTA builds each partition's sub-table in shared
+// memory from tuples that bulk copies (cp.async.bulk, completion on an
+// mbarrier) bring in, and writes it out.  Probe rows are not partitioned: each
+// reads its sub-table in place.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -1016,9 +1014,10 @@ std::unique_ptr<Pairs> HashProbe(Context& c, const HashTable& ht, const std::str
     // unique build keys, probe rows in table order: one match word per row,
     // compacted (a selection's rows may come in any order, and more than
     // once, so it takes the pair list below).  From kMatchRowsMin rows on
-    // unordered pairs are made so, too: as a pair list 3M probes of 6M rows
-    // took 95 us against 80, 20M of 30M 1121 against 589, but 100k 13
-    // against 33 for the more launches.
+    // unordered pairs are made so, too (all kernels of a probe): as a pair
+    // list 3M probes of 6M rows took 103 us against 81, 20M of 30M 1243
+    // against 571 (the words 501, the pairs 70), but 100k of 100k 14 against 35
+    // for the more launches.
     int32_t* match = arena.AllocT<int32_t>(static_cast<size_t>(n));
     const int64_t tiles = (n + kMatchTile - 1) / kMatchTile;
     uint64_t* counts = arena.AllocT<uint64_t>(static_cast<size_t>(tiles) + 1);

@@ -33,7 +33,9 @@ class ResultColumn:
 class Result:
     """A query result.  Columns and the printer-format lines are read from
     the C result handle on first access; the handle is freed with the
-    object."""
+    object.  Up to 24 MB (9 bytes per value), all columns are views of one
+    array: a program that keeps one column of many results keeps the others'
+    memory too, unless it copies it (``col.values.copy()``)."""
 
     def __init__(self, columns: List[ResultColumn] = None, lines: List[str] = None):
         self._columns = columns
