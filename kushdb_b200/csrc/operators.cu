@@ -808,8 +808,9 @@ __global__ void SortKeyFill(const void* __restrict__ data, const int8_t* __restr
         case 2: k = static_cast<uint64_t>(static_cast<int64_t>(static_cast<const int32_t*>(data)[r])) ^ (1ULL << 63); break;
         case 3: k = static_cast<uint64_t>(static_cast<const int64_t*>(data)[r]) ^ (1ULL << 63); break;
         case 4: {
-          const uint64_t b = __double_as_longlong(static_cast<const double*>(data)[r]);
-          k = (b >> 63) ? ~b : (b | (1ULL << 63));
+          int64_t b = __double_as_longlong(static_cast<const double*>(data)[r]);
+          if (b == INT64_MIN) b = 0;  // -0.0 equals 0.0
+          k = static_cast<uint64_t>(b ^ ((b >> 63) | INT64_MIN));
           break;
         }
         default: k = static_cast<uint64_t>(rank[static_cast<const int32_t*>(data)[r]]); break;

@@ -77,3 +77,15 @@ def test_nan_keys_lose_no_row(engine, n, keys, asc, nulls):
         rank = ~rank
     place = [(a, b if asc[-1] else not b, 0 if b else c) for a, b, c in zip(g.tolist(), null.tolist(), rank.tolist())]
     assert place == sorted(place)
+
+
+# kdb_sort: the same order, ties in input order
+@pytest.mark.parametrize("n", [40, 2049, 20_000])
+@pytest.mark.parametrize("asc", [True, False])
+def test_sort_rows_of_zeros_and_infinities(engine, n, asc):
+    from kushdb_b200.operators import sort_rows
+    t = _table(f"sr{n}{asc}", n, False, False)
+    engine.register_table(t)
+    k = t.columns["k"].values + 0.0  # one zero
+    want = np.argsort(k if asc else -k, kind="stable")
+    assert np.array_equal(sort_rows(engine, t.name, ["k"], [asc]).rows(), want)
