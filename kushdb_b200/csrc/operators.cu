@@ -762,6 +762,7 @@ void* StreamMemory::Alloc(Context& c, size_t bytes) {
   void* p = nullptr;
   KDB_CUDA(cudaMallocAsync(&p, std::max<size_t>(bytes, 16), c.stream));
   held_.push_back(p);
+  bytes_ += bytes;
   return p;
 }
 
@@ -769,6 +770,17 @@ StreamMemory::~StreamMemory() {
   if (held_.empty()) return;
   cudaSetDevice(device_);
   for (void* p : held_) cudaFreeAsync(p, stream_.get());
+  // The pool itself gives nothing back, and what it keeps is lost to every other
+  // allocation (columns, other libraries).  Mapping it again costs about a
+  // millisecond per GB (100M BIGINT rows 8.7 ms, 12.6 when 4 GiB were kept), so
+  // a tenth of the memory stays for the next table.
+  if (bytes_ < (size_t(64) << 20)) return;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, device_) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      reserved > kPoolKept && cudaStreamSynchronize(stream_.get()) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, kPoolKept);
 }
 
 static int64_t SelCount(const Context& c, const std::string& table, const SelVec* sel) {

@@ -14,7 +14,8 @@
 namespace kdb {
 namespace ops {
 
-// Device memory from the stream-ordered pool that belongs to an object.
+// Device memory from the stream-ordered pool that belongs to an object.  When
+// a large object goes, the pool gives back what it holds beyond kPoolKept.
 class StreamMemory {
  public:
   StreamMemory() = default;
@@ -22,10 +23,12 @@ class StreamMemory {
   StreamMemory& operator=(const StreamMemory&) = delete;
   ~StreamMemory();
   void* Alloc(Context& c, size_t bytes);
+  static constexpr uint64_t kPoolKept = uint64_t(16) << 30;
 
  private:
   std::shared_ptr<CUstream_st> stream_;
   int device_ = 0;
+  size_t bytes_ = 0;
   std::vector<void*> held_;
 };
 

@@ -504,3 +504,17 @@ def test_objects_closed_after_their_engine():
     with Engine(0) as e:
         e.register_table(t)
         assert len(HashTable(e, "late", "k").probe("late", "k")[0]) == 5000
+
+
+# a closed table's memory is there for other allocations, up to the 16 GiB that the pool keeps
+def test_large_table_gives_its_memory_back(engine):
+    import torch
+    from kushdb_b200.operators import HashTable
+    t = _key_table("giant", np.arange(120_000_000), None, np.int64, "BIGINT")
+    engine.register_table(t)
+    free = torch.cuda.mem_get_info()[0]
+    h = HashTable(engine, "giant", "k", load_factor=0.06, fanout=1)
+    assert h.info()[2] >= 32 << 30
+    h.close()
+    assert torch.cuda.mem_get_info()[0] >= free - (16 << 30) - (64 << 20)
+    engine.drop_table("giant")
